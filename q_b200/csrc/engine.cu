@@ -407,9 +407,7 @@ struct Batch {
     if (max_nsol > 0)
       launch("atom_terms", [&] { k_atom_terms<<<dim3(cdiv(max_nsol, 128), nsys), 128, 0, s1>>>(p); });
     if (any_wpol) {
-      launch("watpol_rank", [&] { k_watpol_rank<<<dim3(std::max(max_nshell, 1), nsys), WPOL_BLOCK, watpol_smem, s2>>>(p); });
-      if (p.n_wp_tiles > 0)
-        launch("watpol", [&] { k_watpol_force<<<p.n_wp_tiles, WPOL_BLOCK, 0, s2>>>(p); });
+      launch("watpol", [&] { k_watpol<<<dim3(std::max(max_nshell, 1), nsys), WPOL_BLOCK, watpol_smem, s2>>>(p); });
     }
     join_streams();
     check_launch("force kernels");
@@ -1314,12 +1312,10 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       P.lf_atoms = dev_upload(lf, o);
     }
     {
-      std::vector<int2> pk, wp, qw;
+      std::vector<int2> pk, qw;
       for (int s = 0; s < n; s++) {
         const SysDev &S = B.sysh[s];
         for (int i0 = 0; i0 < std::max(S.nwat, S.nsol); i0 += 256) pk.push_back(make_int2(s, i0));
-        if (S.wpol && S.nshell > 0)
-          for (int i0 = 0; i0 < S.nwat; i0 += WPOL_BLOCK) wp.push_back(make_int2(s, i0));
         if (S.nq > 0)
           for (int i0 = 0; i0 < S.nwat; i0 += 128) qw.push_back(make_int2(s, i0));
       }
@@ -1329,8 +1325,8 @@ void build(Batch &B, qb_handle *const *hs, int n) {
           for (int ig = 0; ig < B.sysh[s].ncgp_sol; ig++) pwg.push_back(make_int2(s, ig));
       P.n_pw_groups = (int)pwg.size();
       P.pw_groups = dev_upload(pwg, o);
-      P.n_pk_tiles = (int)pk.size(); P.n_wp_tiles = (int)wp.size(); P.n_qw_tiles = (int)qw.size();
-      P.pk_tiles = dev_upload(pk, o); P.wp_tiles = dev_upload(wp, o); P.qw_tiles = dev_upload(qw, o);
+      P.n_pk_tiles = (int)pk.size(); P.n_qw_tiles = (int)qw.size();
+      P.pk_tiles = dev_upload(pk, o); P.qw_tiles = dev_upload(qw, o);
     }
     // other molecules: local atoms, constraints grouped into dependency levels
     std::vector<int4> info, info2;
@@ -1475,14 +1471,12 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     P.hr = dev_alloc<HistRef>(1, o);
     CUDA_TRY(cudaMemcpy(P.hr, &none, sizeof none, cudaMemcpyHostToDevice));
   }
-  B.watpol_smem = (size_t)B.max_nwat * (sizeof(double) + sizeof(int));   // member angles and indices
+  B.watpol_smem = (size_t)B.max_nwat * (sizeof(double) + 2 * sizeof(uint16_t));   // member angles, indices and order
   P.wtheta = dev_alloc<double>(std::max(woff, 1), o);
   P.wshell = dev_alloc<int8_t>(std::max(woff, 1), o);
-  P.wrank = dev_alloc<int>(std::max(woff, 1), o);
-  P.wshn = dev_alloc<int>((size_t)n * MAX_SHELLS, o);
   if (B.any_wpol) {
     if (B.watpol_smem > 200 * 1024) fail(QB_ERR_UNSUPPORTED, "too many waters for the polarisation kernel");
-    CUDA_TRY(cudaFuncSetAttribute(k_watpol_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(k_watpol, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   }
 }
 

@@ -117,8 +117,6 @@ struct DevPtrs {
   float4 *wrec32;            // their FP32 form (mixed engine): the packed and FP32 water-water kernels'
   double *wtheta;            // per water: dipole angle of the polarisation restraint
   int8_t *wshell;            // per water: polarisation shell (-1: none)
-  int *wrank;                // per water: rank in its shell
-  int *wshn;                 // [s*MAX_SHELLS + shell] members
   float *crg, *winv;
   double *mass;
   int *iac, *iq, *cgp, *asys;
@@ -188,10 +186,10 @@ struct DevPtrs {
   int *ww_mid;                             // per water: list entries below its own index (ascending lists)
   int *lf_atoms, n_lf;
   // blocks of the per-water kernels, (system, first index) each, only where
-  // a system has work: the water pass (256 waters or solute atoms), the
-  // polarisation forces (WPOL_BLOCK waters) and Q-water (128 list entries)
-  int2 *pk_tiles, *wp_tiles, *qw_tiles;
-  int n_pk_tiles, n_wp_tiles, n_qw_tiles;
+  // a system has work: the water pass (256 waters or solute atoms) and
+  // Q-water (128 list entries)
+  int2 *pk_tiles, *qw_tiles;
+  int n_pk_tiles, n_qw_tiles;
   int2 *pw_groups;                         // (system, solute group) of systems with waters
   int n_pw_groups;                     // atoms k_leapfrog moves (all but 3-constraint molecules')
   int *ww_n, *ww_sp;                       // count per water; [gw*ww_nch + c] count below chunk c's end
