@@ -110,6 +110,20 @@ struct Batch {
   bool streams_on = true;
   std::vector<int2> lrf_dims;   // per system with LRF: (charge groups, source tiles)
   size_t watpol_smem = 0;
+  // k_nb_qw: warps sharing the Q atoms of one group of 32 waters, warps per block
+  int qw_groups = 1, qw_warps = 4;
+  // As many warps (1, 2, 4 or 8) as keep the launch within 16 warps per SM.
+  // Kernel time with 1 / 2 / 4 / 8: 33 water groups (one window) 12 / 8 / 6 /
+  // 5.6 us; 693 (21 windows, FP32) 10 / 8 / 11 / 14; 1,353 (41 windows) 15 /
+  // 18 / 18 / 26; 2,772 (84 windows, FP32) 23 / 26 / 31 / 50.
+  void qw_plan(int sms) {
+    long long groups = 0;
+    for (auto &S : sysh)
+      if (S.nq > 0) groups += (S.nwat + 31) / 32;
+    qw_groups = 1;
+    while (qw_groups < QW_MAXWARPS && 2 * qw_groups * groups <= 16LL * sms) qw_groups *= 2;
+    qw_warps = std::max(4, qw_groups);
+  }
   int q_states = 0;           // state count shared by every system with Q atoms (0: they differ)
   int max_nq = 0;
   // profiling
@@ -379,28 +393,23 @@ struct Batch {
         launch("nb_ww", [&] { k_nb_ww<false, false><<<gw, WW_BLOCK, smem, stream>>>(p, wpb); });
       }
       if (any_q && p.n_qw_tiles > 0) launch("nb_qw", [&] {
-        const int g = p.n_qw_tiles;
-        if (any_hlj) {   // hydrogen LJ: the generic state count only
-          if (max_nq > NQ_SHARED) k_nb_qw<0, false, true><<<g, 128, 0, s2>>>(p);
-          else k_nb_qw<0, true, true><<<g, 128, 0, s2>>>(p);
-          return;
-        }
-        if (max_nq > NQ_SHARED) { k_nb_qw<0, false, false><<<g, 128, 0, s2>>>(p); return; }
+        const int g = p.n_qw_tiles, qg = qw_groups, nt = 32 * qw_warps;
+        if (any_hlj) { k_nb_qw<0, true><<<g, nt, 0, s2>>>(p, qg); return; }   // the generic state count only
         // the mixed engine's non-recording steps: forces alone in FP32
         if (fast_ww) {
           switch (q_states) {
-            case 1: k_nb_qw<1, true, false, true><<<g, 128, 0, s2>>>(p); break;
-            case 2: k_nb_qw<2, true, false, true><<<g, 128, 0, s2>>>(p); break;
-            default: k_nb_qw<0, true, false, true><<<g, 128, 0, s2>>>(p);
+            case 1: k_nb_qw<1, false, true><<<g, nt, 0, s2>>>(p, qg); break;
+            case 2: k_nb_qw<2, false, true><<<g, nt, 0, s2>>>(p, qg); break;
+            default: k_nb_qw<0, false, true><<<g, nt, 0, s2>>>(p, qg);
           }
           return;
         }
         switch (q_states) {
-          case 1: k_nb_qw<1, true, false><<<g, 128, 0, s2>>>(p); break;
-          case 2: k_nb_qw<2, true, false><<<g, 128, 0, s2>>>(p); break;
-          case 3: k_nb_qw<3, true, false><<<g, 128, 0, s2>>>(p); break;
-          case 4: k_nb_qw<4, true, false><<<g, 128, 0, s2>>>(p); break;
-          default: k_nb_qw<0, true, false><<<g, 128, 0, s2>>>(p);
+          case 1: k_nb_qw<1, false><<<g, nt, 0, s2>>>(p, qg); break;
+          case 2: k_nb_qw<2, false><<<g, nt, 0, s2>>>(p, qg); break;
+          case 3: k_nb_qw<3, false><<<g, nt, 0, s2>>>(p, qg); break;
+          case 4: k_nb_qw<4, false><<<g, nt, 0, s2>>>(p, qg); break;
+          default: k_nb_qw<0, false><<<g, nt, 0, s2>>>(p, qg);
         }
       });
     }
@@ -813,6 +822,8 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   std::vector<int> iqseq, qiac;
   std::vector<float> qcrg;
   std::vector<double> qavdw, qbvdw, sc, qq_el;
+  std::vector<QwAtom> qwa;
+  std::vector<QwState> qws;
   std::vector<int8_t> qconn;
   std::vector<int4> qq;
   std::vector<int2> bij; std::vector<double2> bpar;
@@ -1085,6 +1096,41 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       S.aH[0] = V.type_avdw[3 * V.iac_hw]; S.aH[1] = V.type_avdw[3 * V.iac_hw + 1];
       S.bH[0] = V.type_bvdw[3 * V.iac_hw]; S.bH[1] = V.type_bvdw[3 * V.iac_hw + 1];
     }
+    // Q-water tables (k_nb_qw): LJ codes and products with the water types,
+    // charge products in single precision as crg_ow*qcrg
+    for (int q = 0; q < V.nqat; q++) {
+      QwAtom A{};
+      A.atom = aoff + V.iqseq[q];
+      const int t = V.iac[V.iqseq[q]], ncol = V.natyps + V.nqat;
+      int lj = 1, ljh = 1;
+      if (V.nwat > 0) {
+        lj = V.ljcod[V.iac_ow * V.natyps + t];
+        lj_pair(S.arith, V.type_avdw[3 * t + lj - 1], S.aO[lj - 1], V.type_bvdw[3 * t + lj - 1], S.bO[lj - 1], A.A, A.B);
+        if (S.hlj) {
+          ljh = V.ljcod[V.iac_hw * V.natyps + t];
+          lj_pair(S.arith, V.type_avdw[3 * t + ljh - 1], S.aH[ljh - 1], V.type_bvdw[3 * t + ljh - 1], S.bH[ljh - 1],
+                  A.AH, A.BH);
+        }
+      }
+      qwa.push_back(A);
+      for (int k = 0; k < MAXS; k++) {
+        QwState Q{};
+        if (k < V.nstates && V.nwat > 0) {
+          const float c = V.qcrg[q * V.nstates + k];
+          Q.qO = S.crg_ow * c;
+          Q.qH = S.crg_hw * c;
+          const int ti = V.qiac[q * V.nstates + k];
+          const double a = ti < V.nqlib ? V.qavdw[3 * ti] : 0.0, b = ti < V.nqlib ? V.qbvdw[3 * ti] : 0.0;
+          lj_pair(S.arith, a, S.aO[lj - 1], b, S.bO[lj - 1], Q.A, Q.B);
+          if (S.qvdw) Q.sc = V.sc_lookup[((size_t)q * ncol + V.iac_ow) * V.nstates + k];
+          if (S.hlj) {
+            lj_pair(S.arith, a, S.aH[ljh - 1], b, S.bH[ljh - 1], Q.AH, Q.BH);
+            if (S.qvdw) Q.scH = V.sc_lookup[((size_t)q * ncol + V.iac_hw) * V.nstates + k];
+          }
+        }
+        qws.push_back(Q);
+      }
+    }
     SysState &st = sst[s];
     std::memset(&st, 0, sizeof st);
     st.Tscale_sol = st.Tscale_solv = 1.0;
@@ -1262,6 +1308,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   P.lrft = dev_upload(lrft, o);
   P.iqseq = dev_upload(iqseq, o); P.qcrg = dev_upload(qcrg, o); P.qiac = dev_upload(qiac, o);
   P.qavdw = dev_upload(qavdw, o); P.qbvdw = dev_upload(qbvdw, o); P.sc = dev_upload(sc, o);
+  P.qwa = dev_upload(qwa, o); P.qws = dev_upload(qws, o);
   P.qconn = dev_upload(qconn, o); P.qq = dev_upload(qq, o); P.qq_el = dev_upload(qq_el, o);
   P.bij = dev_upload(bij, o); P.bpar = dev_upload(bpar, o); P.aijk = dev_upload(aijk, o); P.apar = dev_upload(apar, o); P.aub = dev_upload(aub, o);
   P.tijkl = dev_upload(tijkl, o); P.tpar = dev_upload(tpar, o); P.iijkl = dev_upload(iijkl, o); P.ipar = dev_upload(ipar, o);
@@ -1312,12 +1359,15 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       P.lf_atoms = dev_upload(lf, o);
     }
     {
+      int sms = 148;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B.opt.device);
+      B.qw_plan(sms);
       std::vector<int2> pk, qw;
       for (int s = 0; s < n; s++) {
         const SysDev &S = B.sysh[s];
         for (int i0 = 0; i0 < std::max(S.nwat, S.nsol); i0 += 256) pk.push_back(make_int2(s, i0));
         if (S.nq > 0)
-          for (int i0 = 0; i0 < S.nwat; i0 += 128) qw.push_back(make_int2(s, i0));
+          for (int i0 = 0; i0 < S.nwat; i0 += 32 * (B.qw_warps / B.qw_groups)) qw.push_back(make_int2(s, i0));
       }
       std::vector<int2> pwg;
       for (int s = 0; s < n; s++)

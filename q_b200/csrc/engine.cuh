@@ -23,7 +23,6 @@ constexpr int LRF_STRIDE = 24;
 constexpr int MAX_SHELLS = 4;
 // one history record: step, E[QB_NE], EQ[MAXS*QB_NEQ], r_kl of the off-diagonal functions [MAXS]
 constexpr int HIST_REC = 1 + QB_NE + MAXS * QB_NEQ + MAXS;
-constexpr int NQ_SHARED = 64;    // Q atoms whose water forces are reduced in shared memory
 // F_SHAKE: in a SHAKE constraint; F_SH3: in a 3-constraint molecule, moved by k_leapfrog_shake3
 enum AtomFlags : uint8_t { F_EXCL = 1, F_SHELL = 2, F_HEAVY = 4, F_SHAKE = 8, F_SH3 = 16 };
 
@@ -34,6 +33,19 @@ struct PwAtom {
   double4 lj;
   float2 q;
   int atom, pad;
+};
+
+// A Q atom's interaction parameters for the water O and H sites: the LJ
+// products of its topology type (hard core, the same in every state; H: with
+// hydrogen LJ), and per state the single precision charge products, the LJ
+// products of its Q type and the soft-core shifts.
+struct QwAtom {
+  double A, B, AH, BH;
+  int atom, pad;
+};
+struct QwState {
+  float qO, qH;
+  double A, B, sc, AH, BH, scH;
 };
 
 // Per-system record (read-only on the device during a run).
@@ -138,6 +150,8 @@ struct DevPtrs {
   int *qiac;                // [gq*MAXS + st] local Q type
   double *qavdw, *qbvdw;    // per system segments [qlib_off + 3*t + code-1]
   double *sc;               // per system segments [sc_off + (iq*(natyps+nq)+col)*S + st]
+  QwAtom *qwa;              // [gq]
+  QwState *qws;             // [gq*MAXS + st]
   int8_t *qconn;            // per system segments [qconn_off + (st*nsol + i)*nq + iq]
   int4 *qq;                 // (gq, gj, gjq or -1, lj | st<<8)
   double *qq_el;
@@ -187,7 +201,7 @@ struct DevPtrs {
   int *lf_atoms, n_lf;
   // blocks of the per-water kernels, (system, first index) each, only where
   // a system has work: the water pass (256 waters or solute atoms) and
-  // Q-water (128 list entries)
+  // Q-water (one block's list entries)
   int2 *pk_tiles, *qw_tiles;
   int n_pk_tiles, n_qw_tiles;
   int2 *pw_groups;                         // (system, solute group) of systems with waters

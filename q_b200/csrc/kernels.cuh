@@ -1824,74 +1824,58 @@ __device__ __forceinline__ void nb_qp_body(DevPtrs &P, int bx, int s, int gx) {
   }
 }
 
-// nonbond_qw_spc (md.f90:11302): Q atoms with the listed waters, one thread
-// per water, all Q atoms and states in the thread.  The Q atoms' positions
-// and per-state parameters (charge products with the water O and H in single
-// precision as crg_ow*qcrg, LJ products with the water O, soft-core shifts)
-// are staged in shared memory once per block.  Q-atom gradients are reduced
-// per warp, then per block in shared memory (NQ_SHARED atoms at most; global
-// atomics beyond).
+// nonbond_qw_spc (md.f90:11302): Q atoms with the listed waters, all states in
+// the thread.  The Q atoms' parameters for the water sites (charge products in
+// single precision as crg_ow*qcrg, LJ products with the water types, soft-core
+// shifts) are static tables (QwAtom, QwState), staged with the Q atoms'
+// positions in shared memory QW_CHUNK Q atoms at a time.
 // With hydrogen LJ (nonbon2_qw, md.f90:9798; nonbond_qw_3atom, 11545) the two
 // hydrogen sites add LJ with their own type's parameters and soft-core shift.
-struct QwState { float qO, qH; double A, B, sc, AH, BH, scH; };
+//
+// Lanes are waters; the qg warps of a group of 32 waters share the Q atoms out
+// among them (warp u of a group takes Q atoms u, u + qg, ... of a chunk).  The
+// chain of one Q atom (reciprocal square roots, soft-core quotients, the warp
+// sum of its gradient) is about 2 us in FP64 and nothing in it is wide, so a
+// thread that walks all Q atoms of its water leaves one system bound by that
+// latency with the chip idle: one window (8 Q atoms, 1,035 waters) took 15 us
+// in FP64 with qg = 1 and takes 5.6 with qg = 8.  Batches that fill the chip with one warp per water group keep qg = 1
+// (Batch::qw_plan): their warps hide each other's latency, and the sharing only adds
+// the staging (41 windows FP64: 15 us with qg = 1, 18 with 2 and 4, 26 with 8;
+// 84 windows FP32: 23, 26, 31 and 50; with parameters derived per block from
+// the type tables instead of staged from the static ones, 18 and 27).
+// F32 (without hydrogen LJ): the mixed engine's steps that record no energies
+// take the forces alone in FP32, as its water-water kernel does.  A water's
+// FP32 sum runs over the Q atoms in order whatever qg is: with qg > 1 the
+// warps leave each (Q atom, water)'s three force factors in shared memory,
+// and the group's warps then sum one component each over the Q atoms, so the
+// result does not depend on the launch shape.
+constexpr int QW_MAXWARPS = 8, QW_CHUNK = 16;
 
-// F32 (with SHQ, without hydrogen LJ): the mixed engine's steps that record
-// no energies take the forces alone in FP32, as its water-water kernel does.
-template <int NSC, bool SHQ, bool HLJ, bool F32 = false>
-__global__ void __launch_bounds__(128, SHQ ? 4 : 1) k_nb_qw(DevPtrs P) {
+template <int NSC, bool HLJ, bool F32 = false>
+__global__ void __launch_bounds__(32 * QW_MAXWARPS, NSC > 0 ? 2 : 1) k_nb_qw(DevPtrs P, int qg) {
   constexpr int NA = NSC > 0 ? NSC : MAXS;
+  using R = typename std::conditional<F32, float, double>::type;
   const int2 tile = P.qw_tiles[blockIdx.x];   // (system, first list entry)
   const int s = tile.x;
   const SysDev &S = P.sys[s];
-  __shared__ double fq[NQ_SHARED * 3];
-  __shared__ double4 qx[NQ_SHARED];        // position; w: LJ code
-  __shared__ double2 qab[NQ_SHARED];       // A, B with the water O (same in every state)
-  __shared__ double2 qabH[NQ_SHARED];      // A, B with a water H (hydrogen LJ only)
-  __shared__ QwState qst[NQ_SHARED * NA];
-  if (S.nq == 0) return;
   const int n = P.st[s].qw_n;
   if (tile.y >= n) return;
-  const int NS = NSC > 0 ? NSC : S.S, ncol = S.natyps + S.nq;
+  __shared__ QwAtom sqa[QW_CHUNK];
+  __shared__ double4 sqx[QW_CHUNK];
+  __shared__ QwState sqs[QW_CHUNK * NA];
+  // F32: force factors [Q atom][site][warp's group of waters]; FP64: each warp's gradients
+  __shared__ R red[F32 ? QW_CHUNK * 3 * (QW_MAXWARPS / 2) * 32 : QW_MAXWARPS * 9 * 32];
+  __shared__ double ered[QW_MAXWARPS * 2 * NA];
+  const int NS = NSC > 0 ? NSC : S.S;
   const bool hlj = HLJ && S.hlj;           // this system's water hydrogens carry LJ
-  const bool shq = SHQ;                    // every system's Q atoms fit the shared tables
-  const int nqs = shq ? S.nq : 0;
-  for (int t = threadIdx.x; t < NQ_SHARED * 3; t += blockDim.x) fq[t] = 0;
-  for (int iq = threadIdx.x; iq < nqs; iq += blockDim.x) {
-    int gq = S.qoff + iq, i = P.iqseq[gq];
-    int lj = P.ljcod[S.ljoff + S.iac_ow * S.natyps + P.iac[i]];
-    int ljh = hlj ? P.ljcod[S.ljoff + S.iac_hw * S.natyps + P.iac[i]] : 1;
-    double4 x = P.x[i];
-    x.w = (double)(lj + 4 * ljh);
-    qx[iq] = x;
-    double A0, B0, AH0 = 0, BH0 = 0;
-    lj_pair(S.arith, P.lja[3 * i + lj - 1], S.aO[lj - 1], P.ljb[3 * i + lj - 1], S.bO[lj - 1], A0, B0);
-    if (hlj) lj_pair(S.arith, P.lja[3 * i + ljh - 1], S.aH[ljh - 1], P.ljb[3 * i + ljh - 1], S.bH[ljh - 1], AH0, BH0);
-    qab[iq] = make_double2(A0, B0);
-    qabH[iq] = make_double2(AH0, BH0);
-    for (int st = 0; st < NS; st++) {
-      QwState q;
-      float c = P.qcrg[gq * MAXS + st];
-      q.qO = S.crg_ow * c;
-      q.qH = S.crg_hw * c;
-      int ti = P.qiac[gq * MAXS + st];
-      lj_pair(S.arith, P.qavdw[S.qlib_off + 3 * ti], S.aO[lj - 1], P.qbvdw[S.qlib_off + 3 * ti], S.bO[lj - 1], q.A, q.B);
-      q.sc = S.qvdw ? P.sc[S.sc_off + ((size_t)iq * ncol + S.iac_ow) * NS + st] : 0.0;
-      q.AH = q.BH = q.scH = 0.0;
-      if (hlj) {
-        lj_pair(S.arith, P.qavdw[S.qlib_off + 3 * ti], S.aH[ljh - 1], P.qbvdw[S.qlib_off + 3 * ti], S.bH[ljh - 1], q.AH,
-                q.BH);
-        q.scH = S.qvdw ? P.sc[S.sc_off + ((size_t)iq * ncol + S.iac_hw) * NS + st] : 0.0;
-      }
-      qst[iq * NA + st] = q;
-    }
-  }
-  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int grp = warp / qg, sub = warp - grp * qg, ng = nw / qg;
   double el[NA], vdw[NA];
 #pragma unroll
   for (int st = 0; st < NA; st++) { el[st] = 0; vdw[st] = 0; }
-  const int k = tile.y + threadIdx.x;
+  const int k = tile.y + 32 * grp + lane;
   const bool act = k < n;
-  const int j = act ? P.qw[S.qw_off + k] : P.qw[S.qw_off];
+  const int j = P.qw[S.qw_off + (act ? k : tile.y)];
   double3 xO = ld3(P.x, j), xH1 = ld3(P.x, j + 1), xH2 = ld3(P.x, j + 2);
   if (S.pbc) {
     // nonbond_qw_spc_box (md.f90:11440-11446): the water at the image of its
@@ -1902,182 +1886,207 @@ __global__ void __launch_bounds__(128, SHQ ? 4 : 1) k_nb_qw(DevPtrs P) {
     xH1.x -= t.x; xH1.y -= t.y; xH1.z -= t.z;
     xH2.x -= t.x; xH2.y -= t.y; xH2.z -= t.z;
   }
-  double fw[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  float fw32[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int iq = 0; iq < S.nq; iq++) {
-    int gq = S.qoff + iq;
-    if (F32 && SHQ && !HLJ) {
-      // forces alone in FP32: differences of the FP64 positions rounded to
-      // FP32, MUFU reciprocal square roots, the states' sums in FP32
-      const double4 xi4 = qx[iq];
-      const float o[3] = {(float)(xO.x - xi4.x), (float)(xO.y - xi4.y), (float)(xO.z - xi4.z)};
-      const float h1[3] = {(float)(xH1.x - xi4.x), (float)(xH1.y - xi4.y), (float)(xH1.z - xi4.z)};
-      const float h2[3] = {(float)(xH2.x - xi4.x), (float)(xH2.y - xi4.y), (float)(xH2.z - xi4.z)};
-      const float r2O = fmaf(o[0], o[0], fmaf(o[1], o[1], o[2] * o[2]));
-      const float rO = rsqrt_ftz(r2O);
-      const float rH1 = rsqrt_ftz(fmaf(h1[0], h1[0], fmaf(h1[1], h1[1], h1[2] * h1[2])));
-      const float rH2 = rsqrt_ftz(fmaf(h2[0], h2[0], fmaf(h2[1], h2[1], h2[2] * h2[2])));
-      const float r2Oi = rO * rO, r2H1 = rH1 * rH1, r2H2 = rH2 * rH2;
-      const float r6hc = r2O * r2O * r2O;
-      float Va0 = 0.f, Vb0 = 0.f;
-      if (!S.qvdw) {
-        const float r6 = r2Oi * r2Oi * r2Oi;
-        Va0 = (float)qab[iq].x * r6 * r6;
-        Vb0 = (float)qab[iq].y * r6;
-      }
-      float dvO = 0.f, dvH1 = 0.f, dvH2 = 0.f;
-#pragma unroll
-      for (int st = 0; st < NA; st++) {
-        if (st >= NS) break;
-        const QwState q = qst[iq * NA + st];
-        float Va = Va0, Vb = Vb0, fsc = 1.f;
-        if (S.qvdw) {
-          const float inv = 1.f / (r6hc + (float)q.sc);
-          Va = (float)q.A * inv * inv;
-          Vb = (float)q.B * inv;
-          fsc = r6hc * inv;
+  R fw[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int q0 = 0; q0 < S.nq; q0 += QW_CHUNK) {
+    const int qn = min(QW_CHUNK, S.nq - q0);
+    __syncthreads();
+    for (int t = threadIdx.x; t < qn; t += blockDim.x) {
+      const QwAtom A = P.qwa[S.qoff + q0 + t];
+      sqa[t] = A;
+      sqx[t] = P.x[A.atom];
+    }
+    for (int t = threadIdx.x; t < qn * NS; t += blockDim.x)
+      sqs[t / NS * NA + t % NS] = P.qws[(size_t)(S.qoff + q0 + t / NS) * MAXS + t % NS];
+    __syncthreads();
+    for (int iq = sub; iq < qn; iq += qg) {
+      const QwAtom &QA = sqa[iq];
+      const double4 xi = sqx[iq];
+      const QwState *qst = sqs + iq * NA;
+      R qacc[3];
+      if (F32) {
+        // differences of the FP64 positions rounded to FP32, MUFU reciprocal
+        // square roots, the states' sums in FP32
+        const float o[3] = {(float)(xO.x - xi.x), (float)(xO.y - xi.y), (float)(xO.z - xi.z)};
+        const float h1[3] = {(float)(xH1.x - xi.x), (float)(xH1.y - xi.y), (float)(xH1.z - xi.z)};
+        const float h2[3] = {(float)(xH2.x - xi.x), (float)(xH2.y - xi.y), (float)(xH2.z - xi.z)};
+        const float r2O = fmaf(o[0], o[0], fmaf(o[1], o[1], o[2] * o[2]));
+        const float rO = rsqrt_ftz(r2O);
+        const float rH1 = rsqrt_ftz(fmaf(h1[0], h1[0], fmaf(h1[1], h1[1], h1[2] * h1[2])));
+        const float rH2 = rsqrt_ftz(fmaf(h2[0], h2[0], fmaf(h2[1], h2[1], h2[2] * h2[2])));
+        const float r2Oi = rO * rO, r2H1 = rH1 * rH1, r2H2 = rH2 * rH2;
+        const float r6hc = r2O * r2O * r2O;
+        float Va0 = 0.f, Vb0 = 0.f;
+        if (!S.qvdw) {
+          const float r6 = r2Oi * r2Oi * r2Oi;
+          Va0 = (float)QA.A * r6 * r6;
+          Vb0 = (float)QA.B * r6;
         }
-        const float lam = (float)S.lambda[st];
-        dvO += r2Oi * (-q.qO * rO - (12.f * Va - 6.f * Vb) * fsc) * lam;
-        dvH1 -= r2H1 * (q.qH * rH1) * lam;
-        dvH2 -= r2H2 * (q.qH * rH2) * lam;
-      }
+        float dvO = 0.f, dvH1 = 0.f, dvH2 = 0.f;
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const float qa = act ? -(dvO * o[c] + dvH1 * h1[c] + dvH2 * h2[c]) : 0.f;
-        fw32[c] = fmaf(dvO, o[c], fw32[c]);
-        fw32[3 + c] = fmaf(dvH1, h1[c], fw32[3 + c]);
-        fw32[6 + c] = fmaf(dvH2, h2[c], fw32[6 + c]);
-        const float t = warp_sumf(qa);
-        if ((threadIdx.x & 31) == 0 && t != 0.f) atomicAdd(&fq[3 * iq + c], (double)t);
-      }
-      continue;
-    }
-    double4 xi4;
-    int lj, ljh;
-    double A0, B0, AH0 = 0, BH0 = 0;
-    if (shq) {
-      xi4 = qx[iq];
-      lj = (int)xi4.w & 3;
-      ljh = (int)xi4.w >> 2;
-      A0 = qab[iq].x; B0 = qab[iq].y;
-      AH0 = qabH[iq].x; BH0 = qabH[iq].y;
-    } else {
-      int i = P.iqseq[gq];
-      xi4 = P.x[i];
-      lj = P.ljcod[S.ljoff + S.iac_ow * S.natyps + P.iac[i]];
-      ljh = hlj ? P.ljcod[S.ljoff + S.iac_hw * S.natyps + P.iac[i]] : 1;
-      lj_pair(S.arith, P.lja[3 * i + lj - 1], S.aO[lj - 1], P.ljb[3 * i + lj - 1], S.bO[lj - 1], A0, B0);
-      if (hlj)
-        lj_pair(S.arith, P.lja[3 * i + ljh - 1], S.aH[ljh - 1], P.ljb[3 * i + ljh - 1], S.bH[ljh - 1], AH0, BH0);
-    }
-    double dO[3] = {xO.x - xi4.x, xO.y - xi4.y, xO.z - xi4.z};
-    double dH1[3] = {xH1.x - xi4.x, xH1.y - xi4.y, xH1.z - xi4.z};
-    double dH2[3] = {xH2.x - xi4.x, xH2.y - xi4.y, xH2.z - xi4.z};
-    double r2O = dO[0] * dO[0] + dO[1] * dO[1] + dO[2] * dO[2];
-    double rH1 = rsqrt(dH1[0] * dH1[0] + dH1[1] * dH1[1] + dH1[2] * dH1[2]);
-    double rH2 = rsqrt(dH2[0] * dH2[0] + dH2[1] * dH2[1] + dH2[2] * dH2[2]);
-    double r6hc = r2O * r2O * r2O;
-    double rO = rsqrt(r2O);
-    r2O = rO * rO;
-    double r2H1 = rH1 * rH1, r2H2 = rH2 * rH2;
-    double dvO = 0, dvH1 = 0, dvH2 = 0, Va = 0, Vb = 0;
-    if (!S.qvdw) {
-      double r6O = 1. / r6hc;
-      Va = A0 * r6O * r6O;
-      Vb = B0 * r6O;
-    }
-    // hydrogen sites: d^6 and the hard-core LJ terms (state independent without qvdw)
-    double d6H1 = 0, d6H2 = 0, VaH1 = 0, VbH1 = 0, VaH2 = 0, VbH2 = 0;
-    if (hlj) {
-      double r6H1 = r2H1 * r2H1 * r2H1, r6H2 = r2H2 * r2H2 * r2H2;
-      d6H1 = 1. / r6H1; d6H2 = 1. / r6H2;
-      if (!S.qvdw) {
-        VaH1 = AH0 * r6H1 * r6H1; VbH1 = BH0 * r6H1;
-        VaH2 = AH0 * r6H2 * r6H2; VbH2 = BH0 * r6H2;
-      }
-    }
+        for (int st = 0; st < NA; st++) {
+          if (st >= NS) break;
+          const QwState &q = qst[st];
+          float Va = Va0, Vb = Vb0, fsc = 1.f;
+          if (S.qvdw) {
+            const float inv = 1.f / (r6hc + (float)q.sc);
+            Va = (float)q.A * inv * inv;
+            Vb = (float)q.B * inv;
+            fsc = r6hc * inv;
+          }
+          const float lam = (float)S.lambda[st];
+          dvO += r2Oi * (-q.qO * rO - (12.f * Va - 6.f * Vb) * fsc) * lam;
+          dvH1 -= r2H1 * (q.qH * rH1) * lam;
+          dvH2 -= r2H2 * (q.qH * rH2) * lam;
+        }
+        if (qg > 1) {
+          R *f = red + ((size_t)iq * 3 * ng + grp) * 32 + lane;
+          f[0] = dvO;
+          f[ng * 32] = dvH1;
+          f[2 * ng * 32] = dvH2;
+        }
 #pragma unroll
-    for (int st = 0; st < NA; st++) {
-      if (st >= NS) break;
-      QwState q;
-      if (shq) q = qst[iq * NA + st];
-      else {
-        float c = P.qcrg[gq * MAXS + st];
-        q.qO = S.crg_ow * c; q.qH = S.crg_hw * c;
-        int ti = P.qiac[gq * MAXS + st];
-        lj_pair(S.arith, P.qavdw[S.qlib_off + 3 * ti], S.aO[lj - 1], P.qbvdw[S.qlib_off + 3 * ti], S.bO[lj - 1], q.A,
-                q.B);
-        q.sc = S.qvdw ? P.sc[S.sc_off + ((size_t)iq * ncol + S.iac_ow) * NS + st] : 0.0;
-        q.AH = q.BH = q.scH = 0.0;
-        if (hlj) {
-          lj_pair(S.arith, P.qavdw[S.qlib_off + 3 * ti], S.aH[ljh - 1], P.qbvdw[S.qlib_off + 3 * ti], S.bH[ljh - 1],
-                  q.AH, q.BH);
-          q.scH = S.qvdw ? P.sc[S.sc_off + ((size_t)iq * ncol + S.iac_hw) * NS + st] : 0.0;
+        for (int c = 0; c < 3; c++) {
+          qacc[c] = act ? -(dvO * o[c] + dvH1 * h1[c] + dvH2 * h2[c]) : 0.f;
+          if (qg == 1) {
+            fw[c] = fmaf(dvO, o[c], (float)fw[c]);
+            fw[3 + c] = fmaf(dvH1, h1[c], (float)fw[3 + c]);
+            fw[6 + c] = fmaf(dvH2, h2[c], (float)fw[6 + c]);
+          }
+          qacc[c] = warp_sumf((float)qacc[c]);
         }
-      }
-      double r6sc = r6hc;
-      if (S.qvdw) {
-        r6sc = r6hc + q.sc;
-        Va = q.A / (r6sc * r6sc);
-        Vb = q.B / r6sc;
-      }
-      double VelO = (double)q.qO * rO;
-      double VelH1 = (double)q.qH * rH1;
-      double VelH2 = (double)q.qH * rH2;
-      double lam = S.lambda[st];
-      dvO += r2O * (-VelO - ((12. * Va - 6. * Vb) * (r6hc / r6sc))) * lam;
-      if (hlj) {
-        double f1 = 1.0, f2 = 1.0;
-        if (S.qvdw) {
-          double s1 = d6H1 + q.scH, s2 = d6H2 + q.scH;
-          VaH1 = q.AH / (s1 * s1); VbH1 = q.BH / s1;
-          VaH2 = q.AH / (s2 * s2); VbH2 = q.BH / s2;
-          f1 = d6H1 / s1; f2 = d6H2 / s2;
-        }
-        dvH1 += r2H1 * (-VelH1 - (12. * VaH1 - 6. * VbH1) * f1) * lam;
-        dvH2 += r2H2 * (-VelH2 - (12. * VaH2 - 6. * VbH2) * f2) * lam;
-        if (act) vdw[st] += VaH1 + VaH2 - VbH1 - VbH2;
       } else {
-        dvH1 -= r2H1 * VelH1 * lam;
-        dvH2 -= r2H2 * VelH2 * lam;
-      }
-      if (act) {
-        el[st] += VelO + VelH1 + VelH2;
-        vdw[st] += Va - Vb;
-      }
-    }
-    double qacc[3];
+        double dO[3] = {xO.x - xi.x, xO.y - xi.y, xO.z - xi.z};
+        double dH1[3] = {xH1.x - xi.x, xH1.y - xi.y, xH1.z - xi.z};
+        double dH2[3] = {xH2.x - xi.x, xH2.y - xi.y, xH2.z - xi.z};
+        double r2O = dO[0] * dO[0] + dO[1] * dO[1] + dO[2] * dO[2];
+        double rH1 = rsqrt(dH1[0] * dH1[0] + dH1[1] * dH1[1] + dH1[2] * dH1[2]);
+        double rH2 = rsqrt(dH2[0] * dH2[0] + dH2[1] * dH2[1] + dH2[2] * dH2[2]);
+        double r6hc = r2O * r2O * r2O;
+        double rO = rsqrt(r2O);
+        r2O = rO * rO;
+        double r2H1 = rH1 * rH1, r2H2 = rH2 * rH2;
+        double dvO = 0, dvH1 = 0, dvH2 = 0, Va = 0, Vb = 0;
+        if (!S.qvdw) {
+          double r6O = 1. / r6hc;
+          Va = QA.A * r6O * r6O;
+          Vb = QA.B * r6O;
+        }
+        // hydrogen sites: d^6 and the hard-core LJ terms (state independent without qvdw)
+        double d6H1 = 0, d6H2 = 0, VaH1 = 0, VbH1 = 0, VaH2 = 0, VbH2 = 0;
+        if (hlj) {
+          double r6H1 = r2H1 * r2H1 * r2H1, r6H2 = r2H2 * r2H2 * r2H2;
+          d6H1 = 1. / r6H1; d6H2 = 1. / r6H2;
+          if (!S.qvdw) {
+            VaH1 = QA.AH * r6H1 * r6H1; VbH1 = QA.BH * r6H1;
+            VaH2 = QA.AH * r6H2 * r6H2; VbH2 = QA.BH * r6H2;
+          }
+        }
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      qacc[c] = act ? -(dvO * dO[c] + dvH1 * dH1[c] + dvH2 * dH2[c]) : 0.0;
-      fw[c] += dvO * dO[c];
-      fw[3 + c] += dvH1 * dH1[c];
-      fw[6 + c] += dvH2 * dH2[c];
-    }
-    // Q-atom gradient: warp reduction, then one shared (or global) atomic per warp
+        for (int st = 0; st < NA; st++) {
+          if (st >= NS) break;
+          const QwState &q = qst[st];
+          double r6sc = r6hc;
+          if (S.qvdw) {
+            r6sc = r6hc + q.sc;
+            Va = q.A / (r6sc * r6sc);
+            Vb = q.B / r6sc;
+          }
+          double VelO = (double)q.qO * rO;
+          double VelH1 = (double)q.qH * rH1;
+          double VelH2 = (double)q.qH * rH2;
+          double lam = S.lambda[st];
+          dvO += r2O * (-VelO - ((12. * Va - 6. * Vb) * (r6hc / r6sc))) * lam;
+          if (hlj) {
+            double f1 = 1.0, f2 = 1.0;
+            if (S.qvdw) {
+              double s1 = d6H1 + q.scH, s2 = d6H2 + q.scH;
+              VaH1 = q.AH / (s1 * s1); VbH1 = q.BH / s1;
+              VaH2 = q.AH / (s2 * s2); VbH2 = q.BH / s2;
+              f1 = d6H1 / s1; f2 = d6H2 / s2;
+            }
+            dvH1 += r2H1 * (-VelH1 - (12. * VaH1 - 6. * VbH1) * f1) * lam;
+            dvH2 += r2H2 * (-VelH2 - (12. * VaH2 - 6. * VbH2) * f2) * lam;
+            if (act) vdw[st] += VaH1 + VaH2 - VbH1 - VbH2;
+          } else {
+            dvH1 -= r2H1 * VelH1 * lam;
+            dvH2 -= r2H2 * VelH2 * lam;
+          }
+          if (act) {
+            el[st] += VelO + VelH1 + VelH2;
+            vdw[st] += Va - Vb;
+          }
+        }
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      double t = warp_sum(qacc[c]);
-      if ((threadIdx.x & 31) == 0 && t != 0.0) {
-        if (shq) atomicAdd(&fq[3 * iq + c], t);
-        else atomicAdd(&P.d[P.iqseq[gq]].x + c, t);
+        for (int c = 0; c < 3; c++) {
+          qacc[c] = act ? -(dvO * dO[c] + dvH1 * dH1[c] + dvH2 * dH2[c]) : 0.0;
+          fw[c] += dvO * dO[c];
+          fw[3 + c] += dvH1 * dH1[c];
+          fw[6 + c] += dvH2 * dH2[c];
+          qacc[c] = warp_sum(qacc[c]);
+        }
+      }
+      // the Q atom's gradient from this warp's waters: lane c adds component c
+      const double t = lane == 0 ? (double)qacc[0] : lane == 1 ? (double)qacc[1] : (double)qacc[2];
+      if (lane < 3 && t != 0.0) atomicAdd(&P.d[QA.atom].x + lane, t);
+    }
+    if (F32 && qg > 1) {
+      // component c of the group's waters by warp c % qg, Q atoms in order
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < 5; u++) {
+        const int c = sub + u * qg;
+        if (c >= 9) break;
+        const int a = c / 3, e = c - 3 * a;
+        const double xc = a == 0 ? (e == 0 ? xO.x : e == 1 ? xO.y : xO.z)
+                          : a == 1 ? (e == 0 ? xH1.x : e == 1 ? xH1.y : xH1.z)
+                                   : (e == 0 ? xH2.x : e == 1 ? xH2.y : xH2.z);
+        const double *qx = &sqx[0].x + e;
+        const R *f = red + ((size_t)a * ng + grp) * 32 + lane;
+        for (int iq = 0; iq < qn; iq++)
+          fw[u] = fmaf((float)f[(size_t)iq * 3 * ng * 32], (float)(xc - qx[4 * iq]), (float)fw[u]);
       }
     }
   }
-  if (F32 && SHQ && !HLJ)
+  if (F32) {
+    if (qg == 1) {
+      if (act)
+        for (int a = 0; a < 3; a++) atomic_add3(P.d, j + a, (double)fw[3 * a], (double)fw[3 * a + 1], (double)fw[3 * a + 2]);
+    } else if (act) {
 #pragma unroll
-    for (int c = 0; c < 9; c++) fw[c] = (double)fw32[c];
-  if (act)
-    for (int a = 0; a < 3; a++) atomic_add3(P.d, j + a, fw[3 * a], fw[3 * a + 1], fw[3 * a + 2]);
-  if (!(F32 && SHQ && !HLJ))
-    for (int st = 0; st < NS; st++) {
-      warp_add(&P.EQ[((size_t)s * MAXS + st) * QB_NEQ + QB_EQ_QW_EL], el[st]);
-      warp_add(&P.EQ[((size_t)s * MAXS + st) * QB_NEQ + QB_EQ_QW_VDW], vdw[st]);
+      for (int u = 0; u < 5; u++) {
+        const int c = sub + u * qg;
+        if (c < 9) atomicAdd(&P.d[j + c / 3].x + c % 3, (double)fw[u]);
+      }
     }
+    return;
+  }
+  // FP64: the waters' gradients summed over each group's warps, the energies over the block
+  if (qg == 1) {
+    if (act)
+      for (int a = 0; a < 3; a++) atomic_add3(P.d, j + a, (double)fw[3 * a], (double)fw[3 * a + 1], (double)fw[3 * a + 2]);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 9; c++) red[F32 ? 0 : (warp * 9 + c) * 32 + lane] = fw[c];
+  }
+#pragma unroll
+  for (int st = 0; st < NA; st++) {
+    if (st >= NS) break;
+    const double a = warp_sum(el[st]), b = warp_sum(vdw[st]);
+    if (lane == 0) { ered[(warp * NA + st) * 2] = a; ered[(warp * NA + st) * 2 + 1] = b; }
+  }
   __syncthreads();
-  for (int t = threadIdx.x; t < nqs * 3; t += blockDim.x)
-    if (fq[t] != 0.0) atomicAdd(&P.d[P.iqseq[S.qoff + t / 3]].x + (t % 3), fq[t]);
+  if (qg > 1 && act)
+    for (int c = sub; c < 9; c += qg) {
+      double f = 0.0;
+      for (int u = 0; u < qg; u++) f += (double)red[F32 ? 0 : ((grp * qg + u) * 9 + c) * 32 + lane];
+      atomicAdd(&P.d[j + c / 3].x + c % 3, f);
+    }
+  if ((int)threadIdx.x < 2 * NS) {
+    const int st = threadIdx.x >> 1, c = threadIdx.x & 1;
+    double e = 0.0;
+    for (int w = 0; w < nw; w++) e += ered[(w * NA + st) * 2 + c];
+    atomicAdd(&P.EQ[((size_t)s * MAXS + st) * QB_NEQ + (c ? QB_EQ_QW_VDW : QB_EQ_QW_EL)], e);
+  }
 }
 
 // nonbond_qq (md.f90:10763): Q-Q and Q-to-bonded-neighbour pairs, all states.
