@@ -125,7 +125,6 @@ struct Batch {
     qw_warps = std::max(4, qw_groups);
   }
   int q_states = 0;           // state count shared by every system with Q atoms (0: they differ)
-  int max_nq = 0;
   // profiling
   bool profiling = false;
   std::vector<std::pair<std::string, std::pair<cudaEvent_t, cudaEvent_t>>> pending;
@@ -317,8 +316,6 @@ struct Batch {
     const bool fast_ww = mixed && !ene;
     // the water pass stores every water gradient and zeroes the solute's
     if (!water_pass_zeroes) CUDA_TRY(cudaMemsetAsync(p.d, 0, sizeof(double4) * (size_t)p.natoms_tot, stream));
-    CUDA_TRY(cudaMemsetAsync(p.E, 0, sizeof(double) * QB_NE * (size_t)nsys, stream));
-    CUDA_TRY(cudaMemsetAsync(p.EQ, 0, sizeof(double) * MAXS * QB_NEQ * (size_t)nsys, stream));
     // waters first: their records, and their per-atom terms as the first
     // gradient contribution (plain stores after the zeroing)
     if (max_nwat > 0) {
@@ -579,8 +576,8 @@ struct Batch {
     check_launch("energy sums");
     E.resize((size_t)nsys * QB_NE);
     EQ.resize((size_t)nsys * MAXS * QB_NEQ);
-    CUDA_TRY(cudaMemcpyAsync(E.data(), P.E, sizeof(double) * E.size(), cudaMemcpyDeviceToHost, stream));
-    CUDA_TRY(cudaMemcpyAsync(EQ.data(), P.EQ, sizeof(double) * EQ.size(), cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaMemcpyAsync(E.data(), P.Eo, sizeof(double) * E.size(), cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaMemcpyAsync(EQ.data(), P.EQo, sizeof(double) * EQ.size(), cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaStreamSynchronize(stream));
   }
 
@@ -608,8 +605,8 @@ struct Batch {
     // the step's energies: bonded terms of the totals, and what every other
     // system keeps
     std::vector<double> E0((size_t)nsys * QB_NE), EQ0((size_t)nsys * MAXS * QB_NEQ);
-    CUDA_TRY(cudaMemcpyAsync(E0.data(), P.E, sizeof(double) * E0.size(), cudaMemcpyDeviceToHost, stream));
-    CUDA_TRY(cudaMemcpyAsync(EQ0.data(), P.EQ, sizeof(double) * EQ0.size(), cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaMemcpyAsync(E0.data(), P.Eo, sizeof(double) * E0.size(), cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaMemcpyAsync(EQ0.data(), P.EQo, sizeof(double) * EQ0.size(), cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaStreamSynchronize(stream));
     std::vector<int> live;
     for (int s : M)
@@ -726,8 +723,8 @@ struct Batch {
       }
     }
     // every system's E and EQ as the step (and the moves) left them
-    CUDA_TRY(cudaMemcpyAsync(P.E, Efin.data(), sizeof(double) * Efin.size(), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(P.EQ, EQfin.data(), sizeof(double) * EQfin.size(), cudaMemcpyHostToDevice, stream));
+    CUDA_TRY(cudaMemcpyAsync(P.Eo, Efin.data(), sizeof(double) * Efin.size(), cudaMemcpyHostToDevice, stream));
+    CUDA_TRY(cudaMemcpyAsync(P.EQo, EQfin.data(), sizeof(double) * EQfin.size(), cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaStreamSynchronize(stream));   // the host vectors are the copies' sources
   }
   double4 *mc_x = nullptr;
@@ -1256,7 +1253,6 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     B.any_lrf |= V.use_LRF != 0;
     if (V.nqat > 0) B.q_states = (!B.any_q || B.q_states == V.nstates) ? V.nstates : 0;
     B.any_q |= V.nqat > 0;
-    B.max_nq = std::max(B.max_nq, V.nqat);
     B.any_shake |= V.shake_constraints > 0;
     B.any_wpol |= S.wpol != 0;
     B.any_prestr |= (V.nrstr_seq + V.nrstr_pos + V.nrstr_dist + V.nrstr_angl + V.nrstr_wall) > 0;
@@ -1512,7 +1508,9 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   P.kin_nblk = std::max(1, (B.max_natom + KIN_BLOCK - 1) / KIN_BLOCK);
   P.kin = dev_alloc<double>((size_t)n * 4, o);
   P.E = dev_alloc<double>((size_t)n * QB_NE, o);
+  P.Eo = dev_alloc<double>((size_t)n * QB_NE, o);
   P.EQ = dev_alloc<double>((size_t)n * MAXS * QB_NEQ, o);
+  P.EQo = dev_alloc<double>((size_t)n * MAXS * QB_NEQ, o);
   P.offd_r = dev_alloc<double>((size_t)n * MAXS, o);
   P.hist = nullptr;
   P.hist_cap = 0;
@@ -1907,9 +1905,9 @@ int qb_batch_energies(qb_batch *bb, int sys, double *E_out, double *EQ_out) {
   return guarded_batch([&] {
     Batch &B = bb->b;
     CUDA_TRY(cudaStreamSynchronize(B.stream));
-    if (E_out) CUDA_TRY(cudaMemcpy(E_out, B.P.E + (size_t)sys * QB_NE, sizeof(double) * QB_NE, cudaMemcpyDeviceToHost));
+    if (E_out) CUDA_TRY(cudaMemcpy(E_out, B.P.Eo + (size_t)sys * QB_NE, sizeof(double) * QB_NE, cudaMemcpyDeviceToHost));
     if (EQ_out && B.sysh[sys].S > 0)
-      CUDA_TRY(cudaMemcpy(EQ_out, B.P.EQ + (size_t)sys * qb::MAXS * QB_NEQ, sizeof(double) * QB_NEQ * B.sysh[sys].S,
+      CUDA_TRY(cudaMemcpy(EQ_out, B.P.EQo + (size_t)sys * qb::MAXS * QB_NEQ, sizeof(double) * QB_NEQ * B.sysh[sys].S,
                           cudaMemcpyDeviceToHost));
   });
 }

@@ -214,8 +214,10 @@ struct DevPtrs {
   // energies
   double *kin;                             // [s*4] kinetic energy of this step: solute all, free, solvent all, free
   int kin_nblk;
-  double *E;                               // [s*QB_NE]
-  double *EQ;                              // [(s*MAXS + st)*QB_NEQ]
+  // energy terms: accumulators of the evaluation under way (k_finish reads
+  // and zeroes them) and the results of the last one
+  double *E, *Eo;                          // [s*QB_NE]
+  double *EQ, *EQo;                        // [(s*MAXS + st)*QB_NEQ]
   double *offd_r;                          // [s*MAXS + io] r_kl of this step's off-diagonal functions
   // history [kind][s][rec][QB_NE + MAXS*QB_NEQ + 1]
   double *hist;

@@ -3345,27 +3345,31 @@ __global__ void __launch_bounds__(KIN_BLOCK) k_kinetic(DevPtrs P) {
 // pot_energy's sums (md.f90:13500-13560): per-state Q totals, the
 // lambda-weighted Q terms and the potential.  Lane st handles state st (its
 // row loaded at once); lane 0 then adds the states in order and forms the
-// totals from one load of the system's energy terms.
+// totals from one load of the system's energy terms.  The terms' accumulators
+// (P.E, P.EQ) are read and zeroed for the next evaluation here, the results
+// kept in P.Eo, P.EQo: two memset nodes less at the head of every step (they
+// were 2 to 3 us of a single system's 63).
 __device__ __forceinline__ void finalize_energy(DevPtrs &P, int s) {
   const SysDev &S = P.sys[s];
   const int lane = threadIdx.x;
-  double *E = P.E + s * QB_NE;
+  double *E = P.E + s * QB_NE, *Eo = P.Eo + s * QB_NE;
   double w[7] = {0, 0, 0, 0, 0, 0, 0};   // this state's bond, angle, torsion, improper, qx_el, qx_vdw, restraint, x lambda
   if (lane < S.S) {
     double *q = P.EQ + ((size_t)s * MAXS + lane) * QB_NEQ;
+    double *qo = P.EQo + ((size_t)s * MAXS + lane) * QB_NEQ;
     double r[QB_NEQ];
 #pragma unroll
     for (int k = 0; k < QB_NEQ; k++) r[k] = q[k];
+#pragma unroll
+    for (int k = 0; k < QB_NEQ; k++) q[k] = 0.0;
     const double lam = S.lambda[lane];
     r[QB_EQ_LAMBDA] = lam;
     r[QB_EQ_QX_EL] = r[QB_EQ_QQ_EL] + r[QB_EQ_QP_EL] + r[QB_EQ_QW_EL];
     r[QB_EQ_QX_VDW] = r[QB_EQ_QQ_VDW] + r[QB_EQ_QP_VDW] + r[QB_EQ_QW_VDW];
     r[QB_EQ_TOTAL] = r[QB_EQ_BOND] + r[QB_EQ_ANGLE] + r[QB_EQ_TORSION] + r[QB_EQ_IMPROPER] + r[QB_EQ_QX_EL] +
                      r[QB_EQ_QX_VDW] + r[QB_EQ_RESTRAINT];
-    q[QB_EQ_LAMBDA] = r[QB_EQ_LAMBDA];
-    q[QB_EQ_QX_EL] = r[QB_EQ_QX_EL];
-    q[QB_EQ_QX_VDW] = r[QB_EQ_QX_VDW];
-    q[QB_EQ_TOTAL] = r[QB_EQ_TOTAL];
+#pragma unroll
+    for (int k = 0; k < QB_NEQ; k++) qo[k] = r[k];
     w[0] = r[QB_EQ_BOND] * lam; w[1] = r[QB_EQ_ANGLE] * lam; w[2] = r[QB_EQ_TORSION] * lam;
     w[3] = r[QB_EQ_IMPROPER] * lam; w[4] = r[QB_EQ_QX_EL] * lam; w[5] = r[QB_EQ_QX_VDW] * lam;
     w[6] = r[QB_EQ_RESTRAINT] * lam;
@@ -3374,6 +3378,8 @@ __device__ __forceinline__ void finalize_energy(DevPtrs &P, int s) {
   if (lane == 0) {
 #pragma unroll
     for (int k = 0; k < QB_NE; k++) e[k] = E[k];
+#pragma unroll
+    for (int k = 0; k < QB_NE; k++) E[k] = 0.0;
   }
   for (int k = 0; k < S.S; k++) {
     double v[7];
@@ -3393,7 +3399,7 @@ __device__ __forceinline__ void finalize_energy(DevPtrs &P, int s) {
                         e[QB_E_Q_IMPROPER] + e[QB_E_QX_EL] + e[QB_E_QX_VDW] + e[QB_E_RST_TOTAL] + e[QB_E_LRF];
     e[QB_E_KINETIC] = P.st[s].kinetic;
 #pragma unroll
-    for (int k = 0; k < QB_NE; k++) E[k] = e[k];
+    for (int k = 0; k < QB_NE; k++) Eo[k] = e[k];
     if (!isfinite(e[QB_E_POTENTIAL])) set_status(&P.st[s], QB_ERR_NAN);
   }
   __syncwarp();
@@ -3448,7 +3454,7 @@ __global__ void k_finish(DevPtrs P, int mode) {
     st.Tfree = Tfree;
     st.Tfree_sol = Tfree_sol;
     st.Tfree_solv = Tfree_solv;
-    if (mode == 1) P.E[s * QB_NE + QB_E_KINETIC] = st.kinetic;
+    if (mode == 1) P.Eo[s * QB_NE + QB_E_KINETIC] = st.kinetic;
   }
   __syncwarp();
   if (mode == 1) {
@@ -3465,8 +3471,8 @@ __global__ void k_finish(DevPtrs P, int mode) {
         double *r = hr.hist + (((size_t)kind * P.nsys + s) * hr.cap + c) * rec_len;
         for (int k = lane; k < rec_len; k += 32)
           r[k] = k == 0 ? (double)is
-                 : k <= QB_NE ? P.E[s * QB_NE + k - 1]
-                 : k <= QB_NE + MAXS * QB_NEQ ? P.EQ[(size_t)s * MAXS * QB_NEQ + k - 1 - QB_NE]
+                 : k <= QB_NE ? P.Eo[s * QB_NE + k - 1]
+                 : k <= QB_NE + MAXS * QB_NEQ ? P.EQo[(size_t)s * MAXS * QB_NEQ + k - 1 - QB_NE]
                                               : P.offd_r[s * MAXS + k - 1 - QB_NE - MAXS * QB_NEQ];
       }
       __syncwarp();
