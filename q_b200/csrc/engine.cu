@@ -84,7 +84,7 @@ struct Batch {
   cudaStream_t stream = nullptr;
   int NB = 1;
   long long istep = 0;
-  int max_natom = 0, max_lrf_blocks = 1, max_nsol = 0, max_nwat = 0, max_ncgp = 0, max_ncgp_sol = 0, max_terms = 0, max_pp = 0, max_ncgp_sol_w = 0, max_qp = 0;
+  int max_natom = 0, max_lrf_blocks = 1, max_nsol = 0, max_nwat = 0, max_ncgp = 0, max_ncgp_sol = 0, max_terms = 0, max_ncgp_sol_w = 0, max_qp = 0;
   bool any_any_atom = false;   // a system with any-atom charge-group cut-offs (iuse_switch_atom 0)
   // periodic box: any system in a box, putting molecules back, at constant pressure
   bool any_box = false, any_put = false, any_npt = false;
@@ -221,23 +221,34 @@ struct Batch {
     // tests read them
     if (any_lrf || any_any_atom)
       launch("cgp_centers", [&] { k_cgp_centers<<<cdiv(p.ncgp_tot, 256), b256, 0, stream>>>(p, force); });
+    auto solute_lists = [&] {
+      if (max_ncgp_sol == 0) return;
+      launch("group_near", [&] { k_group_near<<<dim3(max_ncgp_sol, nsys), 128, 0, stream>>>(p, force); });
+      if (max_nwat > 0) launch("list_pw", [&] { k_list_pw<<<dim3(cdiv(max_ncgp_sol, 4), nsys), 128, 0, stream>>>(p, force); });
+    };
+    // the any-atom LRF windows read the group-pair bits
+    if (any_any_atom) solute_lists();
     fork_streams();
     if (any_lrf) {
       launch("lrf_gather", [&] {
-        if (opt.precision == QB_MIXED && any_box)
-          k_lrf_gather_x2<true><<<dim3(max_lrfx_blocks, nsys), LRFX_BLOCK, 0, s1>>>(p, force);
-        else if (opt.precision == QB_MIXED)
-          k_lrf_gather_x2<false><<<dim3(max_lrfx_blocks, nsys), LRFX_BLOCK, 0, s1>>>(p, force);
-        else
-          k_lrf_gather<false><<<dim3(max_lrf_blocks, nsys), LRF_BLOCK, 0, s1>>>(p, force);
+        const dim3 gx(max_lrfx_blocks, nsys);
+        if (opt.precision == QB_MIXED) {
+          if (any_box && any_any_atom) k_lrf_gather_x2<true, true><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
+          else if (any_box) k_lrf_gather_x2<true, false><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
+          else if (any_any_atom) k_lrf_gather_x2<false, true><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
+          else k_lrf_gather_x2<false, false><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
+        } else {
+          const dim3 g(max_lrf_blocks, nsys);
+          if (any_any_atom) k_lrf_gather<false, true><<<g, LRF_BLOCK, 0, s1>>>(p, force);
+          else k_lrf_gather<false, false><<<g, LRF_BLOCK, 0, s1>>>(p, force);
+        }
       });
     }
     if (max_nwat > 0)
       launch("list_ww", [&] { k_list_ww<<<dim3(cdiv(max_nwat, WL_WPB), nsys), WL_BLOCK, 0, s2>>>(p, force); });
-    if (max_ncgp_sol > 0) {
-      launch("list_pp", [&] { k_list_pp<<<dim3(max_ncgp_sol, nsys), 128, 0, stream>>>(p, force); });
-      if (max_nwat > 0) launch("list_pw", [&] { k_list_pw<<<dim3(cdiv(max_ncgp_sol, 4), nsys), 128, 0, stream>>>(p, force); });
-    }
+    if (!any_any_atom) solute_lists();
+    if (max_nsol > 0)
+      launch("list_pp", [&] { k_list_pp<<<dim3(cdiv(max_nsol, PP_BLOCK / 32), nsys), PP_BLOCK, 0, stream>>>(p, force); });
     // a volume move rebuilds the LRF and the solute and water lists, not the
     // Q-atom lists (md.f90:15734-15744)
     if (any_q && force != 2) {
@@ -338,7 +349,7 @@ struct Batch {
       // pair blocks per system: enough for a large solute to fill the SMs
       // when the batch is small (1184 = 8 blocks per SM over the batch)
       const int cap = std::max(8, 1184 / std::max(nsys, 1));
-      G.pp = max_pp > 0 ? std::min(cdiv(max_pp, 256), cap) : 0;
+      G.pp = max_nsol > 0 ? std::min(cdiv(max_nsol, 8), cap) : 0;
       G.qp = any_q && max_qp > 0 ? std::min(cdiv(max_qp, 256), cap) : 0;
       G.bonded = max_terms > 0 ? cdiv(max_terms, 256) : 0;
       G.qq = any_qq ? 1 : 0;
@@ -842,7 +853,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   std::vector<SysState> sst(n);
   B.sysh.resize(n);
   int ww_cap = 64;
-  long long pp_tot = 0, qp_tot = 0, qw_tot = 0;
+  long long pp_tot = 0, qp_tot = 0, qw_tot = 0, near_tot = 0, nearw_tot = 0;
   int ncgp_sol_tot = 0, pwg_cap = 32;
 
   for (int s = 0; s < n; s++) {
@@ -1196,7 +1207,8 @@ void build(Batch &B, qb_handle *const *hs, int n) {
           if (d2(X, si, V.nat_solute + 3 * iw) <= rpw * rpw) c++;
         pwmax = std::max(pwmax, c);
       }
-      S.pp_cap = (int)(pp * 1.3 + 256);
+      // row entries: every pair from both sides
+      S.pp_cap = (int)std::min(2.0 * std::floor(pp * 1.3 + 256), 2147483000.0);
       if (V.nwat > 0 && V.ncgp_solute > 0)
         pwg_cap = std::max(pwg_cap, std::min(((int)(pwmax * 1.15) + 32 + 31) / 32 * 32, (V.nwat + 31) / 32 * 32));
       S.qp_cap = V.nqat * V.nat_solute + 16;
@@ -1210,7 +1222,11 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       }
       ww_cap = std::max(ww_cap, ((int)(mx * 1.15) + 31) / 32 * 32);
     }
-    S.pp_off = (int)pp_tot; pp_tot += S.pp_cap;
+    S.pp_off = pp_tot; pp_tot += S.pp_cap;
+    S.near_off = (int)near_tot;
+    near_tot += (long long)V.ncgp_solute * ((V.ncgp_solute + 31) / 32);
+    S.nearw_off = (int)nearw_tot;
+    if (!S.switch_atoms) nearw_tot += (long long)V.ncgp_solute * ((V.nwat + 31) / 32);
     S.csoff = ncgp_sol_tot; ncgp_sol_tot += V.ncgp_solute;
     // solute-water tables: each solute group's non-Q atoms with their charge
     // products (single precision, as crg(i)*crg(j)) and LJ products with the
@@ -1247,7 +1263,6 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     B.max_ncgp = std::max(B.max_ncgp, V.ncgp);
     if (V.use_LRF) B.lrf_dims.push_back(make_int2(V.ncgp, S.nlrft));
     B.max_terms = std::max(B.max_terms, V.nbonds + V.nangles + V.ntors + V.nimps);
-    B.max_pp = std::max(B.max_pp, S.pp_cap);
     if (V.nwat > 0) B.max_ncgp_sol_w = std::max(B.max_ncgp_sol_w, V.ncgp_solute);
     B.max_qp = std::max(B.max_qp, S.qp_cap);
     B.any_lrf |= V.use_LRF != 0;
@@ -1430,7 +1445,10 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   P.rs = dev_upload(rs, o); P.rs_fk = dev_upload(rs_fk, o); P.rp = dev_upload(rp, o); P.rp_x = dev_upload(rp_x, o);
   P.rp_fk = dev_upload(rp_fk, o); P.rd = dev_upload(rd, o); P.rd_p = dev_upload(rd_p, o);
   P.ra = dev_upload(ra, o); P.ra_p = dev_upload(ra_p, o); P.rw = dev_upload(rw, o); P.rw_p = dev_upload(rw_p, o);
-  P.pp = dev_alloc<int4>(pp_tot, o);
+  P.pp = dev_alloc<unsigned>(pp_tot, o);
+  P.pp_row = dev_alloc<int2>(x.size(), o);
+  P.near = dev_alloc<unsigned>(near_tot, o);
+  P.nearw = dev_alloc<unsigned>(nearw_tot, o);
   P.pwg_cap = pwg_cap;
   P.pwg = dev_alloc<uint16_t>((size_t)std::max(ncgp_sol_tot, 1) * pwg_cap, o);
   P.pwg_n = dev_alloc<int>(std::max(ncgp_sol_tot, 1), o);
@@ -1670,7 +1688,7 @@ void refresh_workload(Batch &B, int nsteps) {
   for (int k = 0; k < B.P.nwat_tot; k++) ww += wwn[k];
   double pw = 0, pp = 0, qp = 0, qw = 0, sh = 0, cg = B.P.ncgp_tot, its = 0, itmax = 0;
   for (int s = 0; s < B.nsys; s++) {
-    pp += st[s].pp_n; pw += st[s].pw_n; qp += (double)st[s].qp_n * B.sysh[s].S;
+    pp += st[s].pp_n / 2; pw += st[s].pw_n; qp += (double)st[s].qp_n * B.sysh[s].S;
     qw += (double)st[s].qw_n * B.sysh[s].nq * B.sysh[s].S;
     sh += B.views[s].shake_constraints;
     its += (double)st[s].shake_its;

@@ -61,7 +61,9 @@ struct SysDev {
   int sh_off, nsh;            // shake molecules
   int rs_off, nrs, rp_off, nrp, rd_off, nrd, ra_off, nra, rw_off, nrw;
   // dynamic list segments
-  int pp_off, pp_cap, qp_off, qp_cap, qw_off, qw_cap;
+  long long pp_off;
+  int pp_cap, qp_off, qp_cap, qw_off, qw_cap;
+  int near_off, nearw_off;    // words of the group-pair bits
   int csoff;                  // first solute group of this system among all systems' solute groups
   int ff_type, use_lrf, qvdw, wpol, nshell, iac_ow, separate_scaling, has_shake, detail_temps;
   int qp_once;                // lists with Q atoms are built once (Rcq > exclusion radius)
@@ -189,7 +191,9 @@ struct DevPtrs {
   int4 *ra; double2 *ra_p;                 // i, j, k, ipsi; ang, fk
   int4 *rw; double4 *rw_p;                 // i, j, ih; d, fk, aMorse, dMorse
   // dynamic lists
-  int4 *pp;                                // i, j, lj
+  unsigned *pp;                            // rows of the solute atoms: j | LJ code << 30
+  int2 *pp_row;                            // per atom: first entry, entries (solute atoms)
+  unsigned *near, *nearw;                  // solute group pairs within the cut-off; (any-atom) group-water pairs
   uint16_t *pwg;                           // [solute group*pwg_cap + k] local water index
   int *pwg_n, pwg_cap;                     // waters listed per solute group
   struct PwAtom *pwa;                      // non-Q atoms of each solute group (static)

@@ -118,36 +118,27 @@ __global__ void k_cgp_centers(DevPtrs P, int force) {
 
 // The any-atom cut-off tests of iuse_switch_atom 0 (nbpplis2_lrf md.f90:4955,
 // nbpwlis2_lrf 6500, nbqplis2 7700), FP64 as the reference.
-// Solute group pair: inside when any atom pair of the two groups is within
-// rc2; *last receives the squared distance of the last pair computed (the two
-// groups' last atoms when none is inside), which the reference then tests
-// against RcLRF.
-__device__ __forceinline__ bool groups_inside_any(const DevPtrs &P, int gi, int gj, double rc2, double *last) {
-  double r2 = 0.0;
+// Solute group pair: inside when any atom pair of the two groups is within rc2.
+__device__ __forceinline__ bool groups_inside_any(const DevPtrs &P, int gi, int gj, double rc2) {
   for (int ia = P.cg_first[gi]; ia <= P.cg_last[gi]; ia++) {
     const double3 xi = ld3(P.x, P.cg_atoms[ia]);
     for (int ja = P.cg_first[gj]; ja <= P.cg_last[gj]; ja++) {
       const double3 xj = ld3(P.x, P.cg_atoms[ja]);
       const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 <= rc2) { *last = r2; return true; }
+      if (dx * dx + dy * dy + dz * dz <= rc2) return true;
     }
   }
-  *last = r2;
   return false;
 }
 
 // Solute group and a point (a water O or the solute centre): inside when any
-// atom of the group is within rc2 of it; *last as above.
-__device__ __forceinline__ bool group_point_inside_any(const DevPtrs &P, int gi, double3 p, double rc2, double *last) {
-  double r2 = 0.0;
+// atom of the group is within rc2 of it.
+__device__ __forceinline__ bool group_point_inside_any(const DevPtrs &P, int gi, double3 p, double rc2) {
   for (int ia = P.cg_first[gi]; ia <= P.cg_last[gi]; ia++) {
     const double3 xi = ld3(P.x, P.cg_atoms[ia]);
     const double dx = xi.x - p.x, dy = xi.y - p.y, dz = xi.z - p.z;
-    r2 = dx * dx + dy * dy + dz * dz;
-    if (r2 <= rc2) { *last = r2; return true; }
+    if (dx * dx + dy * dy + dz * dz <= rc2) return true;
   }
-  *last = r2;
   return false;
 }
 
@@ -175,40 +166,24 @@ __device__ __forceinline__ int group_point_reach(const DevPtrs &P, int gi, doubl
   return 0;
 }
 
-// Near/far test of an LRF gather pair (target group g, source group h) under
-// iuse_switch_atom 0, when one of them is a solute group: true when the pair
-// takes part in the LRF (outside the any-atom cut-off, last pair within
-// RcLRF).  Groups whose centres are farther apart than the cut-off plus both
-// radii (with a margin) are outside without the atom loop.
-__device__ __forceinline__ bool lrf_window_any(const DevPtrs &P, const SysDev &S, int g, bool g_sol, int h, bool h_sol,
-                                               double rc2) {
-  const double *Lg = P.lrf + (size_t)g * LRF_STRIDE, *Lh = P.lrf + (size_t)h * LRF_STRIDE;
-  const double dx = Lg[0] - Lh[0], dy = Lg[1] - Lh[1], dz = Lg[2] - Lh[2];
-  const double dc = sqrt(dx * dx + dy * dy + dz * dz);
-  const bool far = dc - Lg[LRF_STRIDE - 1] - Lh[LRF_STRIDE - 1] > sqrt(rc2) + 1e-6;
-  double last;
-  bool inside;
-  if (g_sol && h_sol) {
-    if (far) {
-      const double3 a = ld3(P.x, P.cg_atoms[P.cg_last[g]]), b = ld3(P.x, P.cg_atoms[P.cg_last[h]]);
-      last = (a.x - b.x) * (a.x - b.x) + (a.y - b.y) * (a.y - b.y) + (a.z - b.z) * (a.z - b.z);
-      inside = false;
-    } else {
-      inside = groups_inside_any(P, g, h, rc2, &last);
-    }
-  } else {
-    // solute group and water: the group's atoms against the water O
-    const int gs = g_sol ? g : h, gw = g_sol ? h : g;
-    const double3 o = ld3(P.x, P.cg_sw[gw]);
-    if (far) {
-      const double3 a = ld3(P.x, P.cg_atoms[P.cg_last[gs]]);
-      last = (a.x - o.x) * (a.x - o.x) + (a.y - o.y) * (a.y - o.y) + (a.z - o.z) * (a.z - o.z);
-      inside = false;
-    } else {
-      inside = group_point_inside_any(P, gs, o, rc2, &last);
-    }
-  }
-  return !inside && last <= S.RcLRF2;
+// Near/far test of an LRF gather pair (groups g and h of system s) under
+// iuse_switch_atom 0, when one of them is a solute group: whether they are
+// within the any-atom cut-off, from the bits of k_group_near and k_list_pw
+// (built before the gather).  The pair takes part in the LRF when it is
+// outside the cut-off and the last atom pair the reference's loop computes,
+// the groups' last atoms (or the water's O), is within RcLRF.
+__device__ __forceinline__ bool near_any(const DevPtrs &P, const SysDev &S, int gl, int hl) {
+  if (gl < S.ncgp_sol && hl < S.ncgp_sol)
+    return (P.near[S.near_off + (size_t)gl * ((S.ncgp_sol + 31) / 32) + (hl >> 5)] >> (hl & 31)) & 1u;
+  const int sl = min(gl, hl), w = max(gl, hl) - S.ncgp_sol;
+  return (P.nearw[S.nearw_off + (size_t)sl * ((S.nwat + 31) / 32) + (w >> 5)] >> (w & 31)) & 1u;
+}
+
+// The atom whose distance the gather's window tests take: the switching atom,
+// or under iuse_switch_atom 0 a solute group's last atom.
+__device__ __forceinline__ int lrf_ref_atom(const DevPtrs &P, const SysDev &S, int gl) {
+  const int g = S.coff + gl;
+  return S.switch_atoms || gl >= S.ncgp_sol ? P.cg_sw[g] : P.cg_atoms[P.cg_last[g]];
 }
 
 // Multipole contribution of charge q at offset (dx,dy,dz) from a group centre
@@ -307,7 +282,7 @@ __device__ __forceinline__ void lrf_fold(double *m, const double *t) {
 constexpr int LRF_TILE_G = 128, LRF_TILE_A = 512, LRF_BLOCK = 128;
 constexpr int LRF_TILES_PER_BLOCK = 4;   // default source tiles per block (P.lrf_tpb); larger systems use more blocks
 
-template <bool MIXED>
+template <bool MIXED, bool ANY>
 __global__ void __launch_bounds__(LRF_BLOCK, MIXED ? 8 : 5) k_lrf_gather(DevPtrs P, int force) {
   using R = typename std::conditional<MIXED, float, double>::type;
   using R4 = typename std::conditional<MIXED, float4, double4>::type;
@@ -334,7 +309,7 @@ __global__ void __launch_bounds__(LRF_BLOCK, MIXED ? 8 : 5) k_lrf_gather(DevPtrs
     active = !(P.flags[swg] & F_EXCL);
     const double *L = P.lrf + (size_t)g * LRF_STRIDE;
     cx = L[0]; cy = L[1]; cz = L[2];
-    xs = ld3(P.x, swg);
+    xs = ld3(P.x, ANY ? lrf_ref_atom(P, S, gl) : swg);
   }
   const double ox = MIXED ? S.origin[0] : 0.0, oy = MIXED ? S.origin[1] : 0.0, oz = MIXED ? S.origin[2] : 0.0;
   const R ccx = (R)(cx - ox), ccy = (R)(cy - oy), ccz = (R)(cz - oz);
@@ -366,7 +341,7 @@ __global__ void __launch_bounds__(LRF_BLOCK, MIXED ? 8 : 5) k_lrf_gather(DevPtrs
     for (int i = threadIdx.x; i < nh; i += LRF_BLOCK) {
       int h = S.coff + tile.x + i;
       int sw = P.cg_sw[h];
-      double3 p = ld3(P.x, sw);
+      double3 p = ld3(P.x, ANY ? lrf_ref_atom(P, S, tile.x + i) : sw);
       double w = (P.flags[sw] & F_EXCL) ? -1.0 : (tile.x + i < S.ncgp_sol ? 1.0 : 0.0);
       hsw[i] = make_double4(p.x, p.y, p.z, w);
       hrange[i] = make_int2(P.cg_first[h] - a0, P.cg_last[h] - P.cg_first[h] + 1);
@@ -392,13 +367,14 @@ __global__ void __launch_bounds__(LRF_BLOCK, MIXED ? 8 : 5) k_lrf_gather(DevPtrs
         double4 hs = hsw[i];
         if (hs.w < 0.0 || tile.x + i == gl) continue;
         double rc2 = (g_sol && hs.w > 0.0) ? S.Rcpp2 : ((g_sol || hs.w > 0.0) ? S.Rcpw2 : S.Rcww2);
-        if (!S.switch_atoms && (g_sol || hs.w > 0.0)) {
-          if (!lrf_window_any(P, S, g, g_sol, S.coff + tile.x + i, hs.w > 0.0, rc2)) continue;
-        } else {
-          double dx = xs.x - hs.x, dy = xs.y - hs.y, dz = xs.z - hs.z;
-          if (box) min_image(bx, dx, dy, dz);
-          double r2 = dx * dx + dy * dy + dz * dz;
-          if (!(r2 > rc2 && r2 <= S.RcLRF2)) continue;
+        double dx = xs.x - hs.x, dy = xs.y - hs.y, dz = xs.z - hs.z;
+        if (box) min_image(bx, dx, dy, dz);
+        double r2 = dx * dx + dy * dy + dz * dz;
+        if (!(r2 <= S.RcLRF2)) continue;
+        if (ANY && !S.switch_atoms && (g_sol || hs.w > 0.0)) {
+          if (near_any(P, S, gl, tile.x + i)) continue;
+        } else if (!(r2 > rc2)) {
+          continue;
         }
         int2 rg = hrange[i];
         const double3 sh = box ? image_shift(bx, hs.x - cx, hs.y - cy, hs.z - cz) : make_double3(0, 0, 0);
@@ -522,7 +498,7 @@ __device__ __forceinline__ void lrf_finish_x2(const float2 *m, const float2 *t, 
 // adds the totals to the FP64 record with one atomic per component.
 constexpr int LRFX_BLOCK = 128, LRFX_TARGETS = 2 * LRFX_BLOCK;
 
-template <bool BOX>
+template <bool BOX, bool ANY>
 __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int force) {
   const int s = blockIdx.y;
   if (!list_due(P, s, force)) return;
@@ -555,7 +531,7 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
       const double *L = P.lrf + (size_t)g * LRF_STRIDE;
       cen[h] = make_double3(L[0], L[1], L[2]);
       cc[h][0] = (float)(L[0] - ox); cc[h][1] = (float)(L[1] - oy); cc[h][2] = (float)(L[2] - oz);
-      xs[h] = ld3(P.x, swg);
+      xs[h] = ld3(P.x, ANY ? lrf_ref_atom(P, S, gl[h]) : swg);
     }
   }
   // minus the two target centres (positions relative to the origin); in a
@@ -578,7 +554,7 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
     for (int i = threadIdx.x; i < nh; i += LRFX_BLOCK) {
       const int h = S.coff + tile.x + i;
       const int sw = P.cg_sw[h];
-      const double3 p = ld3(P.x, sw);
+      const double3 p = ld3(P.x, ANY ? lrf_ref_atom(P, S, tile.x + i) : sw);
       const double w = (P.flags[sw] & F_EXCL) ? -1.0 : (tile.x + i < S.ncgp_sol ? 1.0 : 0.0);
       hsw[i] = make_double4(p.x, p.y, p.z, w);
       hrange[i] = make_int2(P.cg_first[h] - a0, P.cg_last[h] - P.cg_first[h] + 1);
@@ -602,16 +578,12 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const double rc2 = (gsol[h] && hs.w > 0.0) ? S.Rcpp2 : ((gsol[h] || hs.w > 0.0) ? S.Rcpw2 : S.Rcww2);
-        bool in;
-        if (!S.switch_atoms && (gsol[h] || hs.w > 0.0)) {
-          in = act[h] && tile.x + i != gl[h] &&
-               lrf_window_any(P, S, S.coff + gl[h], gsol[h], S.coff + tile.x + i, hs.w > 0.0, rc2);
-        } else {
-          double dx = xs[h].x - hs.x, dy = xs[h].y - hs.y, dz = xs[h].z - hs.z;
-          if (BOX) min_image(bx, dx, dy, dz);
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          in = act[h] && tile.x + i != gl[h] && r2 > rc2 && r2 <= S.RcLRF2;
-        }
+        double dx = xs[h].x - hs.x, dy = xs[h].y - hs.y, dz = xs[h].z - hs.z;
+        if (BOX) min_image(bx, dx, dy, dz);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        bool in = act[h] && tile.x + i != gl[h] && r2 <= S.RcLRF2;
+        if (ANY && !S.switch_atoms && (gsol[h] || hs.w > 0.0)) in = in && !near_any(P, S, gl[h], tile.x + i);
+        else in = in && r2 > rc2;
         any = any || in;
         (h ? sel.y : sel.x) = in ? 1.f : 0.f;
       }
@@ -833,48 +805,21 @@ __device__ __forceinline__ bool zero_pair(const DevPtrs &P, int i, int j, int lj
          P.ljb[3 * i + lj - 1] * P.ljb[3 * j + lj - 1] == 0.0;
 }
 
-// Solute-solute pair list (nbpplist, md.f90:5175): block (ig, system),
-// threads over jg.  Group pairs are taken once, by the reference's parity rule.
-__global__ void k_list_pp(DevPtrs P, int force) {
-  int s = blockIdx.y;
+// Solute charge-group pairs within the cut-off (the group test of nbpplist,
+// md.f90:5175, on switching atoms or any atom pair), one bit per ordered pair:
+// block (ig, system), threads over jg, a warp's ballot is a word.  The
+// solute-solute list and, under iuse_switch_atom 0, the LRF gather read them.
+__global__ void k_group_near(DevPtrs P, int force) {
+  const int s = blockIdx.y;
   if (!list_due(P, s, force)) return;
   const SysDev &S = P.sys[s];
-  int ig = blockIdx.x;
+  const int ig = blockIdx.x;
   if (ig >= S.ncgp_sol) return;
-  int gi = S.coff + ig;
-  int swi = P.cg_sw[gi];
-  if (P.flags[swi] & F_EXCL) return;
-  double3 xs = ld3(P.x, swi);
-  const int lane = threadIdx.x & 31;
-  // the pairs of group pair (gi, gj), written at out[0..] when out is given;
-  // returns their number
-  auto pairs = [&](int jg, int gj, int4 *out) {
-    int n = 0;
-    for (int ia = P.cg_first[gi]; ia <= P.cg_last[gi]; ia++) {
-      int i = P.cg_atoms[ia];
-      if (P.iq[i] >= 0) continue;
-      for (int ja = P.cg_first[gj]; ja <= P.cg_last[gj]; ja++) {
-        int j = P.cg_atoms[ja];
-        if (ig == jg && i >= j) continue;
-        if (P.iq[j] >= 0) continue;
-        int lj = ljcode(P, S, i, j);
-        if (zero_pair(P, i, j, lj)) continue;
-        if (excluded_pair(P, S, i, j)) continue;
-        if (is14(P, S, i, j)) lj = 3;
-        if (out) out[n] = make_int4(i, j, lj, 0);
-        n++;
-      }
-    }
-    return n;
-  };
-  // rounds in which every lane of a warp takes part, so that a warp reserves
-  // its pairs' slots with one atomic (a per-pair atomic on the system's
-  // counter serialises the ~10^5 pairs of a large solute)
+  const int gi = S.coff + ig, nw = (S.ncgp_sol + 31) / 32;
+  const double3 xs = ld3(P.x, P.cg_sw[gi]);
   for (int base = 0; base < S.ncgp_sol; base += blockDim.x) {
-    const int jg = base + threadIdx.x;
-    const int gj = S.coff + jg;
-    bool inside = jg < S.ncgp_sol && !((ig > jg && ((ig + jg) & 1) == 0) || (ig < jg && ((ig + jg) & 1) == 1));
-    if (inside) inside = !(P.flags[P.cg_sw[gj]] & F_EXCL);
+    const int jg = base + threadIdx.x, gj = S.coff + jg;
+    bool inside = jg < S.ncgp_sol;
     if (inside) {
       if (S.switch_atoms) {
         double3 xj = ld3(P.x, P.cg_sw[gj]);
@@ -883,30 +828,67 @@ __global__ void k_list_pp(DevPtrs P, int force) {
         inside = dx * dx + dy * dy + dz * dz <= S.Rcpp2;
       } else {
         const int reach = groups_reach(P, gi, gj, S.Rcpp2);
-        double last;
-        inside = reach > 0 || (reach == 0 && groups_inside_any(P, gi, gj, S.Rcpp2, &last));
+        inside = reach > 0 || (reach == 0 && groups_inside_any(P, gi, gj, S.Rcpp2));
       }
     }
-    const int n = inside ? pairs(jg, gj, nullptr) : 0;
-    // exclusive prefix of n over the warp, one reservation per warp
-    int pre = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(FULL, pre, o);
-      if (lane >= o) pre += t;
-    }
-    const int total = __shfl_sync(FULL, pre, 31);
-    int first = 0;
-    if (lane == 0 && total > 0) first = atomicAdd(&P.st[s].pp_n, total);
-    first = __shfl_sync(FULL, first, 0);
-    if (n == 0) continue;
-    const int k = first + pre - n;
-    if (k + n <= S.pp_cap) {
-      pairs(jg, gj, P.pp + S.pp_off + k);
-    } else {
-      set_status(&P.st[s], QB_ERR_LIST_OVERFLOW);
+    const unsigned bal = __ballot_sync(FULL, inside);
+    const int w = jg >> 5;
+    if ((threadIdx.x & 31) == 0 && w < nw) P.near[S.near_off + (size_t)ig * nw + w] = bal;
+  }
+}
+
+// Solute-solute pair list (nbpplist, md.f90:5175) as one row per non-Q atom:
+// its partners in both directions, ascending, j | LJ code << 30, so that
+// nb_pp_body sums an atom's gradient in registers instead of adding every
+// pair's two ends with atomics.  A warp per atom scans the system's solute
+// atoms twice, first to count, then to write the row at the place it
+// reserved: 100 us for the 3,000-atom polymer of 318 groups, against 608 with a
+// thread per group pair walking its up to 15 x 15 atom pairs.
+constexpr int PP_BLOCK = 256;
+
+__global__ void __launch_bounds__(PP_BLOCK) k_list_pp(DevPtrs P, int force) {
+  const int s = blockIdx.y;
+  if (!list_due(P, s, force)) return;
+  const SysDev &S = P.sys[s];
+  const int li = blockIdx.x * (PP_BLOCK / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (li >= S.nsol) return;
+  const int i = S.aoff + li, gi = P.cgp[i], ig = gi - S.coff;
+  const unsigned *near = P.near + S.near_off + (size_t)ig * ((S.ncgp_sol + 31) / 32);
+  int first = 0, cnt = 0;
+  if (P.iq[i] < 0 && ig < S.ncgp_sol && !(P.flags[P.cg_sw[gi]] & F_EXCL)) {
+    for (int pass = 0; pass < 2; pass++) {
+      int n = 0;
+      for (int base = 0; base < S.nsol; base += 32) {
+        const int lj_ = base + lane, j = S.aoff + lj_;
+        bool ok = lj_ < S.nsol && lj_ != li;
+        int lj = 0;
+        if (ok) {
+          const int gj = P.cgp[j], jg = gj - S.coff;
+          ok = jg < S.ncgp_sol && ((near[jg >> 5] >> (jg & 31)) & 1u) && P.iq[j] < 0 &&
+               !(P.flags[P.cg_sw[gj]] & F_EXCL);
+          if (ok) {
+            lj = ljcode(P, S, i, j);
+            ok = !zero_pair(P, i, j, lj) && !excluded_pair(P, S, i, j);
+            if (ok && pass && is14(P, S, i, j)) lj = 3;
+          }
+        }
+        const unsigned bal = __ballot_sync(FULL, ok);
+        if (pass && ok) P.pp[S.pp_off + first + n + __popc(bal & ((1u << lane) - 1u))] = (unsigned)j | ((unsigned)lj << 30);
+        n += __popc(bal);
+      }
+      if (pass == 0) {
+        cnt = n;
+        if (lane == 0) first = cnt > 0 ? atomicAdd(&P.st[s].pp_n, cnt) : 0;
+        first = __shfl_sync(FULL, first, 0);
+        if (cnt > S.pp_cap - first) {
+          if (lane == 0) set_status(&P.st[s], QB_ERR_LIST_OVERFLOW);
+          cnt = 0;
+        }
+        if (cnt == 0) break;
+      }
     }
   }
+  if (lane == 0) P.pp_row[i] = make_int2(first, cnt);   // within the system's segment
 }
 
 // Solute-water list (nbpwlist, md.f90:6684): per solute charge group, the
@@ -925,6 +907,7 @@ __global__ void k_list_pw(DevPtrs P, int force) {
   int swi = P.cg_sw[gi];
   uint16_t *out = P.pwg + (size_t)sg * P.pwg_cap;
   int cnt = 0;
+  unsigned *nearw = S.switch_atoms ? nullptr : P.nearw + S.nearw_off + (size_t)ig * ((S.nwat + 31) / 32);
   if (!(P.flags[swi] & F_EXCL)) {
     double3 xs = ld3(P.x, swi);
     for (int base = 0; base < S.nwat; base += 32) {
@@ -939,11 +922,11 @@ __global__ void k_list_pw(DevPtrs P, int force) {
           ok = dx * dx + dy * dy + dz * dz <= S.Rcpw2;
         } else {
           const int reach = group_point_reach(P, gi, xo, S.Rcpw2);
-          double last;
-          ok = reach > 0 || (reach == 0 && group_point_inside_any(P, gi, xo, S.Rcpw2, &last));
+          ok = reach > 0 || (reach == 0 && group_point_inside_any(P, gi, xo, S.Rcpw2));
         }
       }
       unsigned bal = __ballot_sync(FULL, ok);
+      if (nearw && lane == 0) nearw[base >> 5] = bal;
       if (ok) {
         int pos = cnt + __popc(bal & ((1u << lane) - 1u));
         if (pos < P.pwg_cap) out[pos] = (uint16_t)iw;
@@ -985,8 +968,7 @@ __global__ void k_list_qp(DevPtrs P, int force) {
       if (S.pbc) min_image(bx, dx, dy, dz);
       if (dx * dx + dy * dy + dz * dz > S.Rcq2) continue;
     } else {
-      double last;
-      if (!group_point_inside_any(P, gi, make_double3(S.xp[0], S.xp[1], S.xp[2]), S.Rcq2, &last)) continue;
+      if (!group_point_inside_any(P, gi, make_double3(S.xp[0], S.xp[1], S.xp[2]), S.Rcq2)) continue;
     }
     int f = P.cg_first[gi], n = P.cg_last[gi] - f + 1;
     // whole warps per round: a warp reserves its entries with one atomic
@@ -1570,25 +1552,30 @@ __global__ void __launch_bounds__(WWX_BLOCK, 2) k_nb_ww_x2(DevPtrs P, int wpb) {
   }
 }
 
-// nonbond_pp (md.f90:10387): one thread per pair.
+// nonbond_pp (md.f90:10387) over the atoms' rows (k_list_pp): a warp per atom,
+// lanes over its partners, the gradient of the atom alone summed over the row
+// and added with one atomic per component; each pair is evaluated from both
+// sides and its energy halved.  The pair terms are some forty FP64 operations, cheap
+// beside three atomics a pair: on the polymer (450,000 pairs) the solute
+// kernel took 59 us with every pair once and its j end by atomics, 50 this way.
 __device__ __forceinline__ void nb_pp_body(DevPtrs &P, int bx, int s, int gx) {
   const SysDev &S = P.sys[s];
-  int n = P.st[s].pp_n;
-  const int4 *L = P.pp + S.pp_off;
   double el = 0, vdw = 0;
-  const int lane = threadIdx.x & 31;
-  for (int k0 = bx * blockDim.x; k0 < n; k0 += gx * blockDim.x) {
-    int k = k0 + threadIdx.x;
-    // the list holds each atom i's pairs of a group pair consecutively: the
-    // lanes with the same i sum their share of i's gradient over the warp and
-    // the first of them adds it with one atomic per component
+  const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  const unsigned *L = P.pp + S.pp_off;
+  for (int li = bx * nwarp + (threadIdx.x >> 5); li < S.nsol; li += gx * nwarp) {
+    const int i = S.aoff + li;
+    const int2 row = P.pp_row[i];
+    if (row.y == 0) continue;
+    const double3 xi = ld3(P.x, i);
+    const float qi = P.crg[i];
     double gi[3] = {0.0, 0.0, 0.0};
-    int i = -1 - lane;
-    if (k < n) {
-      int4 p = L[k];
-      i = p.x;
-      int j = p.y, lj = p.z;
-      double3 xi = ld3(P.x, i), xj = ld3(P.x, j);
+    unsigned next = lane < row.y ? L[row.x + lane] : 0u;
+    for (int k = lane; k < row.y; k += 32) {
+      const unsigned e = next;
+      if (k + 32 < row.y) next = L[row.x + k + 32];
+      const int j = (int)(e & 0x3fffffffu), lj = (int)(e >> 30);
+      double3 xj = ld3(P.x, j);
       double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
       if (S.pbc) {
         // nonbond_pp_box (md.f90:10508-10519): the image of the charge-group
@@ -1599,7 +1586,7 @@ __device__ __forceinline__ void nb_pp_body(DevPtrs &P, int bx, int s, int gx) {
       }
       double r = rsqrt(dx * dx + dy * dy + dz * dz);
       double r2 = r * r, r6 = r2 * r2 * r2;
-      float qq = P.crg[i] * P.crg[j];
+      float qq = qi * P.crg[j];
       double Vel = (double)qq * r;
       if (lj == 3) Vel = Vel * S.el14;
       double Va, Vb;
@@ -1613,31 +1600,16 @@ __device__ __forceinline__ void nb_pp_body(DevPtrs &P, int bx, int s, int gx) {
         Vb = r6 * P.ljb[3 * i + lj - 1] * P.ljb[3 * j + lj - 1];
       }
       double dv = r2 * (-Vel - 12. * Va + 6. * Vb);
-      gi[0] = -dv * dx; gi[1] = -dv * dy; gi[2] = -dv * dz;
-      atomic_add3(P.d, j, dv * dx, dv * dy, dv * dz);
+      gi[0] -= dv * dx; gi[1] -= dv * dy; gi[2] -= dv * dz;
       el += Vel;
       vdw += Va - Vb;
     }
-    // runs of equal i in consecutive lanes: a segmented sum towards each
-    // run's first lane (end: the next run's first lane)
-    const int prev = __shfl_up_sync(FULL, i, 1);
-    const bool head = lane == 0 || prev != i;
-    const unsigned heads = __ballot_sync(FULL, head);
-    const unsigned later = lane == 31 ? 0u : heads & ~((2u << lane) - 1u);
-    const int end = later ? __ffs(later) - 1 : 32;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const bool take = lane + o < end;
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const double t = __shfl_down_sync(FULL, gi[c], o);
-        if (take) gi[c] += t;
-      }
-    }
-    if (i >= 0 && head) atomic_add3(P.d, i, gi[0], gi[1], gi[2]);
+    for (int c = 0; c < 3; c++) gi[c] = warp_sum(gi[c]);
+    if (lane == 0) atomic_add3(P.d, i, gi[0], gi[1], gi[2]);
   }
-  warp_add(&P.E[s * QB_NE + QB_E_PP_EL], el);
-  warp_add(&P.E[s * QB_NE + QB_E_PP_VDW], vdw);
+  warp_add(&P.E[s * QB_NE + QB_E_PP_EL], 0.5 * el);
+  warp_add(&P.E[s * QB_NE + QB_E_PP_VDW], 0.5 * vdw);
 }
 
 // nonbond_pw (md.f90:10631) over the group list: one thread per (listed
