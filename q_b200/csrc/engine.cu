@@ -73,6 +73,10 @@ struct EventPair {
 
 struct KernelStat { double ms = 0; long long launches = 0; };
 
+// Blocks per SM (of the one-part form) up to which the mixed LRF gather splits
+// its sums over a block's warps.
+constexpr int LRFX_CS_BLOCKS = 1;
+
 struct Batch {
   int nsys = 0;
   qb_options opt{};
@@ -231,16 +235,15 @@ struct Batch {
     fork_streams();
     if (any_lrf) {
       launch("lrf_gather", [&] {
-        const dim3 gx(max_lrfx_blocks, nsys);
         if (opt.precision == QB_MIXED) {
-          if (any_box && any_any_atom) k_lrf_gather_x2<true, true><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
-          else if (any_box) k_lrf_gather_x2<true, false><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
-          else if (any_any_atom) k_lrf_gather_x2<false, true><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
-          else k_lrf_gather_x2<false, false><<<gx, LRFX_BLOCK, 0, s1>>>(p, force);
+          if (any_box && any_any_atom) lrf_gather_mixed<true, true>(s1, force);
+          else if (any_box) lrf_gather_mixed<true, false>(s1, force);
+          else if (any_any_atom) lrf_gather_mixed<false, true>(s1, force);
+          else lrf_gather_mixed<false, false>(s1, force);
         } else {
           const dim3 g(max_lrf_blocks, nsys);
-          if (any_any_atom) k_lrf_gather<false, true><<<g, LRF_BLOCK, 0, s1>>>(p, force);
-          else k_lrf_gather<false, false><<<g, LRF_BLOCK, 0, s1>>>(p, force);
+          if (any_any_atom) k_lrf_gather<true><<<g, LRF_BLOCK, 0, s1>>>(p, force);
+          else k_lrf_gather<false><<<g, LRF_BLOCK, 0, s1>>>(p, force);
         }
       });
     }
@@ -285,13 +288,38 @@ struct Batch {
   bool forking() const { return !profiling && side[0] && streams_on; }
 
   int max_lrfx_blocks = 1;   // the packed (two targets per thread) gather's grid
-  void set_lrf_tpb(int tpb) {
+  // tpb source tiles per block.  FP64: with one, up to 8 blocks share a tile
+  // while that leaves the gather below four blocks per SM (with more, every
+  // block pays its staging and 20 atomics per target for a shorter chain).
+  // Mixed: four warps share the sums of a block's targets (lrfx_cs 4) while the
+  // launch has at most LRFX_CS_BLOCKS blocks per SM: at 315 blocks (21
+  // windows) sharing took 518 us a rebuild against 461.
+  int lrfx_cs = 1;
+  void set_lrf_tpb(int tpb, bool share = true, int sms = 148) {
     P.lrf_tpb = tpb;
-    max_lrf_blocks = max_lrfx_blocks = 1;
+    P.lrf_sub = 1;
+    lrfx_cs = 1;
+    int blocks = 1;
+    long long all = 0, allx = 0;
     for (const int2 &d : lrf_dims) {
-      max_lrf_blocks = std::max(max_lrf_blocks, cdiv(d.x, LRF_BLOCK) * cdiv(d.y, tpb));
-      max_lrfx_blocks = std::max(max_lrfx_blocks, cdiv(d.x, LRFX_TARGETS) * cdiv(d.y, tpb));
+      const int b = cdiv(d.x, LRF_BLOCK) * cdiv(d.y, tpb);
+      blocks = std::max(blocks, b);
+      all += b;
+      allx += cdiv(d.x, lrfx_targets(1)) * cdiv(d.y, tpb);
     }
+    if (share && tpb == 1)
+      while (P.lrf_sub < 8 && all * P.lrf_sub * 2 <= 4LL * sms) P.lrf_sub *= 2;
+    if (allx <= LRFX_CS_BLOCKS * (long long)sms) lrfx_cs = 4;
+    max_lrf_blocks = blocks * P.lrf_sub;
+    max_lrfx_blocks = 1;
+    for (const int2 &d : lrf_dims)
+      max_lrfx_blocks = std::max(max_lrfx_blocks, cdiv(d.x, lrfx_targets(lrfx_cs)) * cdiv(d.y, tpb));
+  }
+  template <bool BOX, bool ANY>
+  void lrf_gather_mixed(cudaStream_t st, int force) {
+    const dim3 g(max_lrfx_blocks, nsys);
+    if (lrfx_cs == 4) k_lrf_gather_x2<BOX, ANY, 4><<<g, LRFX_BLOCK, 0, st>>>(P, force);
+    else k_lrf_gather_x2<BOX, ANY, 1><<<g, LRFX_BLOCK, 0, st>>>(P, force);
   }
   void fork_streams() {
     if (!forking()) return;
@@ -1754,7 +1782,9 @@ void get_tuning(const Batch &B, qb_tuning *t) {
   t->ww_chunk_max = B.ww_chunk_max;
 }
 
-void set_tuning(Batch &B, const qb_tuning &t) {
+// share: small batches may split a source tile of the LRF gather over blocks
+// (a caller's own setting is taken as it is)
+void set_tuning(Batch &B, const qb_tuning &t, bool share) {
   if (t.lrf_tiles_per_block < 1 || t.lrf_tiles_per_block > 1024) fail(QB_ERR_ARG, "lrf_tiles_per_block out of range");
   if (t.ww_chunk % 32 || t.ww_chunk < B.ww_chunk_floor || t.ww_chunk > B.ww_chunk_max)
     fail(QB_ERR_ARG, "ww_chunk must be a multiple of 32 within the batch's range");
@@ -1763,7 +1793,7 @@ void set_tuning(Batch &B, const qb_tuning &t) {
   if (t.water_pass_per_atom != 0 && t.water_pass_per_atom != 1) fail(QB_ERR_ARG, "water_pass_per_atom must be 0 or 1");
   CUDA_TRY(cudaStreamSynchronize(B.stream));
   B.drop_graphs();
-  B.set_lrf_tpb(t.lrf_tiles_per_block);
+  B.set_lrf_tpb(t.lrf_tiles_per_block, share);
   B.P.ww_chunk = t.ww_chunk;
   B.P.ww_nch = (std::max(B.max_nwat, 1) + t.ww_chunk - 1) / t.ww_chunk;
   B.streams_on = t.side_streams != 0;
@@ -1800,7 +1830,7 @@ int qb_batch_set_tuning(qb_batch *bb, const qb_tuning *t) {
   if (!bb || !t) { qb::set_error("invalid argument"); return QB_ERR_ARG; }
   return guarded_batch([&] {
     CUDA_TRY(cudaSetDevice(bb->b.opt.device));
-    qb::set_tuning(bb->b, *t);
+    qb::set_tuning(bb->b, *t, false);
   });
 }
 
@@ -1815,7 +1845,7 @@ int qb_batch_autotune(qb_batch *bb, int steps_per_trial, qb_tuning *out) {
     qb::get_tuning(B, &best);
     int trials = 0;
     auto run = [&](const qb_tuning &t) {
-      qb::set_tuning(B, t);
+      qb::set_tuning(B, t, true);
       trials++;
       double ms = qb::time_steps(B, steps);
       qb::clear_history(B);
@@ -1857,7 +1887,7 @@ int qb_batch_autotune(qb_batch *bb, int steps_per_trial, qb_tuning *out) {
       t.side_streams = !best.side_streams;
       consider(t);
     }
-    qb::set_tuning(B, best);
+    qb::set_tuning(B, best, true);
     best.trials = trials;
     best.ms_per_step = best_ms;
     best.ms_per_step_before = before;

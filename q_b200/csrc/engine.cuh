@@ -214,7 +214,7 @@ struct DevPtrs {
   int ww_cap, ww_chunk, ww_nch;
   int2 *ww_tiles;                          // water-water force blocks: (system, first water)
   int n_ww_tiles;
-  int lrf_tpb;                             // source tiles swept by one block of the LRF gather
+  int lrf_tpb, lrf_sub;                    // source tiles swept by one block of the LRF gather; blocks sharing a tile
   // energies
   double *kin;                             // [s*4] kinetic energy of this step: solute all, free, solvent all, free
   int kin_nblk;

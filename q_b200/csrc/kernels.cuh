@@ -186,10 +186,6 @@ __device__ __forceinline__ int lrf_ref_atom(const DevPtrs &P, const SysDev &S, i
   return S.switch_atoms || gl >= S.ncgp_sol ? P.cg_sw[g] : P.cg_atoms[P.cg_last[g]];
 }
 
-// Multipole contribution of charge q at offset (dx,dy,dz) from a group centre
-// (md.f90:5581-5636), accumulated in the symmetric form m[20] = phi0,
-// phi1[x,y,z], phi2[xx,xy,xz,yy,yz,zz], phi3[xxx,xxy,xxz,xyy,xyz,xzz,yyy,yyz,
-// yzz,zzz]: the reference's 9 and 27 components are copies of these.
 // 1/sqrt(v) on the MUFU unit (rsqrt.approx.ftz.f32, <= 2 ulp); the squared
 // distances it is used on are never denormal.
 __device__ __forceinline__ float rsqrt_ftz(float v) {
@@ -202,66 +198,55 @@ __device__ __forceinline__ float rsq(float v) { return rsqrt_ftz(v); }
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ double rsq(double v) { return rsqrt(v); }
 
-template <class R>
-__device__ __forceinline__ void lrf_accumulate(R *m, R q, R dx, R dy, R dz) {
-  R r2 = dx * dx + dy * dy + dz * dz;
-  R rinv = rsq(r2), ri2 = rinv * rinv;
-  R f0 = q * rinv * ri2;              // q / r^3
-  m[0] += f0 * r2;
-  m[1] -= f0 * dx; m[2] -= f0 * dy; m[3] -= f0 * dz;
-  R f1 = R(3) * f0 * ri2;
-  R f1x = f1 * dx, f1y = f1 * dy, f1z = f1 * dz;
-  m[4] += f1x * dx - f0; m[5] += f1x * dy; m[6] += f1x * dz;
-  m[7] += f1y * dy - f0; m[8] += f1y * dz; m[9] += f1z * dz - f0;
-  R f2 = -f1 * ri2;
-  R x5 = R(5) * dx, y5 = R(5) * dy, z5 = R(5) * dz;
-  R xx = x5 * dx, yy = y5 * dy, zz = z5 * dz, xy = x5 * dy;
-  m[10] += f2 * (xx * dx - R(3) * r2 * dx);
-  m[11] += f2 * (xx * dy - r2 * dy);
-  m[12] += f2 * (xx * dz - r2 * dz);
-  m[13] += f2 * (yy * dx - r2 * dx);
-  m[14] += f2 * (xy * dz);
-  m[15] += f2 * (zz * dx - r2 * dx);
-  m[16] += f2 * (yy * dy - R(3) * r2 * dy);
-  m[17] += f2 * (yy * dz - r2 * dz);
-  m[18] += f2 * (zz * dy - r2 * dy);
-  m[19] += f2 * (zz * dz - R(3) * r2 * dz);
+// Multipole contribution of charge q at offset d = (x, y, z) from a group
+// centre (md.f90:5581-5636).  The record's 20 components are phi0, phi1[x,y,z],
+// phi2[xx,xy,xz,yy,yz,zz] and phi3[xxx,xxy,xxz,xyy,xyz,xzz,yyy,yyz,yzz,zzz]
+// (the reference's 9 and 27 are copies of these); phi2 and phi3 are
+// derivatives of 1/r and so traceless: zz = -(xx + yy), xxx = -(xyy + xzz),
+// yyy = -(xxy + yzz), zzz = -(xxz + yyz).  The sums kept per target, LRF_NSUM:
+//   A[0] = sum q/r         A[1..3] = sum f0 d         A[4] = sum f0
+//   A[5..7] = sum f1 d     A[8..12] = sum f1 {xx, xy, xz, yy, yz}
+//   A[13..19] = sum f2 {xxy, xxz, xyy, xyz, xzz, yyz, yzz}
+// with f0 = q/r^3, f1 = 3 q/r^5, f2 = 15 q/r^7; lrf_fold forms the record:
+// phi1 = -A[1..3], phi2_ab = f1 sums - delta_ab A[4], phi3_abc = -(f2 sums -
+// the delta terms of A[5..7]).  44 operations a charge and a reciprocal root,
+// against 61 for the 20 components one by one.
+constexpr int LRF_NSUM = 20;
+
+__device__ __forceinline__ void lrf_accumulate(double *A, double q, double x, double y, double z) {
+  const double r2 = fma(x, x, fma(y, y, z * z));
+  const double rinv = rsqrt(r2), ri2 = rinv * rinv;
+  const double a = q * rinv, f0 = a * ri2;
+  A[0] += a;
+  A[1] = fma(f0, x, A[1]); A[2] = fma(f0, y, A[2]); A[3] = fma(f0, z, A[3]);
+  A[4] += f0;
+  const double c3 = 3.0 * ri2, f1 = f0 * c3;
+  const double ax = f1 * x, ay = f1 * y, az = f1 * z;
+  A[5] += ax; A[6] += ay; A[7] += az;
+  const double pxx = ax * x, pxy = ax * y, pyy = ay * y, pzz = az * z;
+  A[8] += pxx; A[9] += pxy; A[10] = fma(ax, z, A[10]); A[11] += pyy; A[12] = fma(ay, z, A[12]);
+  const double c5 = 5.0 * ri2, vx = c5 * x, vy = c5 * y, vz = c5 * z;
+  A[13] = fma(pxx, vy, A[13]); A[14] = fma(pxx, vz, A[14]); A[15] = fma(pyy, vx, A[15]);
+  A[16] = fma(pxy, vz, A[16]); A[17] = fma(pzz, vx, A[17]); A[18] = fma(pyy, vz, A[18]);
+  A[19] = fma(pzz, vy, A[19]);
 }
 
-// The same sums with the diagonal terms of phi2 and phi3 factored out:
-// m[0..19] as above without them, plus t[0] = sum f0 and t[1..3] = sum
-// f2*r2*d; lrf_fold applies them once at the end (phi2_aa -= t0,
-// phi3_aab -= t_b for a != b, phi3_aaa -= 3 t_a).  22 fewer operations per
-// charge; used by the mixed-precision gather.
-__device__ __forceinline__ void lrf_accumulate_split(float *m, float *t, float q, float dx, float dy, float dz) {
-  float r2 = dx * dx + dy * dy + dz * dz;
-  float rinv = rsqrt_ftz(r2), ri2 = rinv * rinv;
-  float f0 = q * rinv * ri2;
-  m[0] = fmaf(f0, r2, m[0]);
-  m[1] = fmaf(-f0, dx, m[1]); m[2] = fmaf(-f0, dy, m[2]); m[3] = fmaf(-f0, dz, m[3]);
-  t[0] += f0;
-  float f1 = 3.f * f0 * ri2;
-  float ax = f1 * dx, ay = f1 * dy, az = f1 * dz;
-  m[4] = fmaf(ax, dx, m[4]); m[5] = fmaf(ax, dy, m[5]); m[6] = fmaf(ax, dz, m[6]);
-  m[7] = fmaf(ay, dy, m[7]); m[8] = fmaf(ay, dz, m[8]); m[9] = fmaf(az, dz, m[9]);
-  float f2 = -f1 * ri2;
-  float w = f2 * r2;
-  t[1] = fmaf(w, dx, t[1]); t[2] = fmaf(w, dy, t[2]); t[3] = fmaf(w, dz, t[3]);
-  float u = 5.f * f2;
-  float px = u * dx, py = u * dy;
-  float qxx = px * dx, qxy = px * dy, qxz = px * dz, qyy = py * dy, qyz = py * dz, qzz = u * dz * dz;
-  m[10] = fmaf(qxx, dx, m[10]); m[11] = fmaf(qxx, dy, m[11]); m[12] = fmaf(qxx, dz, m[12]);
-  m[13] = fmaf(qxy, dy, m[13]); m[14] = fmaf(qxy, dz, m[14]); m[15] = fmaf(qxz, dz, m[15]);
-  m[16] = fmaf(qyy, dy, m[16]); m[17] = fmaf(qyy, dz, m[17]); m[18] = fmaf(qyz, dz, m[18]);
-  m[19] = fmaf(qzz, dz, m[19]);
-}
-
-__device__ __forceinline__ void lrf_fold(double *m, const double *t) {
-  m[4] -= t[0]; m[7] -= t[0]; m[9] -= t[0];
-  m[10] -= 3. * t[1]; m[11] -= t[2]; m[12] -= t[3];
-  m[13] -= t[1]; m[15] -= t[1];
-  m[16] -= 3. * t[2]; m[17] -= t[3]; m[18] -= t[2];
-  m[19] -= 3. * t[3];
+// The record's 20 components from the sums.
+__device__ __forceinline__ void lrf_fold(const double *A, double *m) {
+  m[0] = A[0];
+  m[1] = -A[1]; m[2] = -A[2]; m[3] = -A[3];
+  m[4] = A[8] - A[4]; m[5] = A[9]; m[6] = A[10]; m[7] = A[11] - A[4]; m[8] = A[12];
+  m[9] = -(m[4] + m[7]);
+  m[11] = A[6] - A[13];                // xxy
+  m[12] = A[7] - A[14];                // xxz
+  m[13] = A[5] - A[15];                // xyy
+  m[14] = -A[16];                      // xyz
+  m[15] = A[5] - A[17];                // xzz
+  m[17] = A[7] - A[18];                // yyz
+  m[18] = A[6] - A[19];                // yzz
+  m[10] = -(m[13] + m[15]);            // xxx
+  m[16] = -(m[11] + m[18]);            // yyy
+  m[19] = -(m[12] + m[17]);            // zzz
 }
 
 // LRF multipoles of every charge group, gathered (nbpplist_lrf 5448,
@@ -271,48 +256,62 @@ __device__ __forceinline__ void lrf_fold(double *m, const double *t) {
 // charge here).  The reference visits each unordered pair once and adds to
 // both groups; the gather adds the same contributions.
 //
-// One thread per group g, blockIdx.y = system.  The system's groups are swept
-// in tiles (consecutive groups, at most LRF_TILE_G groups and LRF_TILE_A
-// atoms, boundaries precomputed on the host): a tile's switching atoms and
-// atom positions/charges are staged in shared memory and read as broadcasts.
-// The group-pair window test is FP64 in both precisions.  Mixed precision:
-// atom offsets from the group centre in FP32 (positions relative to the
-// sphere centre, |offset| >= ~7 A here), each tile summed in FP32 and added to
-// FP64 totals.
+// FP64 engine: one thread per group g, blockIdx.y = system.  The system's
+// groups are swept in tiles (consecutive groups, at most LRF_TILE_G groups and
+// LRF_TILE_A atoms, boundaries precomputed on the host): a tile's switching
+// atoms and atom positions/charges are staged in shared memory and read as
+// broadcasts.  A block sweeps lrf_tpb tiles, or in a small batch a 1/lrf_sub
+// part of one (Batch::set_lrf_tpb): one system's gather is bound by the chain
+// of the charges a thread walks, not by their number (a rebuild of one 480-group
+// sphere 138 us with a tile per block, 17 with an eighth; 1,067 groups 138 and
+// 36; 41 windows, tiles as they were, 1,148 to 790 us by the fewer operations).
 constexpr int LRF_TILE_G = 128, LRF_TILE_A = 512, LRF_BLOCK = 128;
 constexpr int LRF_TILES_PER_BLOCK = 4;   // default source tiles per block (P.lrf_tpb); larger systems use more blocks
 
-template <bool MIXED, bool ANY>
-__global__ void __launch_bounds__(LRF_BLOCK, MIXED ? 8 : 5) k_lrf_gather(DevPtrs P, int force) {
-  using R = typename std::conditional<MIXED, float, double>::type;
-  using R4 = typename std::conditional<MIXED, float4, double4>::type;
-  int s = blockIdx.y;
+// A block's share of the sources: tiles [t0, t1) of the system, and of each
+// the groups [h0, h1) of its part.
+struct LrfShare { int gchunk, t0, t1, part, sub; };
+
+__device__ __forceinline__ LrfShare lrf_share(const DevPtrs &P, const SysDev &S, int bx) {
+  LrfShare r;
+  r.sub = P.lrf_sub;
+  r.part = bx % r.sub;
+  bx /= r.sub;
+  const int hsplit = max((S.nlrft + P.lrf_tpb - 1) / P.lrf_tpb, 1);
+  r.gchunk = bx / hsplit;
+  r.t0 = (bx - r.gchunk * hsplit) * P.lrf_tpb;
+  r.t1 = min(r.t0 + P.lrf_tpb, S.nlrft);
+  return r;
+}
+
+__device__ __forceinline__ int2 lrf_part(const LrfShare &B, int2 tile) {
+  const int nh = tile.y - tile.x;
+  return make_int2(tile.x + nh * B.part / B.sub, tile.x + nh * (B.part + 1) / B.sub);
+}
+
+template <bool ANY>
+__global__ void __launch_bounds__(LRF_BLOCK, 5) k_lrf_gather(DevPtrs P, int force) {
+  const int s = blockIdx.y;
   if (!list_due(P, s, force)) return;
   const SysDev &S = P.sys[s];
   if (!S.use_lrf) return;
-  // block -> (chunk of target groups, range of source tiles)
-  const int tpb = P.lrf_tpb;
-  const int hsplit = (S.nlrft + tpb - 1) / tpb;
-  const int gchunk = blockIdx.x / max(hsplit, 1), hpart = blockIdx.x % max(hsplit, 1);
-  if (hsplit == 0 || gchunk * LRF_BLOCK >= S.ncgp) return;
-  const int t0 = hpart * tpb, t1 = min(t0 + tpb, S.nlrft);
-  __shared__ double4 hsw[LRF_TILE_G];      // switching atom; w: -1 excluded, 1 solute, 0 water
+  const LrfShare B = lrf_share(P, S, blockIdx.x);
+  if (S.nlrft == 0 || B.gchunk * LRF_BLOCK >= S.ncgp) return;
+  __shared__ double4 hsw[LRF_TILE_G];      // window-test atom; w: -1 excluded, 1 solute, 0 water
   __shared__ int2 hrange[LRF_TILE_G];      // first atom slot, atom count
-  __shared__ R4 hat[LRF_TILE_A];           // atom position (mixed: from the sphere centre), charge
-  int gl = gchunk * LRF_BLOCK + threadIdx.x;
-  int g = S.coff + gl;
+  __shared__ double4 hat[LRF_TILE_A];      // atom position, charge
+  const int gl = B.gchunk * LRF_BLOCK + threadIdx.x;
+  const int g = S.coff + gl;
   bool active = gl < S.ncgp;
   double cx = 0, cy = 0, cz = 0;
   double3 xs = make_double3(0, 0, 0);
   if (active) {
-    int swg = P.cg_sw[g];
+    const int swg = P.cg_sw[g];
     active = !(P.flags[swg] & F_EXCL);
     const double *L = P.lrf + (size_t)g * LRF_STRIDE;
     cx = L[0]; cy = L[1]; cz = L[2];
     xs = ld3(P.x, ANY ? lrf_ref_atom(P, S, gl) : swg);
   }
-  const double ox = MIXED ? S.origin[0] : 0.0, oy = MIXED ? S.origin[1] : 0.0, oz = MIXED ? S.origin[2] : 0.0;
-  const R ccx = (R)(cx - ox), ccy = (R)(cy - oy), ccz = (R)(cz - oz);
   const bool g_sol = gl < S.ncgp_sol;
   // periodic box: pair windows on the switching atoms' nearest image; a
   // source group's charges enter at the image nearest the target centre
@@ -320,95 +319,54 @@ __global__ void __launch_bounds__(LRF_BLOCK, MIXED ? 8 : 5) k_lrf_gather(DevPtrs
   // nbwwlist_box_lrf 8601-8694)
   const bool box = S.pbc != 0;
   const BoxD bx = box_of(P, s);
-  // FP64 totals: registers (FP64 path) or this thread's column in shared memory (mixed)
-  __shared__ double mtot[MIXED ? 24 : 1][MIXED ? LRF_BLOCK : 1];
-  double m[MIXED ? 1 : 20];
-  R mt[20];
-  float tt[4];
-  if (MIXED) {
+  const double rcl = S.RcLRF2, rcww = S.Rcww2, rcpw = S.Rcpw2, rcpp = S.Rcpp2;
+  double A[LRF_NSUM];
 #pragma unroll
-    for (int k = 0; k < 24; k++) mtot[k][threadIdx.x] = 0.0;
-  } else {
-#pragma unroll
-    for (int k = 0; k < 20; k++) m[k] = 0.0;
-  }
-  for (int t = t0; t < t1; t++) {
-    int2 tile = P.lrft[S.lrft_off + t];
-    int nh = tile.y - tile.x;
-    int a0 = P.cg_first[S.coff + tile.x];
-    int na = P.cg_last[S.coff + tile.y - 1] - a0 + 1;
+  for (int k = 0; k < LRF_NSUM; k++) A[k] = 0.0;
+  for (int t = B.t0; t < B.t1; t++) {
+    const int2 tile = lrf_part(B, P.lrft[S.lrft_off + t]);
+    const int nh = tile.y - tile.x;
+    if (nh == 0) continue;
+    const int a0 = P.cg_first[S.coff + tile.x];
+    const int na = P.cg_last[S.coff + tile.y - 1] - a0 + 1;
     __syncthreads();
     for (int i = threadIdx.x; i < nh; i += LRF_BLOCK) {
-      int h = S.coff + tile.x + i;
-      int sw = P.cg_sw[h];
-      double3 p = ld3(P.x, ANY ? lrf_ref_atom(P, S, tile.x + i) : sw);
-      double w = (P.flags[sw] & F_EXCL) ? -1.0 : (tile.x + i < S.ncgp_sol ? 1.0 : 0.0);
+      const int h = S.coff + tile.x + i;
+      const int sw = P.cg_sw[h];
+      const double3 p = ld3(P.x, ANY ? lrf_ref_atom(P, S, tile.x + i) : sw);
+      const double w = (P.flags[sw] & F_EXCL) ? -1.0 : (tile.x + i < S.ncgp_sol ? 1.0 : 0.0);
       hsw[i] = make_double4(p.x, p.y, p.z, w);
       hrange[i] = make_int2(P.cg_first[h] - a0, P.cg_last[h] - P.cg_first[h] + 1);
     }
     for (int i = threadIdx.x; i < na; i += LRF_BLOCK) {
-      int at = P.cg_atoms[a0 + i];
-      double4 p = P.x[at];
-      bool qsol = (at - S.aoff) < S.nsol && P.iq[at] >= 0;
-      R4 v;
-      v.x = (R)(p.x - ox); v.y = (R)(p.y - oy); v.z = (R)(p.z - oz);
-      v.w = qsol ? R(0) : (R)P.crg[at];
-      hat[i] = v;
+      const int at = P.cg_atoms[a0 + i];
+      const double4 p = P.x[at];
+      const bool qsol = (at - S.aoff) < S.nsol && P.iq[at] >= 0;
+      hat[i] = make_double4(p.x, p.y, p.z, qsol ? 0.0 : (double)P.crg[at]);
     }
     __syncthreads();
-    if (active) {
-      if (MIXED) {
-#pragma unroll
-        for (int k = 0; k < 20; k++) mt[k] = R(0);
-#pragma unroll
-        for (int k = 0; k < 4; k++) tt[k] = 0.f;
+    if (!active) continue;
+    for (int i = 0; i < nh; i++) {
+      const double4 hs = hsw[i];
+      if (hs.w < 0.0 || tile.x + i == gl) continue;
+      double dx = xs.x - hs.x, dy = xs.y - hs.y, dz = xs.z - hs.z;
+      if (box) min_image(bx, dx, dy, dz);
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      if (!(r2 <= rcl)) continue;
+      if (ANY && !S.switch_atoms && (g_sol || hs.w > 0.0)) {
+        if (near_any(P, S, gl, tile.x + i)) continue;
+      } else if (!(r2 > ((g_sol && hs.w > 0.0) ? rcpp : ((g_sol || hs.w > 0.0) ? rcpw : rcww)))) {
+        continue;
       }
-      for (int i = 0; i < nh; i++) {
-        double4 hs = hsw[i];
-        if (hs.w < 0.0 || tile.x + i == gl) continue;
-        double rc2 = (g_sol && hs.w > 0.0) ? S.Rcpp2 : ((g_sol || hs.w > 0.0) ? S.Rcpw2 : S.Rcww2);
-        double dx = xs.x - hs.x, dy = xs.y - hs.y, dz = xs.z - hs.z;
-        if (box) min_image(bx, dx, dy, dz);
-        double r2 = dx * dx + dy * dy + dz * dz;
-        if (!(r2 <= S.RcLRF2)) continue;
-        if (ANY && !S.switch_atoms && (g_sol || hs.w > 0.0)) {
-          if (near_any(P, S, gl, tile.x + i)) continue;
-        } else if (!(r2 > rc2)) {
-          continue;
-        }
-        int2 rg = hrange[i];
-        const double3 sh = box ? image_shift(bx, hs.x - cx, hs.y - cy, hs.z - cz) : make_double3(0, 0, 0);
-        if (MIXED) {
-          // a zero charge adds exact zeros; water groups (3 atoms) unrolled
-          const R scx = ccx + (R)sh.x, scy = ccy + (R)sh.y, scz = ccz + (R)sh.z;
-          if (rg.y == 3) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-              R4 a = hat[rg.x + k];
-              lrf_accumulate_split((float *)mt, tt, (float)a.w, (float)(a.x - scx), (float)(a.y - scy),
-                                   (float)(a.z - scz));
-            }
-          } else {
-            for (int k = 0; k < rg.y; k++) {
-              R4 a = hat[rg.x + k];
-              lrf_accumulate_split((float *)mt, tt, (float)a.w, (float)(a.x - scx), (float)(a.y - scy),
-                                   (float)(a.z - scz));
-            }
-          }
-        } else {
-          for (int k = 0; k < rg.y; k++) {
-            R4 a = hat[rg.x + k];
-            if (a.w != R(0))
-              lrf_accumulate<double>(m, (double)a.w, (double)a.x - cx - sh.x, (double)a.y - cy - sh.y,
-                                     (double)a.z - cz - sh.z);
-          }
-        }
+      const int2 rg = hrange[i];
+      double scx = cx, scy = cy, scz = cz;
+      if (box) {
+        const double3 sh = image_shift(bx, hs.x - cx, hs.y - cy, hs.z - cz);
+        scx += sh.x; scy += sh.y; scz += sh.z;
       }
-      if (MIXED) {
-#pragma unroll
-        for (int k = 0; k < 20; k++) mtot[k][threadIdx.x] += (double)mt[k];
-#pragma unroll
-        for (int k = 0; k < 4; k++) mtot[20 + k][threadIdx.x] += (double)tt[k];
+      for (int k = 0; k < rg.y; k++) {
+        const double4 a = hat[rg.x + k];
+        if (a.w != 0.0) lrf_accumulate(A, a.w, a.x - scx, a.y - scy, a.z - scz);
       }
     }
   }
@@ -416,110 +374,149 @@ __global__ void __launch_bounds__(LRF_BLOCK, MIXED ? 8 : 5) k_lrf_gather(DevPtrs
   // k_cgp_centers)
   if (active) {
     double *L = P.lrf + (size_t)g * LRF_STRIDE;
-    if (MIXED) {
-      double mm[20], t4[4];
+    double m[20];
+    lrf_fold(A, m);
 #pragma unroll
-      for (int k = 0; k < 20; k++) mm[k] = mtot[k][threadIdx.x];
-#pragma unroll
-      for (int k = 0; k < 4; k++) t4[k] = mtot[20 + k][threadIdx.x];
-      lrf_fold(mm, t4);
-#pragma unroll
-      for (int k = 0; k < 20; k++)
-        if (mm[k] != 0.0) atomicAdd(&L[3 + k], mm[k]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 20; k++)
-        if (m[MIXED ? 0 : k] != 0.0) atomicAdd(&L[3 + k], m[MIXED ? 0 : k]);
-    }
+    for (int k = 0; k < 20; k++)
+      if (m[k] != 0.0) atomicAdd(&L[3 + k], m[k]);
   }
 }
 
 // -------------------------------------------- packed FP32x2 LRF gather
 
-// lrf_accumulate_split for two target groups at once (.x and .y), on the
-// packed FP32x2 pipes.  Sign conventions differ so that every update is one
-// fused multiply-add: m[1..3] hold +sum f0*d (phi1 = -m[1..3]), m[10..19] and
-// t[1..3] hold the phi3 sums with f2 taken positive (phi3 = -(fold of them));
-// lrf_finish_x2 restores the signs.
+// The sums of one charge for two target groups at once (.x and .y), on the
+// packed FP32x2 pipes: m[0..19] in the order of the record without the
+// diagonal terms of phi2 and phi3, which t[0] = sum f0 and t[1..3] = sum f1 d
+// hold for the fold at the end.  Every update is one fused multiply-add:
+// m[1..3] hold +sum f0 d (phi1 = -m[1..3]), m[10..19] and t[1..3] the phi3
+// sums with f2 taken positive (phi3 = -(fold of them)); lrfx_fold restores
+// the signs.
 // sel is 1 for a target inside the pair's window and 0 outside it (its
 // charge q is then 0); unsel = 1 - sel.  A half outside the window may sit at
 // distance 0 (a one-atom group against itself), so its r2 is replaced by 1
 // before the reciprocal: every term of that half is then an exact 0.
-__device__ __forceinline__ void lrf_accumulate_x2(float2 *m, float2 *t, float2 q, float2 dx, float2 dy, float2 dz,
-                                                  float2 sel, float2 unsel) {
+// The 24 sums are independent chains; part C of CS takes its share of them:
+// all (CS 1), or one of four (phi0, phi1, t0 and phi2's x row | the rest of
+// phi2 and t | phi3's xx, xy, xz rows | the rest), each sum with the same
+// operations in the same order whatever CS is.
+template <int CS> struct LrfxPart { static constexpr int n = CS == 1 ? 24 : 8; };
+
+__host__ __device__ constexpr int lrfx_slot(int cs, int c, int k) {
+  // component (0..19 m, 20..23 t) of accumulator k of part c; -1: none
+  if (cs == 1) return k;
+  constexpr int tab[4][8] = {{0, 1, 2, 3, 20, 4, 5, 6}, {7, 8, 9, 21, 22, 23, -1, -1}, {10, 11, 12, 13, 14, 15, -1, -1},
+                             {16, 17, 18, 19, -1, -1, -1, -1}};
+  return tab[c][k];
+}
+
+template <int CS, int C>
+__device__ __forceinline__ void lrfx_accumulate(float2 *A, float2 q, float2 dx, float2 dy, float2 dz, float2 sel,
+                                                float2 unsel) {
   const float2 three = make_float2(3.f, 3.f), five = make_float2(5.f, 5.f);
   const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
   const float2 r2s = __ffma2_rn(r2, sel, unsel);
   const float2 rinv = make_float2(rsqrt_ftz(r2s.x), rsqrt_ftz(r2s.y));
   const float2 ri2 = __fmul2_rn(rinv, rinv);
   const float2 f0 = __fmul2_rn(__fmul2_rn(q, rinv), ri2);          // q / r^3
-  m[0] = __ffma2_rn(f0, r2, m[0]);
-  m[1] = __ffma2_rn(f0, dx, m[1]); m[2] = __ffma2_rn(f0, dy, m[2]); m[3] = __ffma2_rn(f0, dz, m[3]);
-  t[0] = __fadd2_rn(t[0], f0);
+  auto at = [](int comp) {
+    int r = 0;
+#pragma unroll
+    for (int k = 0; k < LrfxPart<CS>::n; k++)
+      if (lrfx_slot(CS, C, k) == comp) r = k;
+    return r;
+  };
+  auto fma_to = [&](int comp, float2 a, float2 b) { A[at(comp)] = __ffma2_rn(a, b, A[at(comp)]); };
+  if (CS == 1 || C == 0) {
+    fma_to(0, f0, r2);
+    fma_to(1, f0, dx); fma_to(2, f0, dy); fma_to(3, f0, dz);
+    A[at(20)] = __fadd2_rn(A[at(20)], f0);
+  }
   const float2 f1 = __fmul2_rn(__fmul2_rn(f0, ri2), three);        // 3 q / r^5
-  const float2 ax = __fmul2_rn(f1, dx), ay = __fmul2_rn(f1, dy), az = __fmul2_rn(f1, dz);
-  m[4] = __ffma2_rn(ax, dx, m[4]); m[5] = __ffma2_rn(ax, dy, m[5]); m[6] = __ffma2_rn(ax, dz, m[6]);
-  m[7] = __ffma2_rn(ay, dy, m[7]); m[8] = __ffma2_rn(ay, dz, m[8]); m[9] = __ffma2_rn(az, dz, m[9]);
+  if (CS == 1 || C == 0) {
+    const float2 ax = __fmul2_rn(f1, dx);
+    fma_to(4, ax, dx); fma_to(5, ax, dy); fma_to(6, ax, dz);
+    if (CS != 1) return;
+  }
+  if (CS == 1 || C == 1) {
+    const float2 ay = __fmul2_rn(f1, dy), az = __fmul2_rn(f1, dz);
+    fma_to(7, ay, dy); fma_to(8, ay, dz); fma_to(9, az, dz);
+  }
   const float2 f2 = __fmul2_rn(f1, ri2);                            // 3 q / r^7 (the negated f2)
-  const float2 w = __fmul2_rn(f2, r2);
-  t[1] = __ffma2_rn(w, dx, t[1]); t[2] = __ffma2_rn(w, dy, t[2]); t[3] = __ffma2_rn(w, dz, t[3]);
+  if (CS == 1 || C == 1) {
+    const float2 w = __fmul2_rn(f2, r2);
+    fma_to(21, w, dx); fma_to(22, w, dy); fma_to(23, w, dz);
+    if (CS != 1) return;
+  }
   const float2 u = __fmul2_rn(f2, five);
-  const float2 px = __fmul2_rn(u, dx), py = __fmul2_rn(u, dy), pz = __fmul2_rn(u, dz);
-  const float2 qxx = __fmul2_rn(px, dx), qxy = __fmul2_rn(px, dy), qxz = __fmul2_rn(px, dz);
-  const float2 qyy = __fmul2_rn(py, dy), qyz = __fmul2_rn(py, dz), qzz = __fmul2_rn(pz, dz);
-  m[10] = __ffma2_rn(qxx, dx, m[10]); m[11] = __ffma2_rn(qxx, dy, m[11]); m[12] = __ffma2_rn(qxx, dz, m[12]);
-  m[13] = __ffma2_rn(qxy, dy, m[13]); m[14] = __ffma2_rn(qxy, dz, m[14]); m[15] = __ffma2_rn(qxz, dz, m[15]);
-  m[16] = __ffma2_rn(qyy, dy, m[16]); m[17] = __ffma2_rn(qyy, dz, m[17]); m[18] = __ffma2_rn(qyz, dz, m[18]);
-  m[19] = __ffma2_rn(qzz, dz, m[19]);
+  if (CS == 1 || C == 2) {
+    const float2 px = __fmul2_rn(u, dx);
+    const float2 qxx = __fmul2_rn(px, dx), qxy = __fmul2_rn(px, dy), qxz = __fmul2_rn(px, dz);
+    fma_to(10, qxx, dx); fma_to(11, qxx, dy); fma_to(12, qxx, dz);
+    fma_to(13, qxy, dy); fma_to(14, qxy, dz); fma_to(15, qxz, dz);
+  }
+  if (CS == 1 || C == 3) {
+    const float2 py = __fmul2_rn(u, dy), pz = __fmul2_rn(u, dz);
+    const float2 qyy = __fmul2_rn(py, dy), qyz = __fmul2_rn(py, dz), qzz = __fmul2_rn(pz, dz);
+    fma_to(16, qyy, dy); fma_to(17, qyy, dz); fma_to(18, qyz, dz);
+    fma_to(19, qzz, dz);
+  }
 }
 
-// One target's packed sums (half h of every float2) as the record's 20
-// components in FP64: the diagonal terms folded in, the signs restored.
-__device__ __forceinline__ void lrf_finish_x2(const float2 *m, const float2 *t, int h, double *out) {
-  double tt[4];
+// One target's 24 sums as the record's 20 components in FP64: the diagonal
+// terms folded in, the signs restored.
+__device__ __forceinline__ void lrfx_fold(double *m, const double *t) {
+  m[4] -= t[0]; m[7] -= t[0]; m[9] -= t[0];
+  m[10] -= 3. * t[1]; m[11] -= t[2]; m[12] -= t[3];
+  m[13] -= t[1]; m[15] -= t[1];
+  m[16] -= 3. * t[2]; m[17] -= t[3]; m[18] -= t[2];
+  m[19] -= 3. * t[3];
 #pragma unroll
-  for (int k = 0; k < 20; k++) out[k] = (double)(h ? m[k].y : m[k].x);
+  for (int k = 1; k < 4; k++) m[k] = -m[k];
 #pragma unroll
-  for (int k = 0; k < 4; k++) tt[k] = (double)(h ? t[k].y : t[k].x);
-  lrf_fold(out, tt);
-#pragma unroll
-  for (int k = 1; k < 4; k++) out[k] = -out[k];
-#pragma unroll
-  for (int k = 10; k < 20; k++) out[k] = -out[k];
+  for (int k = 10; k < 20; k++) m[k] = -m[k];
 }
 
 // The mixed-precision LRF gather (nbpp/pw/wwlist_lrf, md.f90:5448, 6864,
-// 8370) with two target groups per thread: targets gl and gl + LRFX_BLOCK of
-// the block's chunk of 2*LRFX_BLOCK groups, each source charge applied to
+// 8370) with two target groups per thread, each source charge applied to
 // both with packed FP32x2 arithmetic (a target outside the pair's window
 // takes a zero charge).  Source tiles are staged as in k_lrf_gather, atom
 // positions and charges duplicated into both halves of their float2 words;
 // the group-pair window test is FP64.  Each block sums its tiles in FP32 and
 // adds the totals to the FP64 record with one atomic per component.
-constexpr int LRFX_BLOCK = 128, LRFX_TARGETS = 2 * LRFX_BLOCK;
+// CS 4: the block's four warps take the four parts of the sums of 64 targets
+// (CS 1: a warp all sums of its 64, 256 a block).  A quarter of the chain per
+// thread and four times the blocks for a batch that cannot fill the chip: the
+// 518-group polymer 76 us a rebuild against about 300.
+constexpr int LRFX_BLOCK = 128;
+__host__ __device__ constexpr int lrfx_targets(int cs) { return 2 * LRFX_BLOCK / cs; }
 
-template <bool BOX, bool ANY>
+template <bool BOX, bool ANY, int CS>
 __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int force) {
   const int s = blockIdx.y;
   if (!list_due(P, s, force)) return;
   const SysDev &S = P.sys[s];
   if (!S.use_lrf) return;
   const int tpb = P.lrf_tpb;
-  const int hsplit = (S.nlrft + tpb - 1) / tpb;
-  const int gchunk = blockIdx.x / max(hsplit, 1), hpart = blockIdx.x % max(hsplit, 1);
-  if (hsplit == 0 || gchunk * LRFX_TARGETS >= S.ncgp) return;
+  const int hsplit = max((S.nlrft + tpb - 1) / tpb, 1);
+  const int gchunk = blockIdx.x / hsplit, hpart = blockIdx.x % hsplit;
+  if (S.nlrft == 0 || gchunk * lrfx_targets(CS) >= S.ncgp) return;
   const int t0 = hpart * tpb, t1 = min(t0 + tpb, S.nlrft);
   __shared__ double4 hsw[LRF_TILE_G];
   __shared__ int2 hrange[LRF_TILE_G];
   __shared__ float4 hxy[LRF_TILE_A], hzq[LRF_TILE_A];   // {x, x, y, y}, {z, z, q, q}
+  __shared__ float2 psum[CS == 1 ? 1 : 24][CS == 1 ? 1 : 32];
   const double ox = S.origin[0], oy = S.origin[1], oz = S.origin[2];
+  // CS 1: thread t takes targets t and t + 128 of the block's 256; CS 4: lane
+  // l of every warp targets l and l + 32 of 64
+  const int part = CS == 1 ? 0 : threadIdx.x >> 5;
+  const int slot = CS == 1 ? threadIdx.x : threadIdx.x & 31;
   int gl[2];
   bool act[2], gsol[2];
   double3 xs[2], cen[2];
   float cc[2][3];
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    gl[h] = gchunk * LRFX_TARGETS + h * LRFX_BLOCK + threadIdx.x;
+    gl[h] = gchunk * lrfx_targets(CS) + h * (lrfx_targets(CS) / 2) + slot;
     act[h] = gl[h] < S.ncgp;
     gsol[h] = gl[h] < S.ncgp_sol;
     xs[h] = cen[h] = make_double3(0, 0, 0);
@@ -540,11 +537,9 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
   float2 ncx = make_float2(-cc[0][0], -cc[1][0]), ncy = make_float2(-cc[0][1], -cc[1][1]),
          ncz = make_float2(-cc[0][2], -cc[1][2]);
   const BoxD bx = box_of(P, s);
-  float2 m[20], t[4];
+  float2 A[LrfxPart<CS>::n];
 #pragma unroll
-  for (int k = 0; k < 20; k++) m[k] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int k = 0; k < 4; k++) t[k] = make_float2(0.f, 0.f);
+  for (int k = 0; k < LrfxPart<CS>::n; k++) A[k] = make_float2(0.f, 0.f);
   for (int tt = t0; tt < t1; tt++) {
     const int2 tile = P.lrft[S.lrft_off + tt];
     const int nh = tile.y - tile.x;
@@ -601,31 +596,70 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
       }
       const int2 rg = hrange[i];
       const float2 unsel = make_float2(1.f - sel.x, 1.f - sel.y);
-      auto atom = [&](int k) {
-        const float4 a = hxy[rg.x + k], b = hzq[rg.x + k];
-        const float2 q = __fmul2_rn(make_float2(b.z, b.w), sel);
-        lrf_accumulate_x2(m, t, q, __fadd2_rn(make_float2(a.x, a.y), ncx), __fadd2_rn(make_float2(a.z, a.w), ncy),
-                          __fadd2_rn(make_float2(b.x, b.y), ncz), sel, unsel);
+      auto group = [&](auto pc) {
+        auto atom = [&](int k) {
+          const float4 a = hxy[rg.x + k], b = hzq[rg.x + k];
+          const float2 q = __fmul2_rn(make_float2(b.z, b.w), sel);
+          lrfx_accumulate<CS, decltype(pc)::value>(A, q, __fadd2_rn(make_float2(a.x, a.y), ncx),
+                                                   __fadd2_rn(make_float2(a.z, a.w), ncy),
+                                                   __fadd2_rn(make_float2(b.x, b.y), ncz), sel, unsel);
+        };
+        if (rg.y == 3) {        // a water: its three atoms as independent chains
+          atom(0);
+          atom(1);
+          atom(2);
+        } else {
+          for (int k = 0; k < rg.y; k++) atom(k);
+        }
       };
-      if (rg.y == 3) {        // a water: its three atoms as independent chains
-        atom(0);
-        atom(1);
-        atom(2);
-      } else {
-        for (int k = 0; k < rg.y; k++) atom(k);
-      }
+      if (CS == 1 || part == 0) group(std::integral_constant<int, 0>());
+      else if (part == 1) group(std::integral_constant<int, 1>());
+      else if (part == 2) group(std::integral_constant<int, 2>());
+      else group(std::integral_constant<int, 3>());
     }
   }
+  if (CS == 1) {
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
-    if (!act[h]) continue;
-    double out[20];
-    lrf_finish_x2(m, t, h, out);
-    double *L = P.lrf + (size_t)(S.coff + gl[h]) * LRF_STRIDE;
+    for (int h = 0; h < 2; h++) {
+      if (!act[h]) continue;
+      double out[20], t[4];
 #pragma unroll
-    for (int k = 0; k < 20; k++)
-      if (out[k] != 0.0) atomicAdd(&L[3 + k], out[k]);
+      for (int k = 0; k < 20; k++) out[k] = (double)(h ? A[k % LrfxPart<CS>::n].y : A[k % LrfxPart<CS>::n].x);
+#pragma unroll
+      for (int k = 0; k < 4; k++) t[k] = (double)(h ? A[(20 + k) % LrfxPart<CS>::n].y : A[(20 + k) % LrfxPart<CS>::n].x);
+      lrfx_fold(out, t);
+      double *L = P.lrf + (size_t)(S.coff + gl[h]) * LRF_STRIDE;
+#pragma unroll
+      for (int k = 0; k < 20; k++)
+        if (out[k] != 0.0) atomicAdd(&L[3 + k], out[k]);
+    }
+    return;
   }
+  // the parts' sums meet in shared memory; warps 0 and 1 fold a half each
+#pragma unroll
+  for (int c = 0; c < 4; c++)
+    if (part == c) {
+#pragma unroll
+      for (int k = 0; k < LrfxPart<CS>::n; k++)
+        if (lrfx_slot(CS, c, k) >= 0) psum[CS == 1 ? 0 : lrfx_slot(CS, c, k)][CS == 1 ? 0 : slot] = A[k];
+    }
+  __syncthreads();
+  if (part > 1) return;
+  const bool on = part == 0 ? act[0] : act[1];
+  if (!on) return;
+  double out[20], t[4];
+#pragma unroll
+  for (int k = 0; k < 24; k++) {
+    const float2 v = psum[CS == 1 ? 0 : k][CS == 1 ? 0 : slot];
+    const double d = (double)(part ? v.y : v.x);
+    if (k < 20) out[k] = d;
+    else t[k - 20] = d;
+  }
+  lrfx_fold(out, t);
+  double *L = P.lrf + (size_t)(S.coff + (part ? gl[1] : gl[0])) * LRF_STRIDE;
+#pragma unroll
+  for (int k = 0; k < 20; k++)
+    if (out[k] != 0.0) atomicAdd(&L[3 + k], out[k]);
 }
 
 // Water-water neighbour list (nbwwlist / nbwwlist_lrf, md.f90:8233, 8370),
