@@ -255,7 +255,7 @@ struct Batch {
     // a volume move rebuilds the LRF and the solute and water lists, not the
     // Q-atom lists (md.f90:15734-15744)
     if (any_q && force != 2) {
-      launch("list_qp", [&] { k_list_qp<<<nsys, 256, 0, stream>>>(p, force); });
+      launch("list_qp", [&] { k_list_qp<<<nsys, QP_LIST_BLOCK, 0, stream>>>(p, force); });
       if (max_nwat > 0) launch("list_qw", [&] { k_list_qw<<<nsys, 256, 0, stream>>>(p, force); });
     }
     join_streams();
@@ -378,7 +378,7 @@ struct Batch {
       // when the batch is small (1184 = 8 blocks per SM over the batch)
       const int cap = std::max(8, 1184 / std::max(nsys, 1));
       G.pp = max_nsol > 0 ? std::min(cdiv(max_nsol, 8), cap) : 0;
-      G.qp = any_q && max_qp > 0 ? std::min(cdiv(max_qp, 256), cap) : 0;
+      G.qp = any_q && max_qp > 0 ? std::min(cdiv(max_qp, 32), cap) : 0;
       G.bonded = max_terms > 0 ? cdiv(max_terms, 256) : 0;
       G.qq = any_qq ? 1 : 0;
       G.qb = any_qb ? 1 : 0;
@@ -860,7 +860,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   std::vector<double> qavdw, qbvdw, sc, qq_el;
   std::vector<QwAtom> qwa;
   std::vector<QwState> qws;
-  std::vector<int8_t> qconn;
+  std::vector<uint8_t> qp_code;
   std::vector<int4> qq;
   std::vector<int2> bij; std::vector<double2> bpar;
   std::vector<int4> aijk; std::vector<double2> apar, aub;
@@ -897,7 +897,6 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     S.coff = (int)cg_first.size(); S.ncgp = V.ncgp; S.ncgp_sol = V.ncgp_solute;
     S.qoff = (int)iqseq.size(); S.nq = V.nqat; S.S = V.nstates; S.natyps = V.natyps;
     S.ljoff = (int)ljcod.size(); S.qlib_off = (int)qavdw.size(); S.sc_off = (int)sc.size();
-    S.qconn_off = (int)qconn.size();
     std::vector<char> shaken(V.natom, 0);
     for (int c = 0; c < V.shake_constraints; c++) shaken[V.shake_i[c]] = shaken[V.shake_j[c]] = 1;
     for (int i = 0; i < V.natom; i++) {
@@ -977,8 +976,24 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     for (int k = 0; k < V.nqlib * 3; k++) { qavdw.push_back(V.qavdw[k]); qbvdw.push_back(V.qbvdw[k]); }
     size_t nsc = (size_t)V.nqat * (V.natyps + V.nqat) * V.nstates;
     for (size_t k = 0; k < nsc; k++) sc.push_back(V.sc_lookup[k]);
-    size_t nqc = (size_t)V.nstates * V.nat_solute * V.nqat;
-    for (size_t k = 0; k < nqc; k++) qconn.push_back(V.qconn[k]);
+    // Q-solute LJ codes (nbqplist, md.f90:7920-7960): an atom within 1-3 of a
+    // Q atom in any state pairs with none; 1-4 neighbours (in state 1) code 3
+    S.qp_code_off = (long long)qp_code.size();
+    if (V.nqat > 0)
+      for (int i = 0; i < V.nat_solute; i++) {
+        bool take = true;
+        for (int st = 0; st < V.nstates && take; st++)
+          for (int q = 0; q < V.nqat; q++)
+            if (V.qconn[((size_t)st * V.nat_solute + i) * V.nqat + q] <= 3) { take = false; break; }
+        for (int q = 0; q < V.nqat; q++) {
+          int lj = 0;
+          if (take) {
+            lj = V.ljcod[V.iac[i] * V.natyps + V.iac[V.iqseq[q]]];
+            if (V.qconn[(size_t)i * V.nqat + q] == 4) lj = 3;
+          }
+          qp_code.push_back((uint8_t)lj);
+        }
+      }
     S.qq_off = (int)qq.size();
     for (int st = 0; st < V.nstates; st++)
       for (int k = V.nbqq_off[st]; k < V.nbqq_off[st] + V.nbqq_count[st]; k++) {
@@ -1239,7 +1254,6 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       S.pp_cap = (int)std::min(2.0 * std::floor(pp * 1.3 + 256), 2147483000.0);
       if (V.nwat > 0 && V.ncgp_solute > 0)
         pwg_cap = std::max(pwg_cap, std::min(((int)(pwmax * 1.15) + 32 + 31) / 32 * 32, (V.nwat + 31) / 32 * 32));
-      S.qp_cap = V.nqat * V.nat_solute + 16;
       S.qw_cap = V.nwat + 16;
       int mx = 0;
       for (int iw = 0; iw < V.nwat; iw++) {
@@ -1282,7 +1296,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
         pwa.push_back(r);
       }
     }
-    S.qp_off = (int)qp_tot; qp_tot += S.qp_cap;
+    S.qp_off = (int)qp_tot; qp_tot += V.nqat > 0 ? V.nat_solute : 0;
     S.qw_off = (int)qw_tot; qw_tot += S.qw_cap;
     B.max_natom = std::max(B.max_natom, V.natom);
     B.max_nsol = std::max(B.max_nsol, V.nat_solute);
@@ -1292,7 +1306,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     if (V.use_LRF) B.lrf_dims.push_back(make_int2(V.ncgp, S.nlrft));
     B.max_terms = std::max(B.max_terms, V.nbonds + V.nangles + V.ntors + V.nimps);
     if (V.nwat > 0) B.max_ncgp_sol_w = std::max(B.max_ncgp_sol_w, V.ncgp_solute);
-    B.max_qp = std::max(B.max_qp, S.qp_cap);
+    if (V.nqat > 0) B.max_qp = std::max(B.max_qp, V.nat_solute);
     B.any_lrf |= V.use_LRF != 0;
     if (V.nqat > 0) B.q_states = (!B.any_q || B.q_states == V.nstates) ? V.nstates : 0;
     B.any_q |= V.nqat > 0;
@@ -1348,7 +1362,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   P.iqseq = dev_upload(iqseq, o); P.qcrg = dev_upload(qcrg, o); P.qiac = dev_upload(qiac, o);
   P.qavdw = dev_upload(qavdw, o); P.qbvdw = dev_upload(qbvdw, o); P.sc = dev_upload(sc, o);
   P.qwa = dev_upload(qwa, o); P.qws = dev_upload(qws, o);
-  P.qconn = dev_upload(qconn, o); P.qq = dev_upload(qq, o); P.qq_el = dev_upload(qq_el, o);
+  P.qq = dev_upload(qq, o); P.qq_el = dev_upload(qq_el, o);
   P.bij = dev_upload(bij, o); P.bpar = dev_upload(bpar, o); P.aijk = dev_upload(aijk, o); P.apar = dev_upload(apar, o); P.aub = dev_upload(aub, o);
   P.tijkl = dev_upload(tijkl, o); P.tpar = dev_upload(tpar, o); P.iijkl = dev_upload(iijkl, o); P.ipar = dev_upload(ipar, o);
   P.qbij = dev_upload(qbij, o); P.qb_on = dev_upload(qb_on, o); P.qbpar = dev_upload(qbpar, o);
@@ -1483,7 +1497,8 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   pwg_off.push_back((int)pwa.size());
   P.pwa = dev_upload(pwa, o);
   P.pwg_off = dev_upload(pwg_off, o);
-  P.qp = dev_alloc<int4>(qp_tot, o); P.qw = dev_alloc<int>(qw_tot, o);
+  P.qp = dev_alloc<int>(qp_tot, o);
+  P.qp_code = dev_upload(qp_code, o); P.qw = dev_alloc<int>(qw_tot, o);
   // water-water staging chunk: a multiple of 32 waters, two blocks per SM
   const int rec_words = B.opt.precision == QB_MIXED ? WatRec<true>::words : WatRec<false>::words;
   const int chunk_max = WW_STAGE_BYTES / (16 * rec_words) / 32 * 32;

@@ -51,7 +51,7 @@ struct QwState {
 // Per-system record (read-only on the device during a run).
 struct SysDev {
   int aoff, natom, nsol, nwat, woff, coff, ncgp, ncgp_sol;
-  int qoff, nq, S, natyps, ljoff, qlib_off, sc_off, qconn_off;
+  int qoff, nq, S, natyps, ljoff, qlib_off, sc_off;
   int lrft_off, nlrft;        // LRF gather tiles (group ranges)
   // static term ranges (global offsets into term arrays)
   int b_off, nb, nb_sol, a_off, na, na_sol, t_off, nt, nt_sol, i_off, ni, ni_sol;
@@ -62,7 +62,8 @@ struct SysDev {
   int rs_off, nrs, rp_off, nrp, rd_off, nrd, ra_off, nra, rw_off, nrw;
   // dynamic list segments
   long long pp_off;
-  int pp_cap, qp_off, qp_cap, qw_off, qw_cap;
+  int pp_cap, qp_off, qw_off, qw_cap;
+  long long qp_code_off;
   int near_off, nearw_off;    // words of the group-pair bits
   int csoff;                  // first solute group of this system among all systems' solute groups
   int ff_type, use_lrf, qvdw, wpol, nshell, iac_ow, separate_scaling, has_shake, detail_temps;
@@ -98,7 +99,7 @@ struct SysDev {
 struct SysState {
   double Tscale_sol, Tscale_solv, Temp, Tfree, Tfree_sol, Tfree_solv, kinetic;
   float theta_corr[MAX_SHELLS], avtheta[MAX_SHELLS], avn_insh[MAX_SHELLS];
-  int istep, status, pp_n, pw_n, qp_n, qw_n, lists_built, hist_n[2];
+  int istep, status, pp_n, pw_n, qp_n, qp_atoms, qw_n, lists_built, hist_n[2];
   // status as of the start of the current step (k_finish copies status into
   // it): the kernels that move atoms read this word, so an error raised in
   // the middle of a step takes effect for every kernel from the next step on
@@ -154,7 +155,6 @@ struct DevPtrs {
   double *sc;               // per system segments [sc_off + (iq*(natyps+nq)+col)*S + st]
   QwAtom *qwa;              // [gq]
   QwState *qws;             // [gq*MAXS + st]
-  int8_t *qconn;            // per system segments [qconn_off + (st*nsol + i)*nq + iq]
   int4 *qq;                 // (gq, gj, gjq or -1, lj | st<<8)
   double *qq_el;
   // bonded terms (global atom indices)
@@ -198,7 +198,8 @@ struct DevPtrs {
   int *pwg_n, pwg_cap;                     // waters listed per solute group
   struct PwAtom *pwa;                      // non-Q atoms of each solute group (static)
   int *pwg_off;                            // [solute group] first entry in pwa; one extra at the end
-  int4 *qp;                                // gq, j, lj, qlj
+  int *qp;                                 // solute atoms listed with the Q atoms
+  uint8_t *qp_code;                        // [qp_code_off + solute atom * nq + iq]: LJ code; 0: not with any Q atom
   int *qw;                                 // water O atoms
   uint16_t *ww;                            // [gw*ww_cap + k] local water index
   int *ww_mid;                             // per water: list entries below its own index (ascending lists)

@@ -118,15 +118,19 @@ __global__ void k_cgp_centers(DevPtrs P, int force) {
 
 // The any-atom cut-off tests of iuse_switch_atom 0 (nbpplis2_lrf md.f90:4955,
 // nbpwlis2_lrf 6500, nbqplis2 7700), FP64 as the reference.
-// Solute group pair: inside when any atom pair of the two groups is within rc2.
+// Solute group pair: inside when any atom pair of the two groups is within
+// rc2; the whole warp takes one pair of groups, lanes its atom pairs.
 __device__ __forceinline__ bool groups_inside_any(const DevPtrs &P, int gi, int gj, double rc2) {
-  for (int ia = P.cg_first[gi]; ia <= P.cg_last[gi]; ia++) {
-    const double3 xi = ld3(P.x, P.cg_atoms[ia]);
-    for (int ja = P.cg_first[gj]; ja <= P.cg_last[gj]; ja++) {
-      const double3 xj = ld3(P.x, P.cg_atoms[ja]);
+  const int fi = P.cg_first[gi], ni = P.cg_last[gi] - fi + 1, fj = P.cg_first[gj], nj = P.cg_last[gj] - fj + 1;
+  for (int t0 = 0; t0 < ni * nj; t0 += 32) {
+    const int t = t0 + (threadIdx.x & 31);
+    bool in = false;
+    if (t < ni * nj) {
+      const double3 xi = ld3(P.x, P.cg_atoms[fi + t / nj]), xj = ld3(P.x, P.cg_atoms[fj + t % nj]);
       const double dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      if (dx * dx + dy * dy + dz * dz <= rc2) return true;
+      in = dx * dx + dy * dy + dz * dz <= rc2;
     }
+    if (__any_sync(FULL, in)) return true;
   }
   return false;
 }
@@ -853,7 +857,7 @@ __global__ void k_group_near(DevPtrs P, int force) {
   const double3 xs = ld3(P.x, P.cg_sw[gi]);
   for (int base = 0; base < S.ncgp_sol; base += blockDim.x) {
     const int jg = base + threadIdx.x, gj = S.coff + jg;
-    bool inside = jg < S.ncgp_sol;
+    bool inside = jg < S.ncgp_sol, ask = false;
     if (inside) {
       if (S.switch_atoms) {
         double3 xj = ld3(P.x, P.cg_sw[gj]);
@@ -862,8 +866,15 @@ __global__ void k_group_near(DevPtrs P, int force) {
         inside = dx * dx + dy * dy + dz * dz <= S.Rcpp2;
       } else {
         const int reach = groups_reach(P, gi, gj, S.Rcpp2);
-        inside = reach > 0 || (reach == 0 && groups_inside_any(P, gi, gj, S.Rcpp2));
+        inside = reach > 0;
+        ask = reach == 0;
       }
+    }
+    // pairs that only the atoms can tell, one after the other by the whole warp
+    for (unsigned todo = __ballot_sync(FULL, ask); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const bool in = groups_inside_any(P, gi, S.coff + base + (threadIdx.x & ~31) + l, S.Rcpp2);
+      if ((threadIdx.x & 31) == l) inside = in;
     }
     const unsigned bal = __ballot_sync(FULL, inside);
     const int w = jg >> 5;
@@ -977,61 +988,56 @@ __global__ void k_list_pw(DevPtrs P, int force) {
   }
 }
 
-// Q-atom / solute list (nbqplist, md.f90:7875): block per system, threads
-// over solute atoms of groups within Rcq of the solute centre; atoms bonded
-// within 1-3 to any Q atom (in any state) belong to the Q-Q list instead.
-__global__ void k_list_qp(DevPtrs P, int force) {
+// Q-atom / solute list (nbqplist, md.f90:7875): the solute atoms of groups
+// within Rcq of the solute centre; atoms bonded within 1-3 to any Q atom (in
+// any state) belong to the Q-Q list instead (qp_code 0).  Every listed atom
+// pairs with every Q atom, with the LJ codes of P.qp_code.  Block per system,
+// threads over solute atoms, ascending.
+constexpr int QP_LIST_BLOCK = 256;
+
+__global__ void __launch_bounds__(QP_LIST_BLOCK) k_list_qp(DevPtrs P, int force) {
   int s = blockIdx.x;
   const SysDev &S = P.sys[s];
   if (S.nq == 0 || !list_due(P, s, force)) return;
   if (S.qp_once && P.st[s].lists_built) return;
-  __syncthreads();
-  if (threadIdx.x == 0) P.st[s].qp_n = 0;
-  __syncthreads();
+  __shared__ int wcount[QP_LIST_BLOCK / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int n = 0;
   // the list's centre: the solute centre, or in a periodic box the nearest
   // image of the Q switching atom (nbqplist_box, md.f90:8005-8014)
   const double3 xq = S.pbc ? ld3(P.x, S.qswitch) : make_double3(S.xp[0], S.xp[1], S.xp[2]);
   const BoxD bx = box_of(P, s);
-  for (int ig = 0; ig < S.ncgp_sol; ig++) {
-    int gi = S.coff + ig;
-    int sw = P.cg_sw[gi];
-    if (P.flags[sw] & F_EXCL) continue;
-    if (S.switch_atoms) {
-      double3 xs = ld3(P.x, sw);
-      double dx = xs.x - xq.x, dy = xs.y - xq.y, dz = xs.z - xq.z;
-      if (S.pbc) min_image(bx, dx, dy, dz);
-      if (dx * dx + dy * dy + dz * dz > S.Rcq2) continue;
-    } else {
-      if (!group_point_inside_any(P, gi, make_double3(S.xp[0], S.xp[1], S.xp[2]), S.Rcq2)) continue;
-    }
-    int f = P.cg_first[gi], n = P.cg_last[gi] - f + 1;
-    // whole warps per round: a warp reserves its entries with one atomic
-    for (int t0 = 0; t0 < n * S.nq; t0 += blockDim.x) {
-      const int t = t0 + threadIdx.x;
-      bool take = t < n * S.nq;
-      int i = 0, iq = 0, li = 0;
-      if (take) {
-        i = P.cg_atoms[f + t / S.nq];
-        iq = t % S.nq;
-        li = i - S.aoff;
-        for (int st = 0; st < S.S && take; st++)
-          for (int q = 0; q < S.nq; q++)
-            if (P.qconn[S.qconn_off + ((size_t)st * S.nsol + li) * S.nq + q] <= 3) { take = false; break; }
+  for (int a0 = 0; a0 < S.nsol; a0 += QP_LIST_BLOCK) {
+    const int li = a0 + threadIdx.x, i = S.aoff + li;
+    bool ok = li < S.nsol && P.qp_code[S.qp_code_off + (size_t)li * S.nq] != 0;
+    if (ok) {
+      const int gi = P.cgp[i], sw = P.cg_sw[gi];
+      ok = gi - S.coff < S.ncgp_sol && !(P.flags[sw] & F_EXCL);
+      if (ok) {
+        if (S.switch_atoms) {
+          double3 xs = ld3(P.x, sw);
+          double dx = xs.x - xq.x, dy = xs.y - xq.y, dz = xs.z - xq.z;
+          if (S.pbc) min_image(bx, dx, dy, dz);
+          ok = dx * dx + dy * dy + dz * dz <= S.Rcq2;
+        } else {
+          ok = group_point_inside_any(P, gi, make_double3(S.xp[0], S.xp[1], S.xp[2]), S.Rcq2);
+        }
       }
-      const unsigned bal = __ballot_sync(FULL, take);
-      const int lane = threadIdx.x & 31;
-      int first = 0;
-      if (lane == 0 && bal) first = atomicAdd(&P.st[s].qp_n, __popc(bal));
-      first = __shfl_sync(FULL, first, 0);
-      if (!take) continue;
-      int qa = P.iqseq[S.qoff + iq];
-      int lj = ljcode(P, S, i, qa);
-      if (P.qconn[S.qconn_off + ((size_t)0 * S.nsol + li) * S.nq + iq] == 4) lj = 3;
-      int qlj = lj == 2 ? 1 : lj;
-      int k = first + __popc(bal & ((1u << lane) - 1u));
-      if (k < S.qp_cap) P.qp[S.qp_off + k] = make_int4(S.qoff + iq, i, lj, qlj);
-      else set_status(&P.st[s], QB_ERR_LIST_OVERFLOW);
     }
+    const unsigned bal = __ballot_sync(FULL, ok);
+    if (lane == 0) wcount[wid] = __popc(bal);
+    __syncthreads();
+    int k = n + __popc(bal & ((1u << lane) - 1u));
+    for (int w = 0; w < QP_LIST_BLOCK / 32; w++) {
+      if (w < wid) k += wcount[w];
+      n += wcount[w];
+    }
+    if (ok) P.qp[S.qp_off + k] = i;      // at most nsol entries, the segment's size
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    P.st[s].qp_atoms = n;
+    P.st[s].qp_n = n * S.nq;
   }
 }
 
@@ -1102,7 +1108,6 @@ __global__ void k_lists_end(DevPtrs P, int force) {
   SysState &st = P.st[s];
   const SysDev &S = P.sys[s];
   if (st.pp_n > S.pp_cap) st.pp_n = S.pp_cap;
-  if (st.qp_n > S.qp_cap) st.qp_n = S.qp_cap;
   st.lists_built = 1;
 }
 
@@ -1755,33 +1760,49 @@ __global__ void __launch_bounds__(PW_BLOCK) k_nb_pw(DevPtrs P) {
   }
 }
 
-// nonbond_qp (md.f90:10980) / nonbond_qp_qvdw (11138): one thread per pair,
-// all states in the thread.
+// nonbond_qp (md.f90:10980) / nonbond_qp_qvdw (11138), all states in the
+// thread.  A block takes 32 listed solute atoms: lanes are atoms, its 8 warps
+// share the Q atoms out; a Q atom's gradient is summed over the warp and added
+// with one atomic per component, the atoms' gradients and the energies meet in
+// shared memory.  A thread per pair with both ends added by atomics put every
+// pair's three Q-atom components on the same few addresses: with 18,500 pairs
+// (the polymer sphere) the solute kernel took 50 us, this way 21.
+constexpr int QP_WARPS = 8;
+
 template <int NSC>
 __device__ __forceinline__ void nb_qp_body(DevPtrs &P, int bx, int s, int gx) {
   const SysDev &S = P.sys[s];
-  int n = P.st[s].qp_n;
+  const int n = P.st[s].qp_atoms;
   const int NS = NSC > 0 ? NSC : S.S;
   const int ncol = S.natyps + S.nq;
   constexpr int NA = NSC > 0 ? NSC : MAXS;
+  __shared__ double red[QP_WARPS][3][32];
+  __shared__ double ered[QP_WARPS][2 * NA];
+  if (bx * 32 >= n) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double el[NA], vdw[NA];
 #pragma unroll
   for (int st = 0; st < NA; st++) { el[st] = 0; vdw[st] = 0; }
-  for (int k0 = bx * blockDim.x; k0 < n; k0 += gx * blockDim.x) {
-    int k = k0 + threadIdx.x;
-    if (k < n) {
-      int4 p = P.qp[S.qp_off + k];
-      int gq = p.x, j = p.y, lj = p.z, qlj = p.w;
-      int i = P.iqseq[gq], iq = gq - S.qoff;
-      double3 xi = ld3(P.x, i), xj = ld3(P.x, j);
-      double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
-      if (S.pbc) {
-        // nonbond_qp_box (md.f90:11060-11068): the image of j's group
-        // switching atom nearest the Q switching atom
-        const double3 a = ld3(P.x, S.qswitch), b = ld3(P.x, switch_of(P, j));
-        const double3 t = image_shift(box_of(P, s), b.x - a.x, b.y - a.y, b.z - a.z);
-        dx -= t.x; dy -= t.y; dz -= t.z;
-      }
+  for (int k0 = bx * 32; k0 < n; k0 += gx * 32) {
+    const bool act = k0 + lane < n;
+    const int j = P.qp[S.qp_off + (act ? k0 + lane : k0)];
+    const double3 xj = ld3(P.x, j);
+    const float cj = P.crg[j];
+    const int tj = P.iac[j];
+    const uint8_t *code = P.qp_code + S.qp_code_off + (size_t)(j - S.aoff) * S.nq;
+    double3 im = make_double3(0, 0, 0);
+    if (S.pbc) {
+      // nonbond_qp_box (md.f90:11060-11068): the image of j's group
+      // switching atom nearest the Q switching atom
+      const double3 a = ld3(P.x, S.qswitch), b = ld3(P.x, switch_of(P, j));
+      im = image_shift(box_of(P, s), b.x - a.x, b.y - a.y, b.z - a.z);
+    }
+    double fj[3] = {0.0, 0.0, 0.0};
+    for (int iq = warp; iq < S.nq; iq += QP_WARPS) {
+      const int gq = S.qoff + iq, i = P.iqseq[gq];
+      const int lj = code[iq], qlj = lj == 2 ? 1 : lj;
+      const double3 xi = ld3(P.x, i);
+      double dx = xj.x - xi.x - im.x, dy = xj.y - xi.y - im.y, dz = xj.z - xi.z - im.z;
       double r2 = dx * dx + dy * dy + dz * dz;
       double dvsum = 0;
       if (!S.qvdw) {
@@ -1792,41 +1813,66 @@ __device__ __forceinline__ void nb_qp_body(DevPtrs &P, int bx, int s, int gx) {
         lj_pair(S.arith, P.lja[3 * i + lj - 1], P.lja[3 * j + lj - 1], P.ljb[3 * i + lj - 1], P.ljb[3 * j + lj - 1],
                 aLJ, bLJ);
         for (int st = 0; st < NS; st++) {
-          float qq = P.qcrg[gq * MAXS + st] * P.crg[j];
+          float qq = P.qcrg[gq * MAXS + st] * cj;
           double Vel = (double)qq * r;
           if (lj == 3) Vel = Vel * S.el14;
           double Va = aLJ * r6 * r6, Vb = bLJ * r6;
           dvsum += r2 * (-Vel - 12. * Va + 6. * Vb) * S.lambda[st];
-          el[st] += Vel;
-          vdw[st] += Va - Vb;
+          if (act) { el[st] += Vel; vdw[st] += Va - Vb; }
         }
       } else {
         double r6 = r2 * r2 * r2;
         double r = rsqrt(r2);
         r2 = r * r;
-        int tj = P.iac[j];
+        const double aj = P.lja[3 * j + qlj - 1], bj = P.ljb[3 * j + qlj - 1];
         for (int st = 0; st < NS; st++) {
           int ti = P.qiac[gq * MAXS + st];
           double aLJ, bLJ;
-          lj_pair(S.arith, P.qavdw[S.qlib_off + 3 * ti + qlj - 1], P.lja[3 * j + lj - 1],
-                  P.qbvdw[S.qlib_off + 3 * ti + qlj - 1], P.ljb[3 * j + lj - 1], aLJ, bLJ);
-          float qq = P.qcrg[gq * MAXS + st] * P.crg[j];
+          lj_pair(S.arith, P.qavdw[S.qlib_off + 3 * ti + qlj - 1], aj, P.qbvdw[S.qlib_off + 3 * ti + qlj - 1], bj, aLJ,
+                  bLJ);
+          float qq = P.qcrg[gq * MAXS + st] * cj;
           double Vel = (double)qq * r;
           if (lj == 3) Vel = Vel * S.el14;
           double r6sc = r6 + P.sc[S.sc_off + ((size_t)iq * ncol + tj) * NS + st];
           double Va = aLJ / (r6sc * r6sc), Vb = bLJ / r6sc;
           dvsum += r2 * (-Vel - (12. * Va - 6. * Vb) * (r6 / r6sc)) * S.lambda[st];
-          el[st] += Vel;
-          vdw[st] += Va - Vb;
+          if (act) { el[st] += Vel; vdw[st] += Va - Vb; }
         }
       }
-      atomic_add3(P.d, i, -dvsum * dx, -dvsum * dy, -dvsum * dz);
-      atomic_add3(P.d, j, dvsum * dx, dvsum * dy, dvsum * dz);
+      if (!act) dvsum = 0.0;
+      const double f[3] = {dvsum * dx, dvsum * dy, dvsum * dz};
+      double t[3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        fj[c] += f[c];
+        t[c] = warp_sum(-f[c]);
+      }
+      const double g = lane == 0 ? t[0] : lane == 1 ? t[1] : t[2];
+      if (lane < 3 && g != 0.0) atomicAdd(&P.d[i].x + lane, g);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 3; c++) red[warp][c][lane] = fj[c];
+    __syncthreads();
+    if (warp < 3 && act) {
+      double f = 0.0;
+#pragma unroll
+      for (int w = 0; w < QP_WARPS; w++) f += red[w][warp][lane];
+      atomicAdd(&P.d[j].x + warp, f);
     }
   }
-  for (int st = 0; st < NS; st++) {
-    warp_add(&P.EQ[((size_t)s * MAXS + st) * QB_NEQ + QB_EQ_QP_EL], el[st]);
-    warp_add(&P.EQ[((size_t)s * MAXS + st) * QB_NEQ + QB_EQ_QP_VDW], vdw[st]);
+#pragma unroll
+  for (int st = 0; st < NA; st++) {
+    if (st >= NS) break;
+    const double a = warp_sum(el[st]), b = warp_sum(vdw[st]);
+    if (lane == 0) { ered[warp][2 * st] = a; ered[warp][2 * st + 1] = b; }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < 2 * NS) {
+    double e = 0.0;
+    for (int w = 0; w < QP_WARPS; w++) e += ered[w][threadIdx.x];
+    atomicAdd(&P.EQ[((size_t)s * MAXS + (threadIdx.x >> 1)) * QB_NEQ +
+                    ((threadIdx.x & 1) ? QB_EQ_QP_VDW : QB_EQ_QP_EL)], e);
   }
 }
 
@@ -2869,7 +2915,7 @@ __device__ __forceinline__ void prestrain_body(DevPtrs &P, int s) {
 struct SoluteGrid { int pp, qp, bonded, qq, qb, pre; };
 
 template <int NSC>
-__global__ void __launch_bounds__(256) k_solute_terms(DevPtrs P, SoluteGrid G) {
+__global__ void __launch_bounds__(32 * QP_WARPS) k_solute_terms(DevPtrs P, SoluteGrid G) {
   int b = blockIdx.x;
   const int s = blockIdx.y;
   if (b < G.pp) { nb_pp_body(P, b, s, G.pp); return; }
