@@ -659,6 +659,7 @@ struct Batch {
     if (!mc_x) {
       mc_x = dev_alloc<double4>(ax, owned);
       mc_lrf = dev_alloc<double>(std::max<size_t>(lx, 1), owned);
+      CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));   // their zeroing, which this stream does not wait for
     }
     std::vector<double> dV(nsys, 0.0), oldV(nsys, 0.0);
     for (int s : live) {
@@ -2038,7 +2039,11 @@ __global__ void k_atoms_to_xyz(double *dst, const double4 *src, int n) {
 }
 
 static double *xyz_scratch(Batch &B) {
-  if (!B.xyz) B.xyz = qb::dev_alloc<double>(3 * (size_t)std::max(B.P.natoms_tot, 1), B.owned);
+  if (!B.xyz) {
+    B.xyz = qb::dev_alloc<double>(3 * (size_t)std::max(B.P.natoms_tot, 1), B.owned);
+    // the zeroing runs on the default stream, which the batch's stream does not wait for
+    CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  }
   return B.xyz;
 }
 
