@@ -76,6 +76,8 @@ struct KernelStat { double ms = 0; long long launches = 0; };
 // Blocks per SM (of the one-part form) up to which the mixed LRF gather splits
 // its sums over a block's warps.
 constexpr int LRFX_CS_BLOCKS = 1;
+// Most waters of a batch that takes the water-water kernels without staging.
+constexpr int WWD_MAX_WATERS = 4096;
 
 struct Batch {
   int nsys = 0;
@@ -97,6 +99,12 @@ struct Batch {
   struct McState { bool started = false; int irand = 0; long long tries = 0, accepted = 0; };
   std::vector<McState> mc;
   int ww_wpb = WW_WPB;          // waters per block of the water-water kernels
+  // the water-water kernels without staging (small batches, one chunk): up to
+  // WWD_MAX_WATERS.  FP64 kernel staged / direct: 2 windows 14 / 8 us, 3 14 / 14, 5
+  // 23 / 18, 8 and more the same, and the step gains only where the others
+  // leave it SMs (1 to 3 windows)
+  bool ww_direct = false;
+  int ww_wpb0 = WW_WPB;         // the default of ww_wpb for this batch
   int max_nshell = 0;           // polarisation shells of the batch's systems, at most
   // the water pass takes a thread per water atom when that many threads
   // still fit on the GPU at once (small batches), else one per water
@@ -116,6 +124,7 @@ struct Batch {
   size_t watpol_smem = 0;
   // k_nb_qw: warps sharing the Q atoms of one group of 32 waters, warps per block
   int qw_groups = 1, qw_warps = 4;
+  bool ww_direct_fits() const { return P.ww_nch == 1 && P.nwat_tot <= WWD_MAX_WATERS; }
   // As many warps (1, 2, 4 or 8) as keep the launch within 16 warps per SM.
   // Kernel time with 1 / 2 / 4 / 8: 33 water groups (one window) 12 / 8 / 6 /
   // 5.6 us; 693 (21 windows, FP32) 10 / 8 / 11 / 14; 1,353 (41 windows) 15 /
@@ -155,7 +164,7 @@ struct Batch {
     if (stream) cudaStreamSynchronize(stream);
     if (pinned) cudaFreeHost(pinned);
     drop_graphs();
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < NSIDE; k++) {
       if (side[k]) { cudaStreamSynchronize(side[k]); cudaStreamDestroy(side[k]); }
       if (ev_join[k]) cudaEventDestroy(ev_join[k]);
     }
@@ -232,7 +241,7 @@ struct Batch {
     };
     // the any-atom LRF windows read the group-pair bits
     if (any_any_atom) solute_lists();
-    fork_streams();
+    fork_streams(2);
     if (any_lrf) {
       launch("lrf_gather", [&] {
         if (opt.precision == QB_MIXED) {
@@ -258,7 +267,7 @@ struct Batch {
       launch("list_qp", [&] { k_list_qp<<<nsys, QP_LIST_BLOCK, 0, stream>>>(p, force); });
       if (max_nwat > 0) launch("list_qw", [&] { k_list_qw<<<nsys, 256, 0, stream>>>(p, force); });
     }
-    join_streams();
+    join_streams(2);
     launch("lists_end", [&] { k_lists_end<<<cdiv(nsys, 128), 128, 0, stream>>>(p, force); });
     check_launch("list kernels");
   }
@@ -270,13 +279,14 @@ struct Batch {
   }
 
   // Side streams of the force fork: after the water pass the force kernels of
-  // a step (all adding with atomics) run on three streams and join before the
+  // a step (all adding with atomics) run on four streams and join before the
   // leap-frog.  Profiling keeps them on the main stream, one at a time.
-  cudaStream_t side[2] = {nullptr, nullptr};
-  cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
+  static constexpr int NSIDE = 3;
+  cudaStream_t side[NSIDE] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[NSIDE] = {};
 
   void make_side_streams() {
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < NSIDE; k++) {
       CUDA_TRY(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
       CUDA_TRY(cudaEventCreateWithFlags(&ev_join[k], cudaEventDisableTiming));
     }
@@ -321,14 +331,15 @@ struct Batch {
     if (lrfx_cs == 4) k_lrf_gather_x2<BOX, ANY, 4><<<g, LRFX_BLOCK, 0, st>>>(P, force);
     else k_lrf_gather_x2<BOX, ANY, 1><<<g, LRFX_BLOCK, 0, st>>>(P, force);
   }
-  void fork_streams() {
+  // the first n of them
+  void fork_streams(int n) {
     if (!forking()) return;
     CUDA_TRY(cudaEventRecord(ev_fork, stream));
-    for (int k = 0; k < 2; k++) CUDA_TRY(cudaStreamWaitEvent(side[k], ev_fork, 0));
+    for (int k = 0; k < n; k++) CUDA_TRY(cudaStreamWaitEvent(side[k], ev_fork, 0));
   }
-  void join_streams() {
+  void join_streams(int n) {
     if (!forking()) return;
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < n; k++) {
       CUDA_TRY(cudaEventRecord(ev_join[k], side[k]));
       CUDA_TRY(cudaStreamWaitEvent(stream, ev_join[k], 0));
     }
@@ -369,7 +380,8 @@ struct Batch {
       }
     }
     cudaStream_t s1 = forking() ? side[0] : stream, s2 = forking() ? side[1] : stream;
-    fork_streams();
+    fork_streams(3);
+    cudaStream_t s3 = forking() ? side[2] : stream;
     // solute terms in one launch (nonbond_pp, nonbond_qp, bonded, nonbond_qq,
     // Q bonded, restraints)
     {
@@ -403,31 +415,33 @@ struct Batch {
         else k_nb_pw<false><<<g, PW_BLOCK, 0, s1>>>(p);
       });
     if (max_nwat > 0) {
-      dim3 gw(p.n_ww_tiles, 1);
       const int wpb = ww_wpb;
-      size_t smem = (size_t)p.ww_chunk * (fast_ww ? WatRec<true>::words : WatRec<false>::words) * sizeof(float4);
-      // hydrogen LJ: the whole batch takes the variant (exact zeros for systems without)
-      if (fast_ww && any_hlj) {
-        launch("nb_ww", [&] { k_nb_ww<true, true><<<gw, WW_BLOCK, smem, stream>>>(p, wpb); });
-      } else if (fast_ww) {
+      const size_t smem32 = (size_t)p.ww_chunk * WatRec<true>::words * sizeof(float4);
+      const size_t smem = (size_t)p.ww_chunk * WatRec<false>::words * sizeof(float4);
+      const dim3 gw(p.n_ww_tiles), gd(p.n_wd_tiles);
+      const int td = 32 * WWD_WATERS;
+      // the packed forces, or hydrogen LJ's FP32 form (the whole batch takes
+      // the variant: exact zeros for systems without)
+      if (fast_ww && any_hlj)
+        launch("nb_ww", [&] { k_nb_ww<true, true><<<gw, WW_BLOCK, smem32, stream>>>(p, wpb); });
+      else if (mixed && !any_hlj)
         launch("nb_ww_x2", [&] {
-          if (any_box) k_nb_ww_x2<true><<<gw, WWX_BLOCK, smem, stream>>>(p, wpb);
-          else k_nb_ww_x2<false><<<gw, WWX_BLOCK, smem, stream>>>(p, wpb);
-        });
-      } else if (any_hlj) {
-        launch("nb_ww", [&] { k_nb_ww<false, true><<<gw, WW_BLOCK, smem, stream>>>(p, wpb); });
-      } else if (mixed) {
-        // a recording step of the mixed engine: the packed kernel's forces,
-        // the energies in FP64 over each pair once
-        const size_t smem32 = (size_t)p.ww_chunk * WatRec<true>::words * sizeof(float4);
-        launch("nb_ww_x2", [&] {
-          if (any_box) k_nb_ww_x2<true><<<gw, WWX_BLOCK, smem32, stream>>>(p, wpb);
+          if (ww_direct && any_box) k_nb_ww_x2_direct<true><<<gd, td / 2, 0, stream>>>(p);
+          else if (ww_direct) k_nb_ww_x2_direct<false><<<gd, td / 2, 0, stream>>>(p);
+          else if (any_box) k_nb_ww_x2<true><<<gw, WWX_BLOCK, smem32, stream>>>(p, wpb);
           else k_nb_ww_x2<false><<<gw, WWX_BLOCK, smem32, stream>>>(p, wpb);
         });
-        launch("nb_ww", [&] { k_nb_ww<false, false, true><<<gw, WW_BLOCK, smem, stream>>>(p, wpb); });
-      } else {
-        launch("nb_ww", [&] { k_nb_ww<false, false><<<gw, WW_BLOCK, smem, stream>>>(p, wpb); });
-      }
+      // FP64: every step of the FP64 engine; of the mixed one the recording
+      // steps' energies (over each pair once, beside the packed forces)
+      if (!fast_ww)
+        launch("nb_ww", [&] {
+          if (any_hlj && ww_direct) k_nb_ww_direct<true><<<gd, td, 0, stream>>>(p);
+          else if (any_hlj) k_nb_ww<false, true><<<gw, WW_BLOCK, smem, stream>>>(p, wpb);
+          else if (mixed && ww_direct) k_nb_ww_direct<false, true><<<gd, td, 0, stream>>>(p);
+          else if (mixed) k_nb_ww<false, false, true><<<gw, WW_BLOCK, smem, stream>>>(p, wpb);
+          else if (ww_direct) k_nb_ww_direct<false><<<gd, td, 0, stream>>>(p);
+          else k_nb_ww<false, false><<<gw, WW_BLOCK, smem, stream>>>(p, wpb);
+        });
       if (any_q && p.n_qw_tiles > 0) launch("nb_qw", [&] {
         const int g = p.n_qw_tiles, qg = qw_groups, nt = 32 * qw_warps;
         if (any_hlj) { k_nb_qw<0, true><<<g, nt, 0, s2>>>(p, qg); return; }   // the generic state count only
@@ -452,9 +466,9 @@ struct Batch {
     if (max_nsol > 0)
       launch("atom_terms", [&] { k_atom_terms<<<dim3(cdiv(max_nsol, 128), nsys), 128, 0, s1>>>(p); });
     if (any_wpol) {
-      launch("watpol", [&] { k_watpol<<<dim3(std::max(max_nshell, 1), nsys), WPOL_BLOCK, watpol_smem, s2>>>(p); });
+      launch("watpol", [&] { k_watpol<<<dim3(std::max(max_nshell, 1), nsys), WPOL_BLOCK, watpol_smem, s3>>>(p); });
     }
-    join_streams();
+    join_streams(3);
     check_launch("force kernels");
   }
 
@@ -790,14 +804,14 @@ struct Batch {
     // other atoms leapfrog, then the general SHAKE; the two paths move
     // disjoint atoms
     const bool fused = any_shake && p.nsh3 > 0;
-    if (fused) fork_streams();
+    if (fused) fork_streams(1);
     if (fused)
       launch("leapfrog_shake3", [&] { k_leapfrog_shake3<<<cdiv(p.nsh3, 128), 128, 0, stream>>>(p); });
     cudaStream_t sl = fused && forking() ? side[0] : stream;
     if (p.n_lf > 0) launch("leapfrog", [&] { k_leapfrog<<<cdiv(p.n_lf, 256), 256, 0, sl>>>(p); });
     if (any_shake && p.nshg > 0)
       launch("shake_general", [&] { k_shake_general<<<p.nshg, SHG_BLOCK, p.shg_smem, sl>>>(p); });
-    if (fused) join_streams();
+    if (fused) join_streams(1);
     launch("finish", [&] { k_finish<<<nsys, 32, 0, stream>>>(p, 1); });
     check_launch("step kernels");
   }
@@ -918,6 +932,13 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       lx.push_back(i < V.nat_solute ? V.listex_bits[i] : 0u);
       l14.push_back(i < V.nat_solute ? V.list14_bits[i] : 0u);
     }
+    {
+      std::vector<char> grouped(V.natom, 0);
+      for (int g = 0; g < V.ncgp; g++)
+        for (int a = V.cgp_first[g]; a <= V.cgp_last[g]; a++) grouped[V.cgpatom[a]] = 1;
+      for (int i = 0; i < V.nat_solute; i++)
+        if (!grouped[i]) flags[aoff + i] |= F_NOGRP;
+    }
     for (int k = 0; k < V.natyps * V.natyps; k++) ljcod.push_back(V.ljcod[k]);
     exl_at.resize(x.size());
     l14_at.resize(x.size());
@@ -982,7 +1003,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     S.qp_code_off = (long long)qp_code.size();
     if (V.nqat > 0)
       for (int i = 0; i < V.nat_solute; i++) {
-        bool take = true;
+        bool take = !(flags[aoff + i] & F_NOGRP);
         for (int st = 0; st < V.nstates && take; st++)
           for (int q = 0; q < V.nqat; q++)
             if (V.qconn[((size_t)st * V.nat_solute + i) * V.nqat + q] <= 3) { take = false; break; }
@@ -1546,6 +1567,15 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     B.ww_tiles_cap = cap;
     P.ww_tiles = dev_alloc<int2>((size_t)cap, o);
     set_ww_tiles(B, B.ww_wpb);
+    B.ww_wpb0 = B.ww_wpb;
+  }
+  {
+    std::vector<int2> wd;
+    for (int s = 0; s < n; s++)
+      for (int i0 = 0; i0 < B.sysh[s].nwat; i0 += WWD_WATERS) wd.push_back(make_int2(s, i0));
+    P.n_wd_tiles = (int)wd.size();
+    P.wd_tiles = dev_upload(wd, o);
+    B.ww_direct = B.ww_direct_fits();
   }
   P.ww_cap = ww_cap;
   P.ww = dev_alloc<uint16_t>((size_t)std::max(woff, 1) * ww_cap, o);
@@ -1809,11 +1839,15 @@ void set_tuning(Batch &B, const qb_tuning &t, bool share) {
   if (t.water_pass_per_atom != 0 && t.water_pass_per_atom != 1) fail(QB_ERR_ARG, "water_pass_per_atom must be 0 or 1");
   CUDA_TRY(cudaStreamSynchronize(B.stream));
   B.drop_graphs();
+  const bool staged = t.ww_chunk != B.P.ww_chunk || t.ww_waters_per_block != B.ww_wpb;
   B.set_lrf_tpb(t.lrf_tiles_per_block, share);
   B.P.ww_chunk = t.ww_chunk;
   B.P.ww_nch = (std::max(B.max_nwat, 1) + t.ww_chunk - 1) / t.ww_chunk;
   B.streams_on = t.side_streams != 0;
   if (t.ww_waters_per_block != B.ww_wpb) set_ww_tiles(B, t.ww_waters_per_block);
+  // a chosen chunk or block size is one of the staged kernels'; the defaults
+  // leave small batches without staging
+  if (staged) B.ww_direct = t.ww_chunk == B.ww_chunk_max && t.ww_waters_per_block == B.ww_wpb0 && B.ww_direct_fits();
   B.water_atom_threads = t.water_pass_per_atom != 0;
   B.lists_stale = true;   // the water-water split counts depend on the chunk
 }

@@ -23,8 +23,9 @@ constexpr int LRF_STRIDE = 24;
 constexpr int MAX_SHELLS = 4;
 // one history record: step, E[QB_NE], EQ[MAXS*QB_NEQ], r_kl of the off-diagonal functions [MAXS]
 constexpr int HIST_REC = 1 + QB_NE + MAXS * QB_NEQ + MAXS;
-// F_SHAKE: in a SHAKE constraint; F_SH3: in a 3-constraint molecule, moved by k_leapfrog_shake3
-enum AtomFlags : uint8_t { F_EXCL = 1, F_SHELL = 2, F_HEAVY = 4, F_SHAKE = 8, F_SH3 = 16 };
+// F_SHAKE: in a SHAKE constraint; F_SH3: in a 3-constraint molecule, moved by k_leapfrog_shake3;
+// F_NOGRP: a solute atom in no charge group
+enum AtomFlags : uint8_t { F_EXCL = 1, F_SHELL = 2, F_HEAVY = 4, F_SHAKE = 8, F_SH3 = 16, F_NOGRP = 32 };
 
 // A non-Q atom of a solute charge group with its interaction parameters for
 // the water O and H sites: LJ products A(O), B(O), A(H), B(H) and single
@@ -215,6 +216,8 @@ struct DevPtrs {
   int ww_cap, ww_chunk, ww_nch;
   int2 *ww_tiles;                          // water-water force blocks: (system, first water)
   int n_ww_tiles;
+  int2 *wd_tiles;                          // blocks of the kernels for small batches (WWD_WATERS waters)
+  int n_wd_tiles;
   int lrf_tpb, lrf_sub;                    // source tiles swept by one block of the LRF gather; blocks sharing a tile
   // energies
   double *kin;                             // [s*4] kinetic energy of this step: solute all, free, solvent all, free

@@ -900,7 +900,7 @@ __global__ void __launch_bounds__(PP_BLOCK) k_list_pp(DevPtrs P, int force) {
   const int i = S.aoff + li, gi = P.cgp[i], ig = gi - S.coff;
   const unsigned *near = P.near + S.near_off + (size_t)ig * ((S.ncgp_sol + 31) / 32);
   int first = 0, cnt = 0;
-  if (P.iq[i] < 0 && ig < S.ncgp_sol && !(P.flags[P.cg_sw[gi]] & F_EXCL)) {
+  if (P.iq[i] < 0 && ig < S.ncgp_sol && !(P.flags[i] & F_NOGRP) && !(P.flags[P.cg_sw[gi]] & F_EXCL)) {
     for (int pass = 0; pass < 2; pass++) {
       int n = 0;
       for (int base = 0; base < S.nsol; base += 32) {
@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(PP_BLOCK) k_list_pp(DevPtrs P, int force) {
         if (ok) {
           const int gj = P.cgp[j], jg = gj - S.coff;
           ok = jg < S.ncgp_sol && ((near[jg >> 5] >> (jg & 31)) & 1u) && P.iq[j] < 0 &&
-               !(P.flags[P.cg_sw[gj]] & F_EXCL);
+               !(P.flags[j] & F_NOGRP) && !(P.flags[P.cg_sw[gj]] & F_EXCL);
           if (ok) {
             lj = ljcode(P, S, i, j);
             ok = !zero_pair(P, i, j, lj) && !excluded_pair(P, S, i, j);
@@ -1467,6 +1467,37 @@ __device__ __forceinline__ void ww_force_x2(const WwI2 &I, const float4 j0, cons
   for (int c = 0; c < 3; c++) gO[c].x = fmaf(w, d[c], gO[c].x);
 }
 
+__device__ __forceinline__ void ww_load_i(const float4 *ri, WwI2 &I) {
+  const float4 a = ri[0], b = ri[1], e = ri[2];
+  I.hO[0] = a.x; I.hO[1] = a.y; I.hO[2] = a.z;
+  I.lO[0] = a.w; I.lO[1] = b.x; I.lO[2] = b.y;
+  I.nrH[0] = make_float2(-b.z, -b.w); I.nrH[1] = make_float2(-e.x, -e.y); I.nrH[2] = make_float2(-e.z, -e.w);
+#pragma unroll
+  for (int q = 0; q < 3; q++) I.nrHs[q] = make_float2(I.nrH[q].y, I.nrH[q].x);
+}
+
+// The gradient of a water (O at atom o), reduced over the half-warp that
+// shared its list and added: O, H1, H2, x y z each.
+__device__ __forceinline__ void ww_store_i(const DevPtrs &P, int o, int hl, unsigned hmask, const float2 *gO,
+                                           const float2 *gH, const float2 *gHs) {
+  float g[9];
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    g[q] = gO[q].x + gO[q].y;
+    g[3 + q] = gH[q].x + gHs[q].y;
+    g[6 + q] = gH[q].y + gHs[q].x;
+  }
+#pragma unroll
+  for (int q = 0; q < 9; q++) {
+#pragma unroll
+    for (int u = 8; u > 0; u >>= 1) g[q] += __shfl_xor_sync(hmask, g[q], u);
+  }
+  float f = g[0];
+#pragma unroll
+  for (int q = 1; q < 9; q++) f = hl == q ? g[q] : f;
+  if (hl < 9) atomicAdd(&P.d[o + hl / 3].x + hl % 3, (double)f);
+}
+
 // nonbond_ww_spc (md.f90:11823) forces of the mixed-precision engine on steps
 // that record no energies: the list walk of k_nb_ww (half a warp per water,
 // the system's records staged in shared memory chunk by chunk) with the pair
@@ -1541,14 +1572,7 @@ __global__ void __launch_bounds__(WWX_BLOCK, 2) k_nb_ww_x2(DevPtrs P, int wpb) {
       const uint16_t *nb = P.ww + (size_t)gw * P.ww_cap;
       const float4 *ri = (iw >= c0 && iw < c0 + cn) ? wsm + (iw - c0) * W : rec + (size_t)iw * W;
       WwI2 I;
-      {
-        const float4 a = ri[0], b = ri[1], e = ri[2];
-        I.hO[0] = a.x; I.hO[1] = a.y; I.hO[2] = a.z;
-        I.lO[0] = a.w; I.lO[1] = b.x; I.lO[2] = b.y;
-        I.nrH[0] = make_float2(-b.z, -b.w); I.nrH[1] = make_float2(-e.x, -e.y); I.nrH[2] = make_float2(-e.z, -e.w);
-#pragma unroll
-        for (int q = 0; q < 3; q++) I.nrHs[q] = make_float2(I.nrH[q].y, I.nrH[q].x);
-      }
+      ww_load_i(ri, I);
       float2 gO[3], gH[3], gHs[3];
 #pragma unroll
       for (int q = 0; q < 3; q++) gO[q] = gH[q] = gHs[q] = make_float2(0.f, 0.f);
@@ -1568,27 +1592,125 @@ __global__ void __launch_bounds__(WWX_BLOCK, 2) k_nb_ww_x2(DevPtrs P, int wpb) {
 #pragma unroll
         for (int u = 0; u < 4; u++) jg[u] = jn[u];
       }
-      // per atom of water i: O, H1, H2 (x, y, z each), reduced over the half-warp
-      float g[9];
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        g[q] = gO[q].x + gO[q].y;
-        g[3 + q] = gH[q].x + gHs[q].y;
-        g[6 + q] = gH[q].y + gHs[q].x;
-      }
-#pragma unroll
-      for (int q = 0; q < 9; q++) {
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) g[q] += __shfl_xor_sync(hmask, g[q], o);
-      }
-      if (hl == 0) {
-        const int oi = S.aoff + S.nsol + 3 * iw;
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-          atomic_add3(P.d, oi + a, (double)g[3 * a], (double)g[3 * a + 1], (double)g[3 * a + 2]);
-      }
+      ww_store_i(P, S.aoff + S.nsol + 3 * iw, hl, hmask, gO, gH, gHs);
     }
   }
+}
+
+// ------------------------------------------- water-water, small batches
+
+// The water-water kernels of batches whose staged blocks cannot fill the SMs
+// (Batch::ww_direct): a warp per water (FP64) or half a warp (packed FP32), its
+// neighbours' records read where they lie (L1 and L2 hold one system's), no
+// staging and no barrier before the pairs.  The list walk, the pair terms and,
+// for the packed form, each lane's entries and the order of its FP32 sums are
+// those of k_nb_ww and k_nb_ww_x2 on one chunk, so the packed forces are the
+// same bit for bit.  One 1,035-water window: FP64 14 to 7 us, packed 7.8 to 4;
+// the 480-water sphere 12 to 6.6.
+constexpr int WWD_WATERS = 8;               // waters per block, (system, first water) in P.wd_tiles
+
+template <bool HLJ, bool EONCE = false>
+__global__ void __launch_bounds__(32 * WWD_WATERS, 2) k_nb_ww_direct(DevPtrs P) {
+  __shared__ double ered[WWD_WATERS][2];
+  constexpr int W = WatRec<false>::words;
+  const int2 tile = P.wd_tiles[blockIdx.x];
+  const int s = tile.x;
+  const SysDev &S = P.sys[s];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int iw = tile.y + warp, gw = S.woff + iw;
+  double el = 0, vdw = 0;
+  if (iw < S.nwat) {
+    const uint16_t *nb = P.ww + (size_t)gw * P.ww_cap;
+    const int ke = P.ww_n[gw];
+    int k = (EONCE ? P.ww_mid[gw] : 0) + lane;
+    int jn = k < ke ? (int)nb[k] : 0;
+    const double2 *rec = reinterpret_cast<const double2 *>(P.wrec + (size_t)S.woff * W);
+    const double2 *rd = rec + (size_t)iw * W;
+    const double2 d0 = rd[0], d1 = rd[1], d2 = rd[2], d3 = rd[3], d4 = rd[4];
+    const double xi[9] = {d0.x, d0.y, d1.x, d1.y, d2.x, d2.y, d3.x, d3.y, d4.x};
+    const float qo = S.crg_ow, qh = S.crg_hw;
+    const double qoo = (double)(qo * qo), qoh = (double)(qo * qh), qhh = (double)(qh * qh);
+    const double ljd[6] = {S.A_OO, S.B_OO, S.A_OH, S.B_OH, S.A_HH, S.B_HH};
+    const bool box = S.pbc != 0;
+    const BoxD bx = box_of(P, s);
+    double fd[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++) fd[q] = 0.0;
+    for (; k < ke; k += 32) {
+      const double2 *rj = rec + (size_t)jn * W;
+      const double2 v0 = rj[0], v1 = rj[1], v2 = rj[2], v3 = rj[3], v4 = rj[4];
+      if (k + 32 < ke) jn = nb[k + 32];
+      double xj[9] = {v0.x, v0.y, v1.x, v1.y, v2.x, v2.y, v3.x, v3.y, v4.x};
+      if (box) {
+        const double3 t = image_shift(bx, xj[0] - xi[0], xj[1] - xi[1], xj[2] - xi[2]);
+#pragma unroll
+        for (int a = 0; a < 3; a++) { xj[3 * a] -= t.x; xj[3 * a + 1] -= t.y; xj[3 * a + 2] -= t.z; }
+      }
+      ww_pair_f64<HLJ>(xi, xj, qoo, qoh, qhh, ljd, fd, el, vdw);
+    }
+    if (!EONCE) {
+      double f = 0.0;
+#pragma unroll
+      for (int q = 0; q < 9; q++) {
+        const double t = warp_sum(fd[q]);
+        if (lane == q) f = t;
+      }
+      if (lane < 9 && ke > 0) atomicAdd(&P.d[S.aoff + S.nsol + 3 * iw + lane / 3].x + lane % 3, f);
+    }
+    el = warp_sum(el);
+    vdw = warp_sum(vdw);
+  }
+  if (lane == 0) { ered[warp][0] = el; ered[warp][1] = vdw; }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double e = 0.0;
+#pragma unroll
+    for (int w = 0; w < WWD_WATERS; w++) e += ered[w][threadIdx.x];
+    atomicAdd(&P.E[s * QB_NE + (threadIdx.x ? QB_E_WW_VDW : QB_E_WW_EL)], EONCE ? e : 0.5 * e);
+  }
+}
+
+template <bool BOX>
+__global__ void __launch_bounds__(16 * WWD_WATERS, 4) k_nb_ww_x2_direct(DevPtrs P) {
+  constexpr int W = WatRec<true>::words;
+  const int2 tile = P.wd_tiles[blockIdx.x];
+  const int s = tile.x;
+  const SysDev &S = P.sys[s];
+  const int hl = threadIdx.x & 15;
+  const unsigned hmask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
+  const int iw = tile.y + (threadIdx.x >> 4), gw = S.woff + iw;
+  if (iw >= S.nwat) return;
+  const int ke = P.ww_n[gw];
+  if (ke == 0) return;
+  const uint16_t *nb = P.ww + (size_t)gw * P.ww_cap;
+  const float4 *rec = P.wrec32 + (size_t)S.woff * W;
+  int jn = hl < ke ? (int)nb[hl] : 0;
+  const float qo = S.crg_ow, qh = S.crg_hw;
+  const float qoo = qo * qo;
+  const float2 qoh2 = dup2(qo * qh), qhh2 = dup2(qh * qh);
+  const float A = (float)S.A_OO, B = (float)S.B_OO;
+  float Lh[3], Ll[3], iL[3];
+  if (BOX) {
+    const BoxD bx = box_of(P, s);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      Lh[q] = (float)bx.L[q];
+      Ll[q] = (float)(bx.L[q] - (double)Lh[q]);
+      iL[q] = (float)bx.iL[q];
+    }
+  }
+  WwI2 I;
+  ww_load_i(rec + (size_t)iw * W, I);
+  float2 gO[3], gH[3], gHs[3];
+#pragma unroll
+  for (int q = 0; q < 3; q++) gO[q] = gH[q] = gHs[q] = make_float2(0.f, 0.f);
+  for (int k = hl; k < ke; k += 16) {
+    const float4 *rj = rec + (size_t)jn * W;
+    const float4 j0 = rj[0], j1 = rj[1], j2 = rj[2];
+    if (k + 16 < ke) jn = nb[k + 16];
+    ww_force_x2<BOX>(I, j0, j1, j2, qoh2, qhh2, qoo, A, B, gO, gH, gHs, Lh, Ll, iL);
+  }
+  ww_store_i(P, S.aoff + S.nsol + 3 * iw, hl, hmask, gO, gH, gHs);
 }
 
 // nonbond_pp (md.f90:10387) over the atoms' rows (k_list_pp): a warp per atom,
