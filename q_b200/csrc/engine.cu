@@ -279,9 +279,9 @@ struct Batch {
   }
 
   // Side streams of the force fork: after the water pass the force kernels of
-  // a step (all adding with atomics) run on four streams and join before the
+  // a step (all adding with atomics) run on five streams and join before the
   // leap-frog.  Profiling keeps them on the main stream, one at a time.
-  static constexpr int NSIDE = 3;
+  static constexpr int NSIDE = 4;
   cudaStream_t side[NSIDE] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[NSIDE] = {};
 
@@ -380,8 +380,8 @@ struct Batch {
       }
     }
     cudaStream_t s1 = forking() ? side[0] : stream, s2 = forking() ? side[1] : stream;
-    fork_streams(3);
-    cudaStream_t s3 = forking() ? side[2] : stream;
+    fork_streams(4);
+    cudaStream_t s3 = forking() ? side[2] : stream, s4 = forking() ? side[3] : stream;
     // solute terms in one launch (nonbond_pp, nonbond_qp, bonded, nonbond_qq,
     // Q bonded, restraints)
     {
@@ -411,8 +411,8 @@ struct Batch {
     if (p.n_pw_groups > 0)
       launch("nb_pw", [&] {
         const dim3 g(p.n_pw_groups, cdiv(p.pwg_cap, PW_BLOCK));
-        if (fast_ww) k_nb_pw<true><<<g, PW_BLOCK, 0, s1>>>(p);
-        else k_nb_pw<false><<<g, PW_BLOCK, 0, s1>>>(p);
+        if (fast_ww) k_nb_pw<true><<<g, PW_BLOCK, 0, s4>>>(p);
+        else k_nb_pw<false><<<g, PW_BLOCK, 0, s4>>>(p);
       });
     if (max_nwat > 0) {
       const int wpb = ww_wpb;
@@ -464,11 +464,11 @@ struct Batch {
       });
     }
     if (max_nsol > 0)
-      launch("atom_terms", [&] { k_atom_terms<<<dim3(cdiv(max_nsol, 128), nsys), 128, 0, s1>>>(p); });
+      launch("atom_terms", [&] { k_atom_terms<<<dim3(cdiv(max_nsol, 128), nsys), 128, 0, s4>>>(p); });
     if (any_wpol) {
       launch("watpol", [&] { k_watpol<<<dim3(std::max(max_nshell, 1), nsys), WPOL_BLOCK, watpol_smem, s3>>>(p); });
     }
-    join_streams(3);
+    join_streams(4);
     check_launch("force kernels");
   }
 
