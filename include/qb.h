@@ -259,8 +259,7 @@ void qb_batch_destroy(qb_batch *b);
 
 #define QB_STATIC_WW_MAX_WATERS 4096
 #define QB_STATIC_WW_MAX_NEIGHBOURS 192
-#define QB_STATIC_WW_SCRATCH_BYTES \
-  ((size_t)(QB_STATIC_WW_MAX_WATERS * QB_STATIC_WW_MAX_NEIGHBOURS + QB_STATIC_WW_MAX_WATERS) * 4)
+#define QB_STATIC_WW_SCRATCH_BYTES ((size_t)(QB_STATIC_WW_MAX_WATERS * 5))
 
 /* SPC/TIP3P water-water electrostatic and Lennard-Jones energy and gradient of
  * one water sphere, computed on buffers the caller owns, with no device memory
@@ -290,9 +289,9 @@ void qb_batch_destroy(qb_batch *b);
  * stream: cudaStream_t (NULL = default stream); the work is queued on it and
  *         the call returns without waiting.
  *
- * Its scratch (the neighbour list) is a fixed array in the library's device
+ * Its scratch (energy sums) is a fixed array in the library's device
  * memory: every GPU that loads the library holds QB_STATIC_WW_SCRATCH_BYTES
- * (about 3 MB) until the process exits.  Systems above
+ * (20 kB) until the process exits.  Systems above
  * QB_STATIC_WW_MAX_WATERS waters are rejected with QB_ERR_ARG.  All calls on a
  * device share that array and it keeps the last call's contents (the call
  * rewrites everything it reads), so calls that overlap on the GPU -- on two
