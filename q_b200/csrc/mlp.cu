@@ -1,18 +1,29 @@
 // mlp.cu -- the lambda-placement network: a 12 -> 64 -> 64 -> 11 perceptron
 // with SiLU, run and trained on the 5th-generation tensor cores (tcgen05).
 //
-// One CTA of 128 threads works on tiles of 128 samples; thread t owns sample
-// row t, which is TMEM lane t of every accumulator.  Each GEMM is one M = 128
+// One CTA of 512 threads works on tiles of 128 samples: warp w takes the
+// sample rows of TMEM lanes 32 (w % 4) .. + 31, and of every accumulator of 64
+// columns the block of 16 that starts at 16 (w / 4).  Each GEMM is one M = 128
 // tcgen05.mma.kind::f16 chain (BF16 operands in shared memory, FP32
 // accumulators in TMEM), issued by thread 0 and completed through an
-// mbarrier.  Operands are K-major in the canonical no-swizzle layout: 8-row x
-// 16-byte core matrices, the two 8-element halves of a 16-wide K slice 128
-// bytes apart (leading byte offset), 8-row groups K*2*8 bytes apart (stride
-// byte offset).  The backward GEMMs that contract over the batch take
-// transposed copies written by the threads, so every operand has that one
-// layout.  Training (Adam) runs all its iterations inside one launch; the
-// FP32 master weights and moments live in global memory, their BF16 copies
-// (and the transposes the backward pass needs) in shared memory.
+// mbarrier.  Operands lie in the canonical no-swizzle layout: 8-row x 16-byte
+// core matrices, the core matrices of one row group 128 bytes apart, row
+// groups 16 bytes x columns apart.  A tile read along its columns (the
+// forward GEMMs, and the data gradients' dz) is a K-major operand; read along
+// its rows (the activations and dz of the weight gradients, which contract
+// over the samples, and W in the data gradients) the same bytes are an
+// MN-major operand, so nothing is transposed or copied.  With M = 128 such an
+// A operand of 16 or 64 columns runs on into the bytes behind each row group:
+// rows of the product that no thread reads.
+//
+// Training (Adam) runs all its iterations inside one launch.  The FP32 master
+// weights and both moments live in shared memory beside the BF16 tiles (they
+// were in global memory, each thread walking its own row: 140 parameters x 6
+// uncoalesced accesses a step), in column order so that the 64 threads of a
+// column hit 64 banks in turn.  A step on 200 samples took 155 us with one
+// warp per row block, scalar BF16 stores, transposed copies and a 5-shuffle
+// sum per column; it takes 36, most of it the six dependent GEMM rounds of
+// each tile (issue, commit, wait) and the two expf and quotients per element.
 //
 // Every wait on the tensor cores is bounded: on time-out the kernel records
 // QB_ERR_TIMEOUT, stops issuing work, frees its TMEM and returns.
@@ -35,30 +46,37 @@ namespace mlp {
 constexpr int IN = QB_MLP_IN, HID = QB_MLP_HIDDEN, OUT = QB_MLP_OUT;
 constexpr int KIN = 16, NOUT = 16;   // padded input features / outputs
 constexpr int ROWS = 128;            // samples per tile = TMEM lanes
-constexpr int THREADS = 128;
+constexpr int THREADS = 512;
 
 // parameter vector offsets (floats)
 constexpr int OW1 = 0, OB1 = OW1 + HID * IN, OW2 = OB1 + HID, OB2 = OW2 + HID * HID, OW3 = OB2 + HID,
               OB3 = OW3 + OUT * HID, NPARAM = OB3 + OUT;
 static_assert(NPARAM == QB_MLP_NPARAM, "parameter layout");
 
-// shared-memory tiles (bytes): K-major canonical layout of R rows x K columns
+// shared-memory tiles (bytes): canonical layout of R rows x K columns
 constexpr int tile_bytes(int R, int K) { return R * K * 2; }
-constexpr int S_X = 0;                                   // A  128 x 16  (x)
-constexpr int S_W1 = S_X + tile_bytes(ROWS, KIN);        // B   64 x 16  (W1)
-constexpr int S_H1 = S_W1 + tile_bytes(HID, KIN);        // A  128 x 64  (h1)
-constexpr int S_W2 = S_H1 + tile_bytes(ROWS, HID);       // B   64 x 64  (W2)
-constexpr int S_H2 = S_W2 + tile_bytes(HID, HID);        // A  128 x 64  (h2)
-constexpr int S_W3 = S_H2 + tile_bytes(ROWS, HID);       // B   16 x 64  (W3, rows 11..15 zero)
-constexpr int S_D3 = S_W3 + tile_bytes(NOUT, HID);       // A  128 x 16  (dz3, cols 11..15 zero)
-constexpr int S_W3T = S_D3 + tile_bytes(ROWS, NOUT);     // B   64 x 16  (W3^T, cols 11..15 zero)
-constexpr int S_D2 = S_W3T + tile_bytes(HID, NOUT);      // A  128 x 64  (dz2)
-constexpr int S_W2T = S_D2 + tile_bytes(ROWS, HID);      // B   64 x 64  (W2^T)
-constexpr int S_AT = S_W2T + tile_bytes(HID, HID);       // A  128 x 128 (dz^T: features x samples)
-constexpr int S_BT = S_AT + tile_bytes(ROWS, ROWS);      // B   64 x 128 (activations^T)
-constexpr int S_END = S_BT + tile_bytes(HID, ROWS);
-constexpr int S_MISC = S_END;                            // mbarrier, TMEM address, bias gradients, loss
-constexpr int SMEM_BYTES = S_MISC + 1024;
+constexpr int S_X = 0;                                   // 128 x 16  x
+constexpr int S_W1 = S_X + tile_bytes(ROWS, KIN);        //  64 x 16  W1
+constexpr int S_H1 = S_W1 + tile_bytes(HID, KIN);        // 128 x 64  h1
+constexpr int S_W2 = S_H1 + tile_bytes(ROWS, HID);       //  64 x 64  W2
+constexpr int S_H2 = S_W2 + tile_bytes(HID, HID);        // 128 x 64  h2
+constexpr int S_W3 = S_H2 + tile_bytes(ROWS, HID);       //  16 x 64  W3, rows 11..15 zero
+constexpr int S_D3 = S_W3 + tile_bytes(NOUT, HID);       // 128 x 16  dz3, columns 11..15 zero
+constexpr int S_D2 = S_D3 + tile_bytes(ROWS, NOUT);      // 128 x 64  dz2
+constexpr int S_D1 = S_D2 + tile_bytes(ROWS, HID);       // 128 x 64  dz1
+constexpr int S_END = S_D1 + tile_bytes(ROWS, HID);
+// FP32 parameters, then (training) first and second moments, each in the
+// order of pidx; the MN-major reads past S_D1 end here
+constexpr int S_PAR = S_END;
+constexpr int PSIZE = (NPARAM + 3) / 4 * 4;
+constexpr int S_GB = S_PAR + 3 * PSIZE * 4;              // bias gradients: b1, b2, b3
+constexpr int S_GBW = S_GB + (2 * HID + NOUT) * 4;       // column sums of each 32 rows
+constexpr int S_MISC = S_GBW + 4 * HID * 4;              // mbarrier, TMEM address, loss
+constexpr int SMEM_BYTES = S_MISC + 64;
+static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+// position of parameter p (the header's row-major order) in shared memory:
+// the weight matrices by columns
+__host__ __device__ constexpr int pidx_w(int off, int rows, int j, int i) { return off + i * rows + j; }
 
 // TMEM columns of the accumulators (128 lanes x 512 columns allocated)
 constexpr int T_Z1 = 0, T_Z2 = 64, T_Z3 = 128, T_DH2 = 144, T_DW3 = 208, T_DH1 = 272, T_DW2 = 336, T_DW1 = 400;
@@ -74,20 +92,29 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// shared-memory matrix descriptor of the 16-wide K slice s of a tile
-__device__ __forceinline__ uint64_t sdesc(uint32_t tile_addr, int K, int s) {
-  const uint32_t a = tile_addr + (uint32_t)s * 256u;
+// shared-memory matrix descriptors of the 16-wide K slice s of a tile with C
+// columns: K-major (K along the columns; leading offset between the K halves,
+// stride between 8-row groups) and MN-major (K along the rows; leading offset
+// between 8-row groups, stride between the 8-column core matrices)
+__device__ __forceinline__ uint64_t desc(uint32_t a, uint32_t lead, uint32_t stride) {
   uint64_t d = 0;
   d |= (uint64_t)((a >> 4) & 0x3FFFu);
-  d |= (uint64_t)((128u >> 4) & 0x3FFFu) << 16;                  // leading byte offset: K halves
-  d |= (uint64_t)(((uint32_t)K * 16u >> 4) & 0x3FFFu) << 32;     // stride byte offset: 8-row groups
+  d |= (uint64_t)((lead >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)((stride >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1 << 46;                                         // descriptor version (sm_100)
   return d;                                                       // base offset 0, no swizzle
 }
+__device__ __forceinline__ uint64_t kdesc(uint32_t tile, int C, int s) {
+  return desc(tile + (uint32_t)s * 256u, 128u, (uint32_t)C * 16u);
+}
+__device__ __forceinline__ uint64_t mdesc(uint32_t tile, int C, int s) {
+  return desc(tile + (uint32_t)s * (uint32_t)C * 32u, (uint32_t)C * 16u, 128u);
+}
 
-// instruction descriptor: D F32, A and B BF16, both K-major, M = 128, N
-__host__ __device__ constexpr uint32_t idesc(int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
+// instruction descriptor: D F32, A and B BF16, M = 128, N; am, bm: MN-major
+__host__ __device__ constexpr uint32_t idesc(int N, int am, int bm) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)am << 15) | ((uint32_t)bm << 16) |
+         ((uint32_t)(N >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
@@ -99,11 +126,15 @@ __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t a, uint64_t b, uin
       : "r"(tmem_d), "l"(a), "l"(b), "r"(id), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
-// D[128 x N] (+)= A[128 x K] * B[N x K]^T over K/16 MMAs
-__device__ __forceinline__ void gemm(uint32_t tmem_d, uint32_t a_tile, int Ka, uint32_t b_tile, int N, bool accumulate) {
-  const uint32_t id = idesc(N);
-  for (int s = 0; s < Ka / 16; s++)
-    mma(tmem_d, sdesc(a_tile, Ka, s), sdesc(b_tile, Ka, s), id, (accumulate || s > 0) ? 1u : 0u);
+// D[128 x N] (+)= A B^T over K/16 MMAs; AM, BM: the operand's tile is read
+// along its rows (MN-major); ca, cb: the tiles' columns
+template <bool AM, bool BM>
+__device__ __forceinline__ void gemm(uint32_t tmem_d, uint32_t a, int ca, uint32_t b, int cb, int N, int K,
+                                     bool accumulate) {
+  const uint32_t id = idesc(N, AM, BM);
+  for (int s = 0; s < K / 16; s++)
+    mma(tmem_d, AM ? mdesc(a, ca, s) : kdesc(a, ca, s), BM ? mdesc(b, cb, s) : kdesc(b, cb, s), id,
+        (accumulate || s > 0) ? 1u : 0u);
 }
 
 __device__ __forceinline__ void commit(uint32_t bar) {
@@ -142,18 +173,46 @@ __device__ __forceinline__ void tld16(uint32_t taddr, float *v) {
   for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[k]);
 }
 
-__device__ __forceinline__ void st_bf16(uint8_t *sm, int tile, int r, int k, int K, float v) {
-  *reinterpret_cast<__nv_bfloat16 *>(sm + tile + kmaj(r, k, K)) = __float2bfloat16_rn(v);
-}
-__device__ __forceinline__ float ld_bf16(const uint8_t *sm, int tile, int r, int k, int K) {
-  return __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(sm + tile + kmaj(r, k, K)));
+// 8 consecutive columns k..k+7 of row r, rounded to BF16: one 16-byte store
+__device__ __forceinline__ void st8(uint8_t *sm, int tile, int r, int k, int K, const float *v) {
+  __nv_bfloat162 p[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) p[c] = __floats2bfloat162_rn(v[2 * c], v[2 * c + 1]);
+  *reinterpret_cast<uint4 *>(sm + tile + kmaj(r, k, K)) = *reinterpret_cast<const uint4 *>(p);
 }
 
-// add v, summed over the warp's 32 rows, to *acc (one shared atomic per warp)
-__device__ __forceinline__ void warp_col_add(float *acc, float v) {
+// Sums of 16 columns over the warp's 32 rows by halving: every step a lane
+// hands half of its columns to its partner (lanes 16, 8, 4, 2 apart, then 1:
+// the association of a butterfly per column, in 16 instead of 80 shuffles).
+// The sums go to out[0..16).
+__device__ __forceinline__ void warp_col_sums(float *v, float *out) {
+  const int lane = threadIdx.x & 31;
+  int base = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(acc, v);
+  for (int n = 8, m = 16; n > 0; n >>= 1, m >>= 1) {
+    const bool up = lane & m;
+#pragma unroll
+    for (int k = 0; k < n; k++) {
+      const float give = up ? v[k] : v[k + n];
+      const float keep = up ? v[k + n] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+    }
+    if (up) base += n;
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  out[base] = v[0];
+}
+
+// A bias gradient: the four row blocks' sums of one column added in the order
+// in which the shared-memory atomics of this kernel's first form arrived (the
+// whole blocks, the first of them last, then the part-filled one), so that a
+// training gives the same bits.
+__device__ __forceinline__ float add_blocks(float acc, const float *sums, int rows) {
+  const int nf = rows >= ROWS ? 4 : rows / 32;
+  for (int w = 1; w < nf; w++) acc += sums[w * HID];
+  if (nf > 0) acc += sums[0];
+  if (nf < 4) acc += sums[nf * HID];
+  return acc;
 }
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
@@ -174,30 +233,9 @@ struct Args {
   float *y;            // [n x OUT] outputs (forward)
   float *grad;         // [NPARAM] (mode 1)
   float *loss;         // [1] (mode 1) or [iters] (mode 2)
-  float *adam_m, *adam_v;   // [NPARAM] (mode 2)
   int *status;
   long long wait_limit;     // try_wait polls of each tensor-core wait before it gives up
 };
-
-// BF16 copies of the weights: W1, W2, W3 as B operands, W2^T and W3^T for
-// the backward data GEMMs.  Thread j < 64 writes row j of W1 and W2 (and
-// column j of their transposes); thread j < 11 writes row j of W3.
-__device__ void stage_weights(uint8_t *sm, const float *P, int j) {
-  if (j < HID) {
-    for (int i = 0; i < KIN; i++) st_bf16(sm, S_W1, j, i, KIN, i < IN ? P[OW1 + j * IN + i] : 0.0f);
-    for (int i = 0; i < HID; i++) {
-      const float w = P[OW2 + j * HID + i];     // W2[out j][in i]
-      st_bf16(sm, S_W2, j, i, HID, w);
-      st_bf16(sm, S_W2T, i, j, HID, w);         // W2^T: row = in i, K = out j
-    }
-  }
-  if (j < NOUT)
-    for (int i = 0; i < HID; i++) {
-      const float w = j < OUT ? P[OW3 + j * HID + i] : 0.0f;
-      st_bf16(sm, S_W3, j, i, HID, w);
-      st_bf16(sm, S_W3T, i, j, NOUT, w);        // W3^T: row = hidden i, K = out j
-    }
-}
 
 __global__ void __launch_bounds__(THREADS, 1) k_mlp(Args A) {
   extern __shared__ __align__(1024) uint8_t sm[];
@@ -205,14 +243,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp(Args A) {
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S_MISC);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + S_MISC + 8);
   int *fail = reinterpret_cast<int *>(sm + S_MISC + 12);
-  float *gb1 = reinterpret_cast<float *>(sm + S_MISC + 16);   // bias gradients
-  float *gb2 = gb1 + HID;
-  float *gb3 = gb2 + HID;
-  float *red = gb3 + NOUT;                                     // [4] per-warp loss
+  float *red = reinterpret_cast<float *>(sm + S_MISC + 16);    // [4] per-warp loss
+  float *P = reinterpret_cast<float *>(sm + S_PAR), *M = P + PSIZE, *V = M + PSIZE;
+  float *gb1 = reinterpret_cast<float *>(sm + S_GB), *gb2 = gb1 + HID, *gb3 = gb2 + HID;
+  float *gbw = reinterpret_cast<float *>(sm + S_GBW);          // [4][HID]
   const uint32_t smb = smem_u32(sm);
   const uint32_t barp = smem_u32(bar);
 
-  for (int k = tid * 16; k < S_END; k += THREADS * 16) *reinterpret_cast<uint4 *>(sm + k) = make_uint4(0, 0, 0, 0);
+  for (int k = tid * 16; k < S_MISC; k += THREADS * 16) *reinterpret_cast<uint4 *>(sm + k) = make_uint4(0, 0, 0, 0);
   if (tid == 0) {
     *fail = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barp) : "memory");
@@ -228,7 +266,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp(Args A) {
   __syncthreads();
   tc_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);   // this warp's TMEM lanes
+  const int quad = warp & 3, cb = (warp >> 2) * 16;                  // this warp's rows and columns
+  const int rt = quad * 32 + (tid & 31);                             // this thread's row of the tile
+  const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);   // this warp's TMEM lanes
   uint32_t phase = 0;
   uint32_t late_phase = 2;   // the phase a wait gave up on (2: none)
 
@@ -251,8 +291,35 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp(Args A) {
     return ok;
   };
 
-  float *P = A.params;
-  stage_weights(sm, P, tid);
+  // the parameters into shared memory, the weight matrices by columns
+  for (int p = tid; p < NPARAM; p += THREADS) {
+    int q = p;
+    if (p < OB1) q = pidx_w(OW1, HID, p / IN, p % IN);
+    else if (p >= OW2 && p < OB2) q = pidx_w(OW2, HID, (p - OW2) / HID, (p - OW2) % HID);
+    else if (p >= OW3 && p < OB3) q = pidx_w(OW3, OUT, (p - OW3) / HID, (p - OW3) % HID);
+    P[q] = A.params[p];
+  }
+  __syncthreads();
+  const int j = rt;                                      // weight row in the gradient and Adam steps
+  // the BF16 tiles of the weights: thread j of the first warps writes row j of W1, W2 and W3
+  if (cb == 0) {
+    float w[8];
+    if (j < HID) {
+      for (int c = 0; c < KIN; c += 8) {
+        for (int k = 0; k < 8; k++) w[k] = c + k < IN ? P[pidx_w(OW1, HID, j, c + k)] : 0.f;
+        st8(sm, S_W1, j, c, KIN, w);
+      }
+      for (int c = 0; c < HID; c += 8) {
+        for (int k = 0; k < 8; k++) w[k] = P[pidx_w(OW2, HID, j, c + k)];
+        st8(sm, S_W2, j, c, HID, w);
+      }
+    }
+    if (j < OUT)
+      for (int c = 0; c < HID; c += 8) {
+        for (int k = 0; k < 8; k++) w[k] = P[pidx_w(OW3, OUT, j, c + k)];
+        st8(sm, S_W3, j, c, HID, w);
+      }
+  }
   const int ntile = (A.n + ROWS - 1) / ROWS;
   const int iters = A.mode == 2 ? A.iters : 1;
   const float gscale = 2.0f / ((float)A.n * (float)OUT);   // d(mean squared error)/dy
@@ -262,142 +329,185 @@ __global__ void __launch_bounds__(THREADS, 1) k_mlp(Args A) {
     if (tid < HID) { gb1[tid] = 0.f; gb2[tid] = 0.f; }
     if (tid < NOUT) gb3[tid] = 0.f;
     float lsum = 0.f;
-    for (int tile = 0; tile < ntile && ok; tile++) {
-      const int row = tile * ROWS + tid;
+    // forward alone: the blocks of the launch share the tiles
+    for (int tile = A.mode == 0 ? blockIdx.x : 0; tile < ntile && ok; tile += A.mode == 0 ? gridDim.x : 1) {
+      const int rows = A.n - tile * ROWS;     // of this tile, or more
+      const int row = tile * ROWS + rt;
       const bool valid = row < A.n;
       // ---- forward
-      for (int i = 0; i < KIN; i++) st_bf16(sm, S_X, tid, i, KIN, (valid && i < IN) ? A.x[(size_t)row * IN + i] : 0.f);
-      ok = run([&] { gemm(tmem + T_Z1, smb + S_X, KIN, smb + S_W1, HID, false); });
+      if (cb < 32) {                            // 8 features each
+        float x[8];
+        const int i0 = cb / 2;
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = (valid && i0 + i < IN) ? A.x[(size_t)row * IN + i0 + i] : 0.f;
+        st8(sm, S_X, rt, i0, KIN, x);
+      }
+      ok = run([&] { gemm<false, false>(tmem + T_Z1, smb + S_X, KIN, smb + S_W1, KIN, HID, KIN, false); });
       if (!ok) break;
-      for (int c = 0; c < HID; c += 16) {
+      {
         float z[16];
-        tld16(lane_base + T_Z1 + c, z);
-        for (int k = 0; k < 16; k++) st_bf16(sm, S_H1, tid, c + k, HID, silu(z[k] + P[OB1 + c + k]));
+        tld16(lane_base + T_Z1 + cb, z);
+#pragma unroll
+        for (int k = 0; k < 16; k++) z[k] = silu(z[k] + P[OB1 + cb + k]);
+        st8(sm, S_H1, rt, cb, HID, z);
+        st8(sm, S_H1, rt, cb + 8, HID, z + 8);
       }
-      ok = run([&] { gemm(tmem + T_Z2, smb + S_H1, HID, smb + S_W2, HID, false); });
+      ok = run([&] { gemm<false, false>(tmem + T_Z2, smb + S_H1, HID, smb + S_W2, HID, HID, HID, false); });
       if (!ok) break;
-      for (int c = 0; c < HID; c += 16) {
+      {
         float z[16];
-        tld16(lane_base + T_Z2 + c, z);
-        for (int k = 0; k < 16; k++) st_bf16(sm, S_H2, tid, c + k, HID, silu(z[k] + P[OB2 + c + k]));
+        tld16(lane_base + T_Z2 + cb, z);
+#pragma unroll
+        for (int k = 0; k < 16; k++) z[k] = silu(z[k] + P[OB2 + cb + k]);
+        st8(sm, S_H2, rt, cb, HID, z);
+        st8(sm, S_H2, rt, cb + 8, HID, z + 8);
       }
-      ok = run([&] { gemm(tmem + T_Z3, smb + S_H2, HID, smb + S_W3, NOUT, false); });
+      ok = run([&] { gemm<false, false>(tmem + T_Z3, smb + S_H2, HID, smb + S_W3, HID, NOUT, HID, false); });
       if (!ok) break;
-      float y[16];
-      tld16(lane_base + T_Z3, y);
-      for (int k = 0; k < OUT; k++) y[k] += P[OB3 + k];
-      if (A.mode == 0) {
-        if (valid)
-          for (int k = 0; k < OUT; k++) A.y[(size_t)row * OUT + k] = y[k];
-        continue;
-      }
-      // ---- output gradient (mean squared error)
-      for (int k = 0; k < NOUT; k++) {
-        float d = 0.f;
-        if (valid && k < OUT) {
-          const float e = y[k] - A.t[(size_t)row * OUT + k];
-          lsum += e * e;
-          d = gscale * e;
+      if (cb == 0) {                            // the outputs: one warp per row block
+        float y[16];
+        tld16(lane_base + T_Z3, y);
+#pragma unroll
+        for (int k = 0; k < OUT; k++) y[k] += P[OB3 + k];
+        if (A.mode == 0) {
+          if (valid)
+#pragma unroll
+            for (int k = 0; k < OUT; k++) A.y[(size_t)row * OUT + k] = y[k];
+        } else {
+          // ---- output gradient (mean squared error)
+#pragma unroll
+          for (int k = 0; k < NOUT; k++) {
+            float d = 0.f;
+            if (valid && k < OUT) {
+              const float e = y[k] - A.t[(size_t)row * OUT + k];
+              lsum += e * e;
+              d = gscale * e;
+            }
+            y[k] = d;
+          }
+          st8(sm, S_D3, rt, 0, NOUT, y);
+          st8(sm, S_D3, rt, 8, NOUT, y + 8);
+          warp_col_sums(y, gbw + quad * HID);
         }
-        st_bf16(sm, S_D3, tid, k, NOUT, d);
-        st_bf16(sm, S_AT, k, tid, ROWS, d);             // dz3^T: row = output k, K = sample
-        warp_col_add(&gb3[k], d);
       }
-      for (int h = 0; h < HID; h++) st_bf16(sm, S_BT, h, tid, ROWS, ld_bf16(sm, S_H2, tid, h, HID));
+      if (A.mode == 0) continue;
       // dh2 = dz3 W3 ; dW3 += dz3^T h2
       ok = run([&] {
-        gemm(tmem + T_DH2, smb + S_D3, NOUT, smb + S_W3T, HID, false);
-        gemm(tmem + T_DW3, smb + S_AT, ROWS, smb + S_BT, HID, tile > 0);
+        gemm<false, true>(tmem + T_DH2, smb + S_D3, NOUT, smb + S_W3, HID, HID, NOUT, false);
+        gemm<true, true>(tmem + T_DW3, smb + S_D3, NOUT, smb + S_H2, HID, HID, ROWS, tile > 0);
       });
       if (!ok) break;
-      for (int c = 0; c < HID; c += 16) {
-        float g[16], z[16];
-        tld16(lane_base + T_DH2 + c, g);
-        tld16(lane_base + T_Z2 + c, z);
-        for (int k = 0; k < 16; k++) {
-          const float d = valid ? g[k] * dsilu(z[k] + P[OB2 + c + k]) : 0.f;
-          st_bf16(sm, S_D2, tid, c + k, HID, d);
-          st_bf16(sm, S_AT, c + k, tid, ROWS, d);       // dz2^T
-          warp_col_add(&gb2[c + k], d);
-        }
-      }
-      for (int h = 0; h < HID; h++) st_bf16(sm, S_BT, h, tid, ROWS, ld_bf16(sm, S_H1, tid, h, HID));
+      if (tid < NOUT) gb3[tid] = add_blocks(gb3[tid], gbw + tid, rows);
+      float g[16], d[16];
+      tld16(lane_base + T_DH2 + cb, g);
+      tld16(lane_base + T_Z2 + cb, d);
+#pragma unroll
+      for (int k = 0; k < 16; k++) d[k] = valid ? g[k] * dsilu(d[k] + P[OB2 + cb + k]) : 0.f;
+      st8(sm, S_D2, rt, cb, HID, d);
+      st8(sm, S_D2, rt, cb + 8, HID, d + 8);
+      __syncthreads();                                  // gbw's last readers
+      warp_col_sums(d, gbw + quad * HID + cb);
       // dh1 = dz2 W2 ; dW2 += dz2^T h1
       ok = run([&] {
-        gemm(tmem + T_DH1, smb + S_D2, HID, smb + S_W2T, HID, false);
-        gemm(tmem + T_DW2, smb + S_AT, ROWS, smb + S_BT, HID, tile > 0);
+        gemm<false, true>(tmem + T_DH1, smb + S_D2, HID, smb + S_W2, HID, HID, HID, false);
+        gemm<true, true>(tmem + T_DW2, smb + S_D2, HID, smb + S_H1, HID, HID, ROWS, tile > 0);
       });
       if (!ok) break;
-      for (int c = 0; c < HID; c += 16) {
-        float g[16], z[16];
-        tld16(lane_base + T_DH1 + c, g);
-        tld16(lane_base + T_Z1 + c, z);
-        for (int k = 0; k < 16; k++) {
-          const float d = valid ? g[k] * dsilu(z[k] + P[OB1 + c + k]) : 0.f;
-          st_bf16(sm, S_AT, c + k, tid, ROWS, d);       // dz1^T
-          warp_col_add(&gb1[c + k], d);
-        }
-      }
-      for (int i = 0; i < KIN; i++) st_bf16(sm, S_BT, i, tid, ROWS, ld_bf16(sm, S_X, tid, i, KIN));
+      if (tid < HID) gb2[tid] = add_blocks(gb2[tid], gbw + tid, rows);
+      tld16(lane_base + T_DH1 + cb, g);
+      tld16(lane_base + T_Z1 + cb, d);
+#pragma unroll
+      for (int k = 0; k < 16; k++) d[k] = valid ? g[k] * dsilu(d[k] + P[OB1 + cb + k]) : 0.f;
+      st8(sm, S_D1, rt, cb, HID, d);
+      st8(sm, S_D1, rt, cb + 8, HID, d + 8);
+      __syncthreads();
+      warp_col_sums(d, gbw + quad * HID + cb);
       // dW1 += dz1^T x
-      ok = run([&] { gemm(tmem + T_DW1, smb + S_AT, ROWS, smb + S_BT, KIN, tile > 0); });
+      ok = run([&] { gemm<true, true>(tmem + T_DW1, smb + S_D1, HID, smb + S_X, KIN, KIN, ROWS, tile > 0); });
       if (!ok) break;
+      if (tid < HID) gb1[tid] = add_blocks(gb1[tid], gbw + tid, rows);
+      __syncthreads();
     }
     if (!ok || A.mode == 0) break;
     // ---- loss of this pass
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if ((tid & 31) == 0) red[warp] = lsum;
+    if ((tid & 31) == 0 && cb == 0) red[quad] = lsum;
     __syncthreads();
     if (tid == 0) {
       const float L = (red[0] + red[1] + red[2] + red[3]) / ((float)A.n * (float)OUT);
       A.loss[A.mode == 2 ? it : 0] = L;
     }
-    // ---- weight gradients from TMEM: thread j holds row j of dW1, dW2 (j < 64), dW3 (j < 11)
-    float g1[16], g2[HID], g3[HID];
-    tld16(lane_base + T_DW1, g1);
-    for (int c = 0; c < HID; c += 16) tld16(lane_base + T_DW2 + c, g2 + c);
-    for (int c = 0; c < HID; c += 16) tld16(lane_base + T_DW3 + c, g3 + c);
-    const int j = tid;
+    // ---- weight gradients from TMEM: row j of dW1, dW2 (j < 64), dW3 (j < 11) on lane j
     if (A.mode == 1) {
-      if (j < HID) {
-        for (int i = 0; i < IN; i++) A.grad[OW1 + j * IN + i] = g1[i];
-        for (int i = 0; i < HID; i++) A.grad[OW2 + j * HID + i] = g2[i];
+      float g[16];
+      tld16(lane_base + T_DW1, g);
+      if (cb == 0 && j < HID)
+        for (int i = 0; i < IN; i++) A.grad[OW1 + j * IN + i] = g[i];
+      tld16(lane_base + T_DW2 + cb, g);
+      if (j < HID)
+        for (int i = 0; i < 16; i++) A.grad[OW2 + j * HID + cb + i] = g[i];
+      tld16(lane_base + T_DW3 + cb, g);
+      if (j < OUT)
+        for (int i = 0; i < 16; i++) A.grad[OW3 + j * HID + cb + i] = g[i];
+      if (cb == 0 && j < HID) {
         A.grad[OB1 + j] = gb1[j];
         A.grad[OB2 + j] = gb2[j];
       }
-      if (j < OUT) {
-        for (int i = 0; i < HID; i++) A.grad[OW3 + j * HID + i] = g3[i];
-        A.grad[OB3 + j] = gb3[j];
-      }
+      if (cb == 0 && j < OUT) A.grad[OB3 + j] = gb3[j];
       break;
     }
-    // ---- Adam step on the FP32 master weights, then fresh BF16 copies
+    // ---- Adam step on the FP32 master weights and their fresh BF16 tiles
     const float t1 = (float)(it + 1);
     const float c1 = 1.0f / (1.0f - powf(A.beta1, t1)), c2 = 1.0f / (1.0f - powf(A.beta2, t1));
     // decoupled weight decay on the weight matrices, not on the biases
     auto adam = [&](int p, float g, float wd) {
-      const float m = A.beta1 * A.adam_m[p] + (1.0f - A.beta1) * g;
-      const float v = A.beta2 * A.adam_v[p] + (1.0f - A.beta2) * g * g;
-      A.adam_m[p] = m;
-      A.adam_v[p] = v;
-      P[p] -= A.lr * ((m * c1) / (sqrtf(v * c2) + A.eps) + wd * P[p]);
+      const float m = A.beta1 * M[p] + (1.0f - A.beta1) * g;
+      const float v = A.beta2 * V[p] + (1.0f - A.beta2) * g * g;
+      M[p] = m;
+      V[p] = v;
+      const float w = P[p] - A.lr * ((m * c1) / (sqrtf(v * c2) + A.eps) + wd * P[p]);
+      P[p] = w;
+      return w;
     };
-    if (j < HID) {
-      for (int i = 0; i < IN; i++) adam(OW1 + j * IN + i, g1[i], A.wd);
-      for (int i = 0; i < HID; i++) adam(OW2 + j * HID + i, g2[i], A.wd);
-      adam(OB1 + j, gb1[j], 0.f);
-      adam(OB2 + j, gb2[j], 0.f);
+    if (quad < 2) {                                     // the lanes that hold the 64 rows
+      float g[16];
+      if (cb == 0) {
+        tld16(lane_base + T_DW1, g);
+#pragma unroll
+        for (int i = 0; i < KIN; i++) g[i] = i < IN ? adam(pidx_w(OW1, HID, j, i < IN ? i : 0), g[i], A.wd) : 0.f;
+        st8(sm, S_W1, j, 0, KIN, g);
+        st8(sm, S_W1, j, 8, KIN, g + 8);
+      }
+      tld16(lane_base + T_DW2 + cb, g);
+#pragma unroll
+      for (int i = 0; i < 16; i++) g[i] = adam(pidx_w(OW2, HID, j, cb + i), g[i], A.wd);
+      st8(sm, S_W2, j, cb, HID, g);
+      st8(sm, S_W2, j, cb + 8, HID, g + 8);
+      if (quad == 0) {
+        tld16(lane_base + T_DW3 + cb, g);
+        if (j < OUT) {
+#pragma unroll
+          for (int i = 0; i < 16; i++) g[i] = adam(pidx_w(OW3, OUT, j, cb + i), g[i], A.wd);
+          st8(sm, S_W3, j, cb, HID, g);
+          st8(sm, S_W3, j, cb + 8, HID, g + 8);
+        }
+      }
+      if (cb == 16) adam(OB1 + j, gb1[j], 0.f);
+      if (cb == 32) adam(OB2 + j, gb2[j], 0.f);
+      if (cb == 48 && j < OUT) adam(OB3 + j, gb3[j], 0.f);
     }
-    if (j < OUT) {
-      for (int i = 0; i < HID; i++) adam(OW3 + j * HID + i, g3[i], A.wd);
-      adam(OB3 + j, gb3[j], 0.f);
-    }
-    __threadfence_block();
     tc_before();
     __syncthreads();
     tc_after();
-    stage_weights(sm, P, tid);
   }
+  if (A.mode == 2 && ok)
+    for (int p = tid; p < NPARAM; p += THREADS) {
+      int q = p;
+      if (p < OB1) q = pidx_w(OW1, HID, p / IN, p % IN);
+      else if (p >= OW2 && p < OB2) q = pidx_w(OW2, HID, (p - OW2) / HID, (p - OW2) % HID);
+      else if (p >= OW3 && p < OB3) q = pidx_w(OW3, OUT, (p - OW3) / HID, (p - OW3) % HID);
+      A.params[p] = P[q];
+    }
 
   // ---- after a wait that gave up, the MMAs it waited for may still run:
   // wait for their commit once more (with the full limit) before the TMEM
@@ -441,39 +551,36 @@ int call(int mode, float *params, const float *x, const float *t, int n, int ite
     cuda(cudaSetDevice(device), "cudaSetDevice");
     const size_t np = NPARAM * sizeof(float), nx = (size_t)n * IN * sizeof(float), ny = (size_t)n * OUT * sizeof(float);
     const int nloss = mode == 2 ? iters : 1;
-    DevBuf dP, dX, dT, dY, dG, dL, dM, dV, dS;
-    cuda(cudaMalloc(&dP.p, np), "cudaMalloc");
-    cuda(cudaMalloc(&dX.p, nx), "cudaMalloc");
-    cuda(cudaMalloc(&dT.p, ny), "cudaMalloc");
-    cuda(cudaMalloc(&dY.p, ny), "cudaMalloc");
-    cuda(cudaMalloc(&dG.p, np), "cudaMalloc");
-    cuda(cudaMalloc(&dL.p, nloss * sizeof(float)), "cudaMalloc");
-    cuda(cudaMalloc(&dM.p, np), "cudaMalloc");
-    cuda(cudaMalloc(&dV.p, np), "cudaMalloc");
-    cuda(cudaMalloc(&dS.p, sizeof(int)), "cudaMalloc");
-    cuda(cudaMemcpy(dP.p, params, np, cudaMemcpyHostToDevice), "upload");
-    cuda(cudaMemcpy(dX.p, x, nx, cudaMemcpyHostToDevice), "upload");
-    if (t) cuda(cudaMemcpy(dT.p, t, ny, cudaMemcpyHostToDevice), "upload");
-    cuda(cudaMemset(dM.p, 0, np), "memset");
-    cuda(cudaMemset(dV.p, 0, np), "memset");
-    cuda(cudaMemset(dS.p, 0, sizeof(int)), "memset");
+    // one allocation: status, parameters, x, t, y, gradient, loss
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t nl = nloss * sizeof(float);
+    const size_t oP = 256, oX = oP + up(np), oT = oX + up(nx), oY = oT + up(ny), oG = oY + up(ny), oL = oG + up(np);
+    DevBuf buf;
+    cuda(cudaMalloc(&buf.p, oL + up(nl)), "cudaMalloc");
+    char *base = static_cast<char *>(buf.p);
+    cuda(cudaMemset(base, 0, sizeof(int)), "memset");
+    cuda(cudaMemcpy(base + oP, params, np, cudaMemcpyHostToDevice), "upload");
+    cuda(cudaMemcpy(base + oX, x, nx, cudaMemcpyHostToDevice), "upload");
+    if (t) cuda(cudaMemcpy(base + oT, t, ny, cudaMemcpyHostToDevice), "upload");
     Args a{};
-    a.params = (float *)dP.p; a.x = (const float *)dX.p; a.t = (const float *)dT.p; a.n = n; a.mode = mode;
-    a.iters = iters; a.y = (float *)dY.p; a.grad = (float *)dG.p; a.loss = (float *)dL.p;
-    a.adam_m = (float *)dM.p; a.adam_v = (float *)dV.p; a.status = (int *)dS.p;
+    a.params = (float *)(base + oP); a.x = (const float *)(base + oX); a.t = (const float *)(base + oT); a.n = n;
+    a.mode = mode;
+    a.iters = iters; a.y = (float *)(base + oY); a.grad = (float *)(base + oG); a.loss = (float *)(base + oL);
+    a.status = (int *)base;
     a.wait_limit = g_wait_limit;
     if (adam) { a.lr = adam->lr; a.beta1 = adam->beta1; a.beta2 = adam->beta2; a.eps = adam->eps; a.wd = adam->weight_decay; }
     cuda(cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES), "smem attribute");
-    k_mlp<<<1, THREADS, SMEM_BYTES>>>(a);
+    // forward alone: a block per tile (a tile is 128 samples, at most 32 of them)
+    k_mlp<<<mode == 0 ? (n + ROWS - 1) / ROWS : 1, THREADS, SMEM_BYTES>>>(a);
     cuda(cudaGetLastError(), "launch of mlp kernel");
     cuda(cudaDeviceSynchronize(), "mlp kernel");
     int st = 0;
-    cuda(cudaMemcpy(&st, dS.p, sizeof(int), cudaMemcpyDeviceToHost), "status");
+    cuda(cudaMemcpy(&st, base, sizeof(int), cudaMemcpyDeviceToHost), "status");
     if (st) throw Error(st, "tensor-core wait timed out in the mlp kernel");
-    if (mode == 0) cuda(cudaMemcpy(y, dY.p, ny, cudaMemcpyDeviceToHost), "download");
-    if (mode == 1) cuda(cudaMemcpy(grad, dG.p, np, cudaMemcpyDeviceToHost), "download");
-    if (mode == 2) cuda(cudaMemcpy(params, dP.p, np, cudaMemcpyDeviceToHost), "download");
-    if (mode > 0) cuda(cudaMemcpy(loss, dL.p, nloss * sizeof(float), cudaMemcpyDeviceToHost), "download");
+    if (mode == 0) cuda(cudaMemcpy(y, a.y, ny, cudaMemcpyDeviceToHost), "download");
+    if (mode == 1) cuda(cudaMemcpy(grad, a.grad, np, cudaMemcpyDeviceToHost), "download");
+    if (mode == 2) cuda(cudaMemcpy(params, a.params, np, cudaMemcpyDeviceToHost), "download");
+    if (mode > 0) cuda(cudaMemcpy(loss, a.loss, nl, cudaMemcpyDeviceToHost), "download");
     return QB_OK;
   } catch (const Error &e) {
     set_error(e.what());
