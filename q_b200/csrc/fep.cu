@@ -136,11 +136,8 @@ __device__ __forceinline__ double evb_hij(const FepDev &D, int i, int j, double 
 // the file's lambdas from its first record.  With EVB coupling the ground
 // state of two states is the lower root of the 2 x 2 secular equation, with
 // the weights c1^2, c2^2 of the diabatic states; of more states, the lowest
-// eigenvalue of the EVB matrix (qfep.f90:310-318).
-__global__ void k_fep_values(FepDev D) {
-  const int f = blockIdx.y;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= D.npts[f]) return;
+// eigenvalue of the EVB matrix (qfep.f90:310-318).  Returns the gap.
+__device__ double point_values(const FepDev &D, int f, int p) {
   double tot[QB_FEP_MAX_STATES];
   for (int st = 0; st < D.ns; st++) {
     const double *e = rec(D, f, p, st);
@@ -177,48 +174,55 @@ __global__ void k_fep_values(FepDev D) {
   double g = 0.0;
   for (int st = 0; st < D.ns; st++) g = g + tot[st] * D.coeff[st];
   D.GAP[q] = g;
+  return g;
 }
 
-// Part 0 (qfep.f90:252-357): per file, the average of every component of
-// every state over the points after nskip, summed in record order and scaled
-// by the single-precision 1./(npts-nskip) of scale_ene.  One thread per
-// (state, component).
-__global__ void k_fep_part0(FepDev D, double *avEQ) {
-  const int f = blockIdx.x, t = threadIdx.x;
-  if (t >= D.ns * QB_NEQ) return;
-  const int st = t / QB_NEQ, c = t % QB_NEQ;
-  const int n = D.npts[f];
-  double s = 0.0;
-  for (int p = D.nskip; p < n; p++) {
-    const double *e = rec(D, f, p, st);
-    s += c == QB_EQ_TOTAL ? eq_total(D, e) : e[c];
-  }
-  const float k = 1.0f / (float)(n - D.nskip);
-  avEQ[((size_t)f * D.ns + st) * QB_NEQ + c] = c == QB_EQ_LAMBDA ? D.lam[f * D.ns + st] : s * (double)k;
-}
+// One block per file: the points' values, the file's energy-gap range over the
+// points after nskip from qfep's starting values 999 / -999 (qfep.f90:200-201,
+// 319-321), and Part 0 (qfep.f90:252-357), the average of every component of
+// every state over those points, scaled by the single-precision
+// 1./(npts-nskip) of scale_ene.  Part 0 takes FILE_SEGS threads per (state,
+// component), each over every FILE_SEGS-th record, their sums added in order:
+// a thread per component walking all records was a chain of loads (72 us for
+// 1,000 records; the three former kernels together 92, a call with the single allocation 2.4 to 1.6 ms).
+constexpr int FILE_COLS = 64, FILE_SEGS = 16, FILE_BLOCK = FILE_COLS * FILE_SEGS;
+static_assert(QB_FEP_MAX_STATES * QB_NEQ <= FILE_COLS, "a column per (state, component)");
 
-// Energy-gap range over the points after nskip, from qfep's starting values
-// 999 / -999 (qfep.f90:200-201, 319-321).
-__global__ void k_fep_gaprange(FepDev D, double *range) {
+__global__ void __launch_bounds__(FILE_BLOCK) k_fep_file(FepDev D, double *avEQ, double *range) {
+  __shared__ double part[FILE_SEGS][FILE_COLS];
   __shared__ double smin[32], smax[32];
+  const int f = blockIdx.x, n = D.npts[f];
   double mn = 999., mx = -999.;
-  for (int f = 0; f < D.nfiles; f++)
-    for (int p = D.nskip + threadIdx.x; p < D.npts[f]; p += blockDim.x) {
-      const double g = D.GAP[D.pstart[f] + p];
-      mn = fmin(mn, g);
-      mx = fmax(mx, g);
-    }
+  for (int p = threadIdx.x; p < n; p += FILE_BLOCK) {
+    const double g = point_values(D, f, p);
+    if (p >= D.nskip) { mn = fmin(mn, g); mx = fmax(mx, g); }
+  }
   for (int o = 16; o > 0; o >>= 1) {
     mn = fmin(mn, __shfl_xor_sync(FULLMASK, mn, o));
     mx = fmax(mx, __shfl_xor_sync(FULLMASK, mx, o));
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) { smin[w] = mn; smax[w] = mx; }
+  const int t = threadIdx.x % FILE_COLS, seg = threadIdx.x / FILE_COLS;
+  const int st = t / QB_NEQ, c = t % QB_NEQ;
+  double s = 0.0;
+  if (t < D.ns * QB_NEQ)
+    for (int p = D.nskip + seg; p < n; p += FILE_SEGS) {
+      const double *e = rec(D, f, p, st);
+      s += c == QB_EQ_TOTAL ? eq_total(D, e) : e[c];
+    }
+  part[seg][t] = s;
   __syncthreads();
+  if (seg == 0 && t < D.ns * QB_NEQ) {
+    double a = part[0][t];
+    for (int k = 1; k < FILE_SEGS; k++) a += part[k][t];
+    const float k = 1.0f / (float)(n - D.nskip);
+    avEQ[((size_t)f * D.ns + st) * QB_NEQ + c] = c == QB_EQ_LAMBDA ? rec(D, f, 0, st)[QB_EQ_LAMBDA] : a * (double)k;
+  }
   if (threadIdx.x == 0) {
-    for (int k = 1; k < (int)(blockDim.x >> 5); k++) { mn = fmin(mn, smin[k]); mx = fmax(mx, smax[k]); }
-    range[0] = fmin(smin[0], mn);
-    range[1] = fmax(smax[0], mx);
+    for (int k = 1; k < FILE_BLOCK / 32; k++) { mn = fmin(mn, smin[k]); mx = fmax(mx, smax[k]); }
+    range[2 * f] = fmin(smin[0], mn);
+    range[2 * f + 1] = fmax(smax[0], mx);
   }
 }
 
@@ -347,7 +351,9 @@ __global__ void k_fep_bins(FepDev D, const double *range, const double *dG, doub
     ac1[t] = 0.0; ac2[t] = 0.0; arx[t] = 0.0;
   }
   __syncthreads();
-  const double gapmin = range[0], xint = (range[1] - range[0]) / (double)D.nbins;
+  double gapmin = range[0], gapmax = range[1];
+  for (int k = 1; k < D.nfiles; k++) { gapmin = fmin(gapmin, range[2 * k]); gapmax = fmax(gapmax, range[2 * k + 1]); }
+  const double xint = (gapmax - gapmin) / (double)D.nbins;
   const double rt = D.rt;
   for (int p = D.nskip + threadIdx.x; p < D.npts[f]; p += blockDim.x) {
     const int q = D.pstart[f] + p;
@@ -398,24 +404,25 @@ __global__ void k_fep_bins(FepDev D, const double *range, const double *dG, doub
   }
 }
 
-template <class T>
-struct DevBuf {
-  T *p = nullptr;
-  explicit DevBuf(size_t n) { FEP_CUDA(cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T))); }
-  ~DevBuf() { if (p) cudaFree(p); }
-  DevBuf(const DevBuf &) = delete;
-  DevBuf &operator=(const DevBuf &) = delete;
+// The analysis's device memory: one allocation, cut into 256-byte aligned
+// pieces (twenty-two separate ones and their release took 1.9 ms of a call's
+// 2.4).  Pieces are laid out first, then allocated.
+struct Arena {
+  char *base = nullptr;
+  size_t bytes = 0;
+  size_t piece(size_t n) {
+    const size_t at = bytes;
+    bytes += (std::max<size_t>(n, 1) + 255) / 256 * 256;
+    return at;
+  }
+  void allocate() { FEP_CUDA(cudaMalloc(&base, bytes)); }
+  template <class T>
+  T *at(size_t off) const { return reinterpret_cast<T *>(base + off); }
+  ~Arena() { if (base) cudaFree(base); }
+  Arena() = default;
+  Arena(const Arena &) = delete;
+  Arena &operator=(const Arena &) = delete;
 };
-
-template <class T>
-void put(T *dst, const std::vector<T> &src, cudaStream_t s) {
-  if (!src.empty()) FEP_CUDA(cudaMemcpyAsync(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice, s));
-}
-
-template <class T>
-void get(std::vector<T> &dst, const T *src, cudaStream_t s) {
-  if (!dst.empty()) FEP_CUDA(cudaMemcpyAsync(dst.data(), src, dst.size() * sizeof(T), cudaMemcpyDeviceToHost, s));
-}
 
 template <class T>
 void give(T *out, const std::vector<T> &v) {
@@ -438,61 +445,87 @@ void fep_run(const FepSource &src, const qb_fep_params &p, int device, cudaStrea
   FEP_CUDA(cudaSetDevice(device));
   std::vector<int> pstart(nfiles);
   long long P = 0;
-  int maxn = 0;
-  for (int f = 0; f < nfiles; f++) { pstart[f] = (int)P; P += src.npts[f]; maxn = std::max(maxn, src.npts[f]); }
+  for (int f = 0; f < nfiles; f++) { pstart[f] = (int)P; P += src.npts[f]; }
   const int nb = p.nbins + 2;
 
-  DevBuf<long long> d_foff(nfiles);
-  DevBuf<int> d_npts(nfiles), d_pstart(nfiles), d_its(nfiles + 2);
-  DevBuf<double> d_lam((size_t)nfiles * ns), d_V((size_t)P * ns), d_VG(P), d_GAP(P);
-  DevBuf<double> d_C1(P), d_C2(P), d_RX(P);
-  DevBuf<long long> d_roff(nfiles);
   if (p.nnoffd < 0) fail(QB_ERR_ARG, "negative number of off-diagonal elements");
   if (p.nnoffd > 0 && (!src.rbase || (int)src.rfoff.size() != nfiles))
     fail(QB_ERR_ARG, "off-diagonal elements without r_xy values");
-  DevBuf<double> d_av((size_t)nfiles * ns * QB_NEQ), d_range(2);
-  DevBuf<double> d_dgf(nfiles + 2), d_dgr(nfiles + 2), d_dgti(nfiles + 2), d_dglu(nfiles + 2), d_dgbar(nfiles + 2);
-  DevBuf<double> d_dG(nfiles + 2), d_part2((size_t)nfiles * nb * QB_FEP_PART2_W);
-  put(d_foff.p, src.foff, stream);
-  put(d_npts.p, src.npts, stream);
-  put(d_pstart.p, pstart, stream);
-  if (p.nnoffd > 0) put(d_roff.p, src.rfoff, stream);
-  for (auto *b : {d_dgf.p, d_dgr.p, d_dgti.p, d_dglu.p, d_dgbar.p})
-    FEP_CUDA(cudaMemsetAsync(b, 0, sizeof(double) * (nfiles + 2), stream));
+  // per-file tables (uploaded together), per-point values, then the results in
+  // the order they are read back: the estimators (zeroed), lambdas, averages, gap ranges
+  Arena M;
+  const size_t nf2 = (size_t)nfiles + 2, P8 = sizeof(double) * (size_t)P;
+  const size_t tab = M.piece(2 * sizeof(long long) * nfiles + 2 * sizeof(int) * nfiles);
+  const size_t oV = M.piece(P8 * ns), oVG = M.piece(P8), oGAP = M.piece(P8), oC1 = M.piece(P8), oC2 = M.piece(P8),
+               oRX = M.piece(P8);
+  const size_t n_est = 5 * nf2, n_lam = (size_t)nfiles * ns, n_av = n_lam * QB_NEQ, n_rng = 2 * (size_t)nfiles;
+  const size_t res = M.piece(sizeof(double) * (n_est + n_lam + n_av + n_rng) + sizeof(int) * nf2);
+  const size_t n_p2 = (size_t)nfiles * nb * QB_FEP_PART2_W;
+  const size_t oP2 = M.piece(sizeof(double) * n_p2), odG = M.piece(sizeof(double) * nf2);
+  const size_t oE = M.piece(src.host ? sizeof(double) * (src.host_n + src.rhost_n) : 0);
+  M.allocate();
+  std::vector<char> th(2 * sizeof(long long) * nfiles + 2 * sizeof(int) * nfiles);
+  long long *t_foff = reinterpret_cast<long long *>(th.data()), *t_roff = t_foff + nfiles;
+  int *t_npts = reinterpret_cast<int *>(t_roff + nfiles), *t_start = t_npts + nfiles;
+  for (int f = 0; f < nfiles; f++) {
+    t_foff[f] = src.foff[f];
+    t_roff[f] = p.nnoffd > 0 ? src.rfoff[f] : 0;
+    t_npts[f] = src.npts[f];
+    t_start[f] = pstart[f];
+  }
+  FEP_CUDA(cudaMemcpyAsync(M.at<char>(tab), th.data(), th.size(), cudaMemcpyHostToDevice, stream));
+  const double *dE = src.base, *dR = src.rbase;
+  if (src.host) {       // the records, then (EVB) every record's r_xy
+    double *e = M.at<double>(oE);
+    FEP_CUDA(cudaMemcpyAsync(e, src.host, sizeof(double) * src.host_n, cudaMemcpyHostToDevice, stream));
+    if (src.rhost_n)
+      FEP_CUDA(cudaMemcpyAsync(e + src.host_n, src.rbase, sizeof(double) * src.rhost_n, cudaMemcpyHostToDevice, stream));
+    dE = e;
+    dR = e + src.host_n;
+  }
+  double *r_est = M.at<double>(res), *r_lam = r_est + n_est, *r_av = r_lam + n_lam, *r_rng = r_av + n_av;
+  int *r_its = reinterpret_cast<int *>(r_rng + n_rng);
+  double *d_part2 = M.at<double>(oP2), *d_dG = M.at<double>(odG);
+  FEP_CUDA(cudaMemsetAsync(r_est, 0, sizeof(double) * (n_est + n_lam + n_av + n_rng) + sizeof(int) * nf2, stream));
   // k_fep_bins writes the rows of bins that hold points; the others must read
   // as empty (count 0), whatever the allocation held before
-  FEP_CUDA(cudaMemsetAsync(d_part2.p, 0, sizeof(double) * (size_t)nfiles * nb * QB_FEP_PART2_W, stream));
-  FEP_CUDA(cudaMemsetAsync(d_its.p, 0, sizeof(int) * (nfiles + 2), stream));
+  FEP_CUDA(cudaMemsetAsync(d_part2, 0, sizeof(double) * n_p2, stream));
 
   FepDev D{};
-  D.E = src.base; D.foff = d_foff.p; D.npts = d_npts.p; D.pstart = d_pstart.p;
+  const long long *d_foff = M.at<long long>(tab), *d_roff = d_foff + nfiles;
+  const int *d_npts = reinterpret_cast<const int *>(d_roff + nfiles);
+  D.E = dE; D.foff = d_foff; D.npts = d_npts; D.pstart = d_npts + nfiles;
   D.rs = src.rec_stride; D.ns = ns; D.nfiles = nfiles; D.nskip = p.nskip; D.gas = p.gas;
   D.nbins = p.nbins; D.nmin = p.nmin; D.rt = p.rt;
   for (int st = 0; st < QB_FEP_MAX_STATES; st++) {
     D.alfa[st] = st == 0 ? 0.0 : p.alfa[st];      // alfa(1)=0. (qfep.f90:264)
     D.coeff[st] = p.coeff[st];
   }
-  D.lam = d_lam.p; D.V = d_V.p; D.VG = d_VG.p; D.GAP = d_GAP.p;
-  D.C1 = d_C1.p; D.C2 = d_C2.p; D.RX = d_RX.p;
-  D.nnoffd = p.nnoffd; D.R = src.rbase; D.roff = d_roff.p; D.rrs = src.r_stride;
+  D.lam = r_lam; D.V = M.at<double>(oV); D.VG = M.at<double>(oVG); D.GAP = M.at<double>(oGAP);
+  D.C1 = M.at<double>(oC1); D.C2 = M.at<double>(oC2); D.RX = M.at<double>(oRX);
+  D.nnoffd = p.nnoffd; D.R = dR; D.roff = d_roff; D.rrs = src.r_stride;
   for (int k = 0; k < QB_FEP_MAX_PAIRS; k++) {
     D.hA[k] = p.evb_A[k]; D.hmu[k] = p.evb_mu[k]; D.heta[k] = p.evb_eta[k]; D.hr0[k] = p.evb_rxy0[k];
   }
 
-  k_fep_values<<<dim3((maxn + FEP_BLOCK - 1) / FEP_BLOCK, nfiles), FEP_BLOCK, 0, stream>>>(D);
-  k_fep_part0<<<nfiles, 64, 0, stream>>>(D, d_av.p);
-  k_fep_gaprange<<<1, 1024, 0, stream>>>(D, d_range.p);
-  PairOut O{d_dgf.p, d_dgr.p, d_dgti.p, d_dglu.p, d_dgbar.p, d_its.p};
+  k_fep_file<<<nfiles, FILE_BLOCK, 0, stream>>>(D, r_av, r_rng);
+  PairOut O{r_est, r_est + nf2, r_est + 2 * nf2, r_est + 3 * nf2, r_est + 4 * nf2, r_its};
   k_fep_pairs<<<nfiles, FEP_BLOCK, 0, stream>>>(D, O);
   FEP_CUDA(cudaGetLastError());
 
-  std::vector<double> lam((size_t)nfiles * ns), av((size_t)nfiles * ns * QB_NEQ), range(2);
-  std::vector<double> dgf(nfiles + 2), dgr(nfiles + 2), dgti(nfiles + 2), dglu(nfiles + 2), dgbar(nfiles + 2);
-  std::vector<int> its(nfiles + 2);
-  get(lam, d_lam.p, stream); get(av, d_av.p, stream); get(range, d_range.p, stream);
-  get(dgf, d_dgf.p, stream); get(dgr, d_dgr.p, stream); get(dgti, d_dgti.p, stream);
-  get(dglu, d_dglu.p, stream); get(dgbar, d_dgbar.p, stream); get(its, d_its.p, stream);
+  std::vector<char> rh(sizeof(double) * (n_est + n_lam + n_av + n_rng) + sizeof(int) * nf2);
+  FEP_CUDA(cudaMemcpyAsync(rh.data(), r_est, rh.size(), cudaMemcpyDeviceToHost, stream));
   FEP_CUDA(cudaStreamSynchronize(stream));
+  const double *h = reinterpret_cast<const double *>(rh.data());
+  auto take = [&](size_t n) { std::vector<double> v(h, h + n); h += n; return v; };
+  const std::vector<double> dgf = take(nf2), dgr = take(nf2), dgti = take(nf2), dglu = take(nf2), dgbar = take(nf2);
+  const std::vector<double> lam = take(n_lam), av = take(n_av), frange = take(n_rng);
+  const std::vector<int> its(reinterpret_cast<const int *>(h), reinterpret_cast<const int *>(h) + nf2);
+  std::vector<double> range(frange.begin(), frange.begin() + 2);
+  for (int f = 1; f < nfiles; f++) {
+    range[0] = std::fmin(range[0], frange[2 * f]);
+    range[1] = std::fmax(range[1], frange[2 * f + 1]);
+  }
 
   // running sums over windows (qfep.f90:412-413, 436-437, 466-469, 511-512, 567, 586-589)
   std::vector<double> dgfsum(nfiles + 2, 0.0), dgrsum(nfiles + 2, 0.0), dG(nfiles + 2, 0.0);
@@ -508,14 +541,14 @@ void fep_run(const FepSource &src, const qb_fep_params &p, int device, cudaStrea
   for (int i = 2; i <= nfiles; i++) dG[i] = dG[i - 1] + 0.5 * (dgf[i - 1] - dgr[i]);
 
   // Part 2 on the device, Part 3 (qfep.f90:721-745) from its rows in file order
-  put(d_dG.p, dG, stream);
+  FEP_CUDA(cudaMemcpyAsync(d_dG, dG.data(), sizeof(double) * nf2, cudaMemcpyHostToDevice, stream));
   const size_t smem = (size_t)nb * (2 * ns + 5) * sizeof(double) + (size_t)nb * sizeof(int);
   if (smem > 48 * 1024)
     FEP_CUDA(cudaFuncSetAttribute(k_fep_bins, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_fep_bins<<<nfiles, FEP_BLOCK, smem, stream>>>(D, d_range.p, d_dG.p, d_part2.p);
+  k_fep_bins<<<nfiles, FEP_BLOCK, smem, stream>>>(D, r_rng, d_dG, d_part2);
   FEP_CUDA(cudaGetLastError());
   std::vector<double> part2((size_t)nfiles * nb * QB_FEP_PART2_W);
-  get(part2, d_part2.p, stream);
+  FEP_CUDA(cudaMemcpyAsync(part2.data(), d_part2, sizeof(double) * n_p2, cudaMemcpyDeviceToHost, stream));
   FEP_CUDA(cudaStreamSynchronize(stream));
 
   std::vector<double> binsum((size_t)nb * 4, 0.0), part3((size_t)nb * QB_FEP_PART3_W, 0.0);
@@ -585,34 +618,23 @@ extern "C" int qb_fep_analyze(const double *energies, const int *npts, int nfile
     }
     if (nstates < 1 || nstates > QB_FEP_MAX_STATES) qb::fail(QB_ERR_ARG, "number of states must be 1..4");
     if (p->nnoffd > 0 && !p->rxy) qb::fail(QB_ERR_ARG, "off-diagonal elements without r_xy values");
-    FEP_CUDA(cudaSetDevice(device));
-    cudaStream_t s;
-    FEP_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    double *dE = nullptr;
-    // the records, then (EVB) every record's r_xy
-    const long long nE = total * src.rec_stride, nR = p->nnoffd > 0 ? total : 0;
-    cudaError_t e = cudaMalloc(&dE, sizeof(double) * std::max<long long>(nE + nR, 1));
-    if (e != cudaSuccess) { cudaStreamDestroy(s); qb::fail(QB_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e)); }
-    try {
-      FEP_CUDA(cudaMemcpyAsync(dE, energies, sizeof(double) * nE, cudaMemcpyHostToDevice, s));
-      src.base = dE;
-      if (nR > 0) {
-        FEP_CUDA(cudaMemcpyAsync(dE + nE, p->rxy, sizeof(double) * nR, cudaMemcpyHostToDevice, s));
-        src.rbase = dE + nE;
-        src.r_stride = 1;
-        long long off = 0;
-        for (int f = 0; f < nfiles; f++) { src.rfoff.push_back(off); off += npts[f]; }
-      }
-      qb::fep_run(src, *p, device, s, out);
-    } catch (...) {
-      cudaStreamSynchronize(s);
-      cudaFree(dE);
-      cudaStreamDestroy(s);
-      throw;
+    const long long nE = total * src.rec_stride;
+    src.host = energies;
+    src.host_n = (size_t)nE;
+    if (p->nnoffd > 0) {
+      src.rbase = p->rxy;
+      src.rhost_n = (size_t)total;
+      src.r_stride = 1;
+      long long off = 0;
+      for (int f = 0; f < nfiles; f++) { src.rfoff.push_back(off); off += npts[f]; }
     }
-    cudaStreamSynchronize(s);
-    cudaFree(dE);
-    cudaStreamDestroy(s);
+    FEP_CUDA(cudaSetDevice(device));
+    struct Stream {
+      cudaStream_t s = nullptr;
+      ~Stream() { if (s) cudaStreamDestroy(s); }
+    } st;
+    FEP_CUDA(cudaStreamCreateWithFlags(&st.s, cudaStreamNonBlocking));
+    qb::fep_run(src, *p, device, st.s, out);
     return QB_OK;
   } catch (const qb::Error &e) {
     qb::set_error(e.what());

@@ -20,6 +20,10 @@ struct FepSource {
   const double *rbase = nullptr;
   std::vector<long long> rfoff;
   int r_stride = 0;
+  // records still on the host (instead of base): host_n doubles, and with EVB
+  // rhost_n r_xy values at rbase; fep_run copies them into its own allocation
+  const double *host = nullptr;
+  size_t host_n = 0, rhost_n = 0;
 };
 
 // Runs the analysis on `stream` and fills `out` (host buffers).  Throws
