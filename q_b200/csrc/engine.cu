@@ -241,7 +241,8 @@ struct Batch {
     };
     // the any-atom LRF windows read the group-pair bits
     if (any_any_atom) solute_lists();
-    fork_streams(2);
+    const unsigned used = (any_lrf ? 1u : 0u) | (max_nwat > 0 ? 2u : 0u);
+    fork_streams(used);
     if (any_lrf) {
       launch("lrf_gather", [&] {
         if (opt.precision == QB_MIXED) {
@@ -267,7 +268,7 @@ struct Batch {
       launch("list_qp", [&] { k_list_qp<<<nsys, QP_LIST_BLOCK, 0, stream>>>(p, force); });
       if (max_nwat > 0) launch("list_qw", [&] { k_list_qw<<<nsys, 256, 0, stream>>>(p, force); });
     }
-    join_streams(2);
+    join_streams(used);
     launch("lists_end", [&] { k_lists_end<<<cdiv(nsys, 128), 128, 0, stream>>>(p, force); });
     check_launch("list kernels");
   }
@@ -293,8 +294,8 @@ struct Batch {
     CUDA_TRY(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
   }
 
-  // Fork the side streams off the main stream / join them back (no-ops when
-  // profiling or without side streams).
+  // Fork the side streams of `mask` off the main stream / join them back
+  // (no-ops when profiling or without side streams).
   bool forking() const { return !profiling && side[0] && streams_on; }
 
   int max_lrfx_blocks = 1;   // the packed (two targets per thread) gather's grid
@@ -331,15 +332,16 @@ struct Batch {
     if (lrfx_cs == 4) k_lrf_gather_x2<BOX, ANY, 4><<<g, LRFX_BLOCK, 0, st>>>(P, force);
     else k_lrf_gather_x2<BOX, ANY, 1><<<g, LRFX_BLOCK, 0, st>>>(P, force);
   }
-  // the first n of them
-  void fork_streams(int n) {
+  void fork_streams(unsigned mask) {
     if (!forking()) return;
     CUDA_TRY(cudaEventRecord(ev_fork, stream));
-    for (int k = 0; k < n; k++) CUDA_TRY(cudaStreamWaitEvent(side[k], ev_fork, 0));
+    for (int k = 0; k < NSIDE; k++)
+      if (mask >> k & 1) CUDA_TRY(cudaStreamWaitEvent(side[k], ev_fork, 0));
   }
-  void join_streams(int n) {
+  void join_streams(unsigned mask) {
     if (!forking()) return;
-    for (int k = 0; k < n; k++) {
+    for (int k = 0; k < NSIDE; k++) {
+      if (!(mask >> k & 1)) continue;
       CUDA_TRY(cudaEventRecord(ev_join[k], side[k]));
       CUDA_TRY(cudaStreamWaitEvent(stream, ev_join[k], 0));
     }
@@ -380,7 +382,10 @@ struct Batch {
       }
     }
     cudaStream_t s1 = forking() ? side[0] : stream, s2 = forking() ? side[1] : stream;
-    fork_streams(4);
+    const bool qw_on = any_q && max_nwat > 0 && p.n_qw_tiles > 0;
+    const unsigned used = (max_nsol > 0 || max_terms > 0 ? 1u : 0u) | (qw_on ? 2u : 0u) | (any_wpol ? 4u : 0u) |
+                          (p.n_pw_groups > 0 || max_nsol > 0 ? 8u : 0u);
+    fork_streams(used);
     cudaStream_t s3 = forking() ? side[2] : stream, s4 = forking() ? side[3] : stream;
     // solute terms in one launch (nonbond_pp, nonbond_qp, bonded, nonbond_qq,
     // Q bonded, restraints)
@@ -442,7 +447,7 @@ struct Batch {
           else if (ww_direct) k_nb_ww_direct<false><<<gd, td, 0, stream>>>(p);
           else k_nb_ww<false, false><<<gw, WW_BLOCK, smem, stream>>>(p, wpb);
         });
-      if (any_q && p.n_qw_tiles > 0) launch("nb_qw", [&] {
+      if (qw_on) launch("nb_qw", [&] {
         const int g = p.n_qw_tiles, qg = qw_groups, nt = 32 * qw_warps;
         if (any_hlj) { k_nb_qw<0, true><<<g, nt, 0, s2>>>(p, qg); return; }   // the generic state count only
         // the mixed engine's non-recording steps: forces alone in FP32
@@ -468,7 +473,7 @@ struct Batch {
     if (any_wpol) {
       launch("watpol", [&] { k_watpol<<<dim3(std::max(max_nshell, 1), nsys), WPOL_BLOCK, watpol_smem, s3>>>(p); });
     }
-    join_streams(4);
+    join_streams(used);
     check_launch("force kernels");
   }
 
@@ -491,8 +496,7 @@ struct Batch {
   }
 
   // Graphs of a whole list cycle: NB steps from a rebuild step, captured
-  // once per pattern of energy-recording steps (bit k + 1: step k records;
-  // bit 0: the run ends with the cycle) and
+  // once per pattern of energy-evaluating steps (bit k: step k does) and
   // replayed as one launch.  Used when every system shares one non-bond
   // interval of at most 62 steps and no volume moves interrupt the cycle.
   std::map<unsigned long long, std::pair<cudaGraphExec_t, long long>> cycle_graphs;
@@ -506,12 +510,12 @@ struct Batch {
   // nsteps >= NB steps from a rebuild step as one cycle graph; `last`: the
   // cycle's last step is the run's last (it evaluates energies)
   void cycle(bool last) {
-    unsigned long long key = last ? 1ull : 0ull;
+    unsigned long long key = 0;
     const long long i0 = istep;
     for (int k = 0; k < NB; k++) {
       istep = i0 + k;
       const int ene = (opt.precision != QB_MIXED || energy_due() || (last && k == NB - 1)) ? 1 : 0;
-      if (ene) key |= 2ull << k;
+      if (ene) key |= 1ull << k;
     }
     istep = i0;
     auto it = cycle_graphs.find(key);
@@ -522,7 +526,7 @@ struct Batch {
       try {
         for (int k = 0; k < NB; k++) {
           istep = i0 + k;
-          const int ene = (key >> (k + 1)) & 1ull;
+          const int ene = (key >> k) & 1ull;
           step_kernels(k == 0 ? 1 : 0, ene);
         }
       } catch (...) {
@@ -847,6 +851,33 @@ void set_ww_tiles(Batch &B, int wpb) {
   CUDA_TRY(cudaMemcpy(B.P.ww_tiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice));
   B.P.n_ww_tiles = (int)tiles.size();
   B.ww_wpb = wpb;
+}
+
+// The most waters (O's at X, 9 doubles apart) within rc2 of one of them;
+// nearest images in a box.
+int most_neighbours(const double *X, int n, const double *box, double rc2) {
+  std::vector<double> x(n), y(n), z(n);
+  for (int i = 0; i < n; i++) { x[i] = X[9 * (size_t)i]; y[i] = X[9 * (size_t)i + 1]; z[i] = X[9 * (size_t)i + 2]; }
+  int most = 0;
+  for (int i = 0; i < n; i++) {
+    int c = 0;
+    if (!box) {
+      for (int j = 0; j < n; j++) {
+        const double dx = x[i] - x[j], dy = y[i] - y[j], dz = z[i] - z[j];
+        c += dx * dx + dy * dy + dz * dz <= rc2;
+      }
+    } else {
+      for (int j = 0; j < n; j++) {
+        double dx = x[i] - x[j], dy = y[i] - y[j], dz = z[i] - z[j];
+        dx -= box[0] * std::round(dx / box[0]);
+        dy -= box[1] * std::round(dy / box[1]);
+        dz -= box[2] * std::round(dz / box[2]);
+        c += dx * dx + dy * dy + dz * dz <= rc2;
+      }
+    }
+    most = std::max(most, c - 1);      // the water itself
+  }
+  return most;
 }
 
 void build(Batch &B, qb_handle *const *hs, int n) {
@@ -1277,13 +1308,7 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       if (V.nwat > 0 && V.ncgp_solute > 0)
         pwg_cap = std::max(pwg_cap, std::min(((int)(pwmax * 1.15) + 32 + 31) / 32 * 32, (V.nwat + 31) / 32 * 32));
       S.qw_cap = V.nwat + 16;
-      int mx = 0;
-      for (int iw = 0; iw < V.nwat; iw++) {
-        int c = 0;
-        for (int jw = 0; jw < V.nwat; jw++)
-          if (jw != iw && d2(X, V.nat_solute + 3 * iw, V.nat_solute + 3 * jw) <= rww * rww) c++;
-        mx = std::max(mx, c);
-      }
+      const int mx = most_neighbours(X + 3 * (size_t)V.nat_solute, V.nwat, pb ? V.boxlength : nullptr, rww * rww);
       ww_cap = std::max(ww_cap, ((int)(mx * 1.15) + 31) / 32 * 32);
     }
     S.pp_off = pp_tot; pp_tot += S.pp_cap;

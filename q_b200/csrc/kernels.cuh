@@ -3518,64 +3518,65 @@ __global__ void __launch_bounds__(KIN_BLOCK) k_kinetic(DevPtrs P) {
 
 // pot_energy's sums (md.f90:13500-13560): per-state Q totals, the
 // lambda-weighted Q terms and the potential.  Lane st handles state st (its
-// row loaded at once); lane 0 then adds the states in order and forms the
-// totals from one load of the system's energy terms.  The terms' accumulators
+// row loaded at once), lane k the system's term k; sums over terms run in the
+// reference's order through shuffles.  The terms' accumulators
 // (P.E, P.EQ) are read and zeroed for the next evaluation here, the results
 // kept in P.Eo, P.EQo: two memset nodes less at the head of every step (they
 // were 2 to 3 us of a single system's 63).
 __device__ __forceinline__ void finalize_energy(DevPtrs &P, int s) {
   const SysDev &S = P.sys[s];
   const int lane = threadIdx.x;
-  double *E = P.E + s * QB_NE, *Eo = P.Eo + s * QB_NE;
+  static_assert(QB_NE <= 32, "a lane per term");
   double w[7] = {0, 0, 0, 0, 0, 0, 0};   // this state's bond, angle, torsion, improper, qx_el, qx_vdw, restraint, x lambda
+  double e = 0.0;
+  if (lane < QB_NE) {
+    e = P.E[s * QB_NE + lane];
+    P.E[s * QB_NE + lane] = 0.0;
+  }
+  // the states' rows through shared memory: whole-warp loads and stores
+  __shared__ double row[MAXS * QB_NEQ];
+  double *q = P.EQ + (size_t)s * MAXS * QB_NEQ, *qo = P.EQo + (size_t)s * MAXS * QB_NEQ;
+  const int nq = S.S * QB_NEQ;
+  for (int k = lane; k < nq; k += 32) {
+    row[k] = q[k];
+    q[k] = 0.0;
+  }
+  __syncwarp();
   if (lane < S.S) {
-    double *q = P.EQ + ((size_t)s * MAXS + lane) * QB_NEQ;
-    double *qo = P.EQo + ((size_t)s * MAXS + lane) * QB_NEQ;
-    double r[QB_NEQ];
-#pragma unroll
-    for (int k = 0; k < QB_NEQ; k++) r[k] = q[k];
-#pragma unroll
-    for (int k = 0; k < QB_NEQ; k++) q[k] = 0.0;
+    double *r = row + lane * QB_NEQ;
     const double lam = S.lambda[lane];
     r[QB_EQ_LAMBDA] = lam;
     r[QB_EQ_QX_EL] = r[QB_EQ_QQ_EL] + r[QB_EQ_QP_EL] + r[QB_EQ_QW_EL];
     r[QB_EQ_QX_VDW] = r[QB_EQ_QQ_VDW] + r[QB_EQ_QP_VDW] + r[QB_EQ_QW_VDW];
     r[QB_EQ_TOTAL] = r[QB_EQ_BOND] + r[QB_EQ_ANGLE] + r[QB_EQ_TORSION] + r[QB_EQ_IMPROPER] + r[QB_EQ_QX_EL] +
                      r[QB_EQ_QX_VDW] + r[QB_EQ_RESTRAINT];
-#pragma unroll
-    for (int k = 0; k < QB_NEQ; k++) qo[k] = r[k];
     w[0] = r[QB_EQ_BOND] * lam; w[1] = r[QB_EQ_ANGLE] * lam; w[2] = r[QB_EQ_TORSION] * lam;
     w[3] = r[QB_EQ_IMPROPER] * lam; w[4] = r[QB_EQ_QX_EL] * lam; w[5] = r[QB_EQ_QX_VDW] * lam;
     w[6] = r[QB_EQ_RESTRAINT] * lam;
   }
-  double e[QB_NE];
-  if (lane == 0) {
+  __syncwarp();
+  for (int k = lane; k < nq; k += 32) qo[k] = row[k];
+  constexpr int into[7] = {QB_E_Q_BOND, QB_E_Q_ANGLE, QB_E_Q_TORSION, QB_E_Q_IMPROPER,
+                           QB_E_QX_EL, QB_E_QX_VDW, QB_E_RST_PROTEIN};
+  for (int k = 0; k < S.S; k++)
 #pragma unroll
-    for (int k = 0; k < QB_NE; k++) e[k] = E[k];
-#pragma unroll
-    for (int k = 0; k < QB_NE; k++) E[k] = 0.0;
-  }
-  for (int k = 0; k < S.S; k++) {
-    double v[7];
-#pragma unroll
-    for (int c = 0; c < 7; c++) v[c] = __shfl_sync(FULL, w[c], k);
-    if (lane == 0) {
-      e[QB_E_Q_BOND] += v[0]; e[QB_E_Q_ANGLE] += v[1]; e[QB_E_Q_TORSION] += v[2]; e[QB_E_Q_IMPROPER] += v[3];
-      e[QB_E_QX_EL] += v[4]; e[QB_E_QX_VDW] += v[5]; e[QB_E_RST_PROTEIN] += v[6];
+    for (int c = 0; c < 7; c++) {
+      const double v = __shfl_sync(FULL, w[c], k);
+      if (lane == into[c]) e += v;
     }
-  }
-  if (lane == 0) {
-    e[QB_E_RST_TOTAL] = e[QB_E_RST_FIX] + e[QB_E_RST_SHELL] + e[QB_E_RST_PROTEIN] + e[QB_E_RST_SOLVENT_RADIAL] +
-                        e[QB_E_RST_WATER_POL];
-    e[QB_E_POTENTIAL] = e[QB_E_P_BOND] + e[QB_E_W_BOND] + e[QB_E_P_ANGLE] + e[QB_E_W_ANGLE] + e[QB_E_P_TORSION] +
-                        e[QB_E_P_IMPROPER] + e[QB_E_PP_EL] + e[QB_E_PP_VDW] + e[QB_E_PW_EL] + e[QB_E_PW_VDW] +
-                        e[QB_E_WW_EL] + e[QB_E_WW_VDW] + e[QB_E_Q_BOND] + e[QB_E_Q_ANGLE] + e[QB_E_Q_TORSION] +
-                        e[QB_E_Q_IMPROPER] + e[QB_E_QX_EL] + e[QB_E_QX_VDW] + e[QB_E_RST_TOTAL] + e[QB_E_LRF];
-    e[QB_E_KINETIC] = P.st[s].kinetic;
-#pragma unroll
-    for (int k = 0; k < QB_NE; k++) Eo[k] = e[k];
-    if (!isfinite(e[QB_E_POTENTIAL])) set_status(&P.st[s], QB_ERR_NAN);
-  }
+  auto term = [&](int k) { return __shfl_sync(FULL, e, k); };
+  const double rst = term(QB_E_RST_FIX) + term(QB_E_RST_SHELL) + term(QB_E_RST_PROTEIN) +
+                     term(QB_E_RST_SOLVENT_RADIAL) + term(QB_E_RST_WATER_POL);
+  const double pot = term(QB_E_P_BOND) + term(QB_E_W_BOND) + term(QB_E_P_ANGLE) + term(QB_E_W_ANGLE) +
+                     term(QB_E_P_TORSION) + term(QB_E_P_IMPROPER) + term(QB_E_PP_EL) + term(QB_E_PP_VDW) +
+                     term(QB_E_PW_EL) + term(QB_E_PW_VDW) + term(QB_E_WW_EL) + term(QB_E_WW_VDW) + term(QB_E_Q_BOND) +
+                     term(QB_E_Q_ANGLE) + term(QB_E_Q_TORSION) + term(QB_E_Q_IMPROPER) + term(QB_E_QX_EL) +
+                     term(QB_E_QX_VDW) + rst + term(QB_E_LRF);
+  if (lane == QB_E_RST_TOTAL) e = rst;
+  if (lane == QB_E_POTENTIAL) e = pot;
+  if (lane == QB_E_KINETIC) e = P.st[s].kinetic;
+  if (lane < QB_NE) P.Eo[s * QB_NE + lane] = e;
+  if (lane == 0 && !isfinite(pot)) set_status(&P.st[s], QB_ERR_NAN);
   __syncwarp();
 }
 
