@@ -282,7 +282,7 @@ struct Batch {
   // Side streams of the force fork: after the water pass the force kernels of
   // a step (all adding with atomics) run on five streams and join before the
   // leap-frog.  Profiling keeps them on the main stream, one at a time.
-  static constexpr int NSIDE = 4;
+  static constexpr int NSIDE = 5;
   cudaStream_t side[NSIDE] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[NSIDE] = {};
 
@@ -366,15 +366,17 @@ struct Batch {
     DevPtrs &p = P;
     const bool mixed = opt.precision == QB_MIXED;
     const bool fast_ww = mixed && !ene;
-    // the water pass stores every water gradient and zeroes the solute's
-    if (!water_pass_zeroes) CUDA_TRY(cudaMemsetAsync(p.d, 0, sizeof(double4) * (size_t)p.natoms_tot, stream));
+    const bool early = p.dlast != nullptr;
+    // early: the gradient is zero already; else the water pass stores every
+    // water gradient and zeroes the solute's
+    if (!early && !water_pass_zeroes) CUDA_TRY(cudaMemsetAsync(p.d, 0, sizeof(double4) * (size_t)p.natoms_tot, stream));
     // waters first: their records, and their per-atom terms as the first
     // gradient contribution (plain stores after the zeroing)
-    if (max_nwat > 0) {
+    if (max_nwat > 0 && !early) {
       if (water_atom_threads) {
         dim3 gp(cdiv(std::max(3 * max_nwat, max_nsol), 256), nsys);
-        if (fast_ww) launch("pack_waters", [&] { k_pack_water_atoms<true><<<gp, 256, 0, stream>>>(p); });
-        else launch("pack_waters", [&] { k_pack_water_atoms<false><<<gp, 256, 0, stream>>>(p); });
+        if (fast_ww) launch("pack_waters", [&] { k_pack_water_atoms<true, false><<<gp, 256, 0, stream>>>(p); });
+        else launch("pack_waters", [&] { k_pack_water_atoms<false, false><<<gp, 256, 0, stream>>>(p); });
       } else if (p.n_pk_tiles > 0) {
         const int gp = p.n_pk_tiles;
         if (fast_ww) launch("pack_waters", [&] { k_pack_waters<true><<<gp, 256, 0, stream>>>(p); });
@@ -384,8 +386,12 @@ struct Batch {
     cudaStream_t s1 = forking() ? side[0] : stream, s2 = forking() ? side[1] : stream;
     const bool qw_on = any_q && max_nwat > 0 && p.n_qw_tiles > 0;
     const unsigned used = (max_nsol > 0 || max_terms > 0 ? 1u : 0u) | (qw_on ? 2u : 0u) | (any_wpol ? 4u : 0u) |
-                          (p.n_pw_groups > 0 || max_nsol > 0 ? 8u : 0u);
+                          (p.n_pw_groups > 0 || max_nsol > 0 ? 8u : 0u) | (early ? 16u : 0u);
     fork_streams(used);
+    if (early) {
+      cudaStream_t s5 = forking() ? side[4] : stream;
+      launch("pack_waters", [&] { k_pack_water_atoms<false, true><<<dim3(cdiv(3 * max_nwat, 128), nsys), 128, 0, s5>>>(p); });
+    }
     cudaStream_t s3 = forking() ? side[2] : stream, s4 = forking() ? side[3] : stream;
     // solute terms in one launch (nonbond_pp, nonbond_qp, bonded, nonbond_qq,
     // Q bonded, restraints)
@@ -471,7 +477,11 @@ struct Batch {
     if (max_nsol > 0)
       launch("atom_terms", [&] { k_atom_terms<<<dim3(cdiv(max_nsol, 128), nsys), 128, 0, s4>>>(p); });
     if (any_wpol) {
-      launch("watpol", [&] { k_watpol<<<dim3(std::max(max_nshell, 1), nsys), WPOL_BLOCK, watpol_smem, s3>>>(p); });
+      launch("watpol", [&] { 
+        const dim3 g(std::max(max_nshell, 1), nsys);
+        if (early) k_watpol<true><<<g, WPOL_BLOCK, watpol_smem, s3>>>(p);
+        else k_watpol<false><<<g, WPOL_BLOCK, watpol_smem, s3>>>(p);
+      });
     }
     join_streams(used);
     check_launch("force kernels");
@@ -544,12 +554,41 @@ struct Batch {
       it = cycle_graphs.emplace(key, std::make_pair(ge, launches - l0)).first;
       launches = l0;
     }
+    clean_gradient();
+    evaluated(true);
     CUDA_TRY(cudaGraphLaunch(it->second.first, stream));
     launches += it->second.second;
     istep = i0 + NB;
   }
 
   bool lists_stale = false;
+
+  // Early force kernels: d is zero before every evaluation.  The steps leave
+  // it so (their leap-frog moves it to dlast); after any other evaluation
+  // it is zeroed here, outside the captured graphs.
+  bool d_zero = false, grad_in_dlast = false;
+  void clean_gradient() {
+    if (P.dlast && !d_zero) CUDA_TRY(cudaMemsetAsync(P.d, 0, sizeof(double4) * (size_t)P.natoms_tot, stream));
+    d_zero = P.dlast != nullptr;
+  }
+  // the gradient of the last evaluation: of a step (leap-frogged) or not
+  double4 *gradient() const { return P.dlast && grad_in_dlast ? P.dlast : P.d; }
+  void evaluated(bool leapfrogged) {
+    grad_in_dlast = leapfrogged;
+    if (!leapfrogged) d_zero = false;
+  }
+
+  // whether this batch takes the early force kernels: one fork at the head of
+  // a step with the water pass's terms among the other forces.  Batches with
+  // the unstaged water-water kernels only (the staged ones read the pass's
+  // records): the pass and a launch gap, 7 us, leave the chain of a step.
+  // 15 A sphere 29.6 to 24.6 us a step, one window 36.9 to 34.7, two 43.6 to 41.
+  // (the FP32 kernel of water with hydrogen LJ reads the pass's records)
+  void set_early() {
+    P.dlast = ww_direct && water_pass_zeroes && !(any_hlj && opt.precision == QB_MIXED) ? dlast_buf : nullptr;
+    d_zero = false;
+  }
+  double4 *dlast_buf = nullptr;
 
   void step() {
     int due = lists_due() ? 1 : 0;
@@ -559,6 +598,8 @@ struct Batch {
       due = 0;
     }
     const int ene = (opt.precision != QB_MIXED || force_energy || energy_due()) ? 1 : 0;
+    clean_gradient();
+    evaluated(true);
     if (!use_graphs || profiling) { step_kernels(due, ene); istep++; return; }
     cudaGraphExec_t &ge = graph[due][ene];
     if (!ge) {
@@ -628,7 +669,9 @@ struct Batch {
   // Energies of the current coordinates as new_potential takes them: the full
   // evaluation (the lists as they stand), summed; E and EQ copied out.
   void evaluate_into(std::vector<double> &E, std::vector<double> &EQ) {
+    clean_gradient();
     pot_energy(1);
+    evaluated(false);
     k_finish<<<nsys, 32, 0, stream>>>(P, 2);
     check_launch("energy sums");
     E.resize((size_t)nsys * QB_NE);
@@ -1601,6 +1644,8 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     P.n_wd_tiles = (int)wd.size();
     P.wd_tiles = dev_upload(wd, o);
     B.ww_direct = B.ww_direct_fits();
+    if (B.ww_direct && B.water_pass_zeroes) B.dlast_buf = dev_alloc<double4>(P.natoms_tot, o);
+    B.set_early();
   }
   P.ww_cap = ww_cap;
   P.ww = dev_alloc<uint16_t>((size_t)std::max(woff, 1) * ww_cap, o);
@@ -1641,7 +1686,8 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   P.wshell = dev_alloc<int8_t>(std::max(woff, 1), o);
   if (B.any_wpol) {
     if (B.watpol_smem > 200 * 1024) fail(QB_ERR_UNSUPPORTED, "too many waters for the polarisation kernel");
-    CUDA_TRY(cudaFuncSetAttribute(k_watpol, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(k_watpol<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CUDA_TRY(cudaFuncSetAttribute(k_watpol<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   }
 }
 
@@ -1872,7 +1918,10 @@ void set_tuning(Batch &B, const qb_tuning &t, bool share) {
   if (t.ww_waters_per_block != B.ww_wpb) set_ww_tiles(B, t.ww_waters_per_block);
   // a chosen chunk or block size is one of the staged kernels'; the defaults
   // leave small batches without staging
-  if (staged) B.ww_direct = t.ww_chunk == B.ww_chunk_max && t.ww_waters_per_block == B.ww_wpb0 && B.ww_direct_fits();
+  if (staged) {
+    B.ww_direct = t.ww_chunk == B.ww_chunk_max && t.ww_waters_per_block == B.ww_wpb0 && B.ww_direct_fits();
+    B.set_early();
+  }
   B.water_atom_threads = t.water_pass_per_atom != 0;
   B.lists_stale = true;   // the water-water split counts depend on the chunk
 }
@@ -2009,7 +2058,9 @@ int qb_batch_evaluate(qb_batch *bb, int energies) {
     Batch &B = bb->b;
     CUDA_TRY(cudaSetDevice(B.opt.device));
     B.build_lists(1);
+    B.clean_gradient();
     B.pot_energy(B.opt.precision == QB_MIXED ? energies : 1);
+    B.evaluated(false);
     qb::k_finish<<<B.nsys, 32, 0, B.stream>>>(B.P, 2);
     B.check_launch("energy sums");
     B.sync_status();
@@ -2071,7 +2122,7 @@ static int set_vec(qb_batch *bb, int sys, double4 *dst, const double *in) {
   });
 }
 
-int qb_batch_gradient(qb_batch *b, int sys, double *d) { return get_vec(b, sys, b ? b->b.P.d : nullptr, d); }
+int qb_batch_gradient(qb_batch *b, int sys, double *d) { return get_vec(b, sys, b ? b->b.gradient() : nullptr, d); }
 int qb_batch_get_coords(qb_batch *b, int sys, double *x) { return get_vec(b, sys, b ? b->b.P.x : nullptr, x); }
 int qb_batch_set_coords(qb_batch *b, int sys, const double *x) {
   int rc = set_vec(b, sys, b ? b->b.P.x : nullptr, x);

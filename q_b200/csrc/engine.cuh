@@ -129,6 +129,7 @@ struct DevPtrs {
   SysState *st;
   // atoms
   double4 *x, *v, *xx, *d;
+  double4 *dlast;            // early force kernels: the last step's gradient (d is zero between steps); else null
   float4 *wrec;              // per-water position records of the water-water kernel
   float4 *wrec32;            // their FP32 form (mixed engine): the packed and FP32 water-water kernels'
   double *wtheta;            // per water: dipole angle of the polarisation restraint

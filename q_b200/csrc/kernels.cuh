@@ -1133,29 +1133,37 @@ constexpr int WW_STAGE_BYTES = 112 * 1024;    // staged records per block: two b
 // watpol (md.f90:15122), per water: the angle between the water dipole and
 // the radius vector from the restraint centre, and the polarisation shell the
 // O lies in (-1: none, or excluded).
+__device__ __forceinline__ int watpol_shell(const SysDev &S, const double *rcu0, double &rc) {
+  rc = sqrt(rcu0[0] * rcu0[0] + rcu0[1] * rcu0[1] + rcu0[2] * rcu0[2]);
+  const int ns = S.nshell;
+  float inner = S.ws_rout[ns - 1] - S.ws_dr[ns - 1];
+  if (!(rc > (double)inner)) return -1;
+  int is;
+  for (is = ns - 1; is >= 1; is--)
+    if (rc <= (double)S.ws_rout[is]) break;
+  return is;
+}
+
+__device__ __forceinline__ double watpol_theta(double4 xO, double4 x1, double4 x2, const double *rcu0, double rc) {
+  double rmu[3] = {x1.x + x2.x - 2. * xO.x, x1.y + x2.y - 2. * xO.y, x1.z + x2.z - 2. * xO.z};
+  double rm = sqrt(rmu[0] * rmu[0] + rmu[1] * rmu[1] + rmu[2] * rmu[2]);
+  double rcu[3];
+  for (int k = 0; k < 3; k++) { rmu[k] /= rm; rcu[k] = rcu0[k] / rc; }
+  double scp = rmu[0] * rcu[0] + rmu[1] * rcu[1] + rmu[2] * rcu[2];
+  if (scp > 1.0) scp = 1.0;
+  if (scp < -1.0) scp = -1.0;
+  return acos(scp);
+}
+
 __device__ __forceinline__ void watpol_angle(const DevPtrs &P, const SysDev &S, int gw, bool excl, double4 xO,
                                              double4 x1, double4 x2) {
   int shell = -1;
   double theta = 0.0;
   if (!excl) {
-    double rmu[3] = {x1.x + x2.x - 2. * xO.x, x1.y + x2.y - 2. * xO.y, x1.z + x2.z - 2. * xO.z};
-    double rm = sqrt(rmu[0] * rmu[0] + rmu[1] * rmu[1] + rmu[2] * rmu[2]);
-    for (int k = 0; k < 3; k++) rmu[k] /= rm;
-    double rcu[3] = {xO.x - S.xw[0], xO.y - S.xw[1], xO.z - S.xw[2]};
-    double rc = sqrt(rcu[0] * rcu[0] + rcu[1] * rcu[1] + rcu[2] * rcu[2]);
-    for (int k = 0; k < 3; k++) rcu[k] /= rc;
-    double scp = rmu[0] * rcu[0] + rmu[1] * rcu[1] + rmu[2] * rcu[2];
-    if (scp > 1.0) scp = 1.0;
-    if (scp < -1.0) scp = -1.0;
-    theta = acos(scp);
-    const int ns = S.nshell;
-    float inner = S.ws_rout[ns - 1] - S.ws_dr[ns - 1];
-    if (rc > (double)inner) {
-      int is;
-      for (is = ns - 1; is >= 1; is--)
-        if (rc <= (double)S.ws_rout[is]) break;
-      shell = is;
-    }
+    const double rcu0[3] = {xO.x - S.xw[0], xO.y - S.xw[1], xO.z - S.xw[2]};
+    double rc;
+    shell = watpol_shell(S, rcu0, rc);
+    theta = watpol_theta(xO, x1, x2, rcu0, rc);
   }
   P.wtheta[gw] = theta;
   P.wshell[gw] = (int8_t)shell;
@@ -1400,6 +1408,15 @@ __global__ void __launch_bounds__(WW_BLOCK, MIXED ? 2 : 1) k_nb_ww(DevPtrs P, in
 
 // ----------------------------------------------- packed FP32x2 water-water
 
+// The packed record of one water: O as hi + lo, the H offsets from it.
+__device__ __forceinline__ void wat_record(const double4 &a, const double4 &b, const double4 &c, float4 *r) {
+  const float hx = (float)a.x, hy = (float)a.y, hz = (float)a.z;
+  const float lx = (float)(a.x - (double)hx), ly = (float)(a.y - (double)hy), lz = (float)(a.z - (double)hz);
+  r[0] = make_float4(hx, hy, hz, lx);
+  r[1] = make_float4(ly, lz, (float)(b.x - a.x), (float)(c.x - a.x));
+  r[2] = make_float4((float)(b.y - a.y), (float)(c.y - a.y), (float)(b.z - a.z), (float)(c.z - a.z));
+}
+
 // Operands of water i on the packed path: O as hi + lo, the H offsets negated
 // in both orders ({-rH1, -rH2} and {-rH2, -rH1}, per component).
 struct WwI2 {
@@ -1601,8 +1618,8 @@ __global__ void __launch_bounds__(WWX_BLOCK, 2) k_nb_ww_x2(DevPtrs P, int wpb) {
 
 // The water-water kernels of batches whose staged blocks cannot fill the SMs
 // (Batch::ww_direct): a warp per water (FP64) or half a warp (packed FP32), its
-// neighbours' records read where they lie (L1 and L2 hold one system's), no
-// staging and no barrier before the pairs.  The list walk, the pair terms and,
+// neighbours' coordinates read where they lie (L1 and L2 hold one system's), no
+// records, no staging and no barrier before the pairs.  The list walk, the pair terms and,
 // for the packed form, each lane's entries and the order of its FP32 sums are
 // those of k_nb_ww and k_nb_ww_x2 on one chunk, so the packed forces are the
 // same bit for bit.  One 1,035-water window: FP64 14 to 7 us, packed 7.8 to 4;
@@ -1612,7 +1629,6 @@ constexpr int WWD_WATERS = 8;               // waters per block, (system, first 
 template <bool HLJ, bool EONCE = false>
 __global__ void __launch_bounds__(32 * WWD_WATERS, 2) k_nb_ww_direct(DevPtrs P) {
   __shared__ double ered[WWD_WATERS][2];
-  constexpr int W = WatRec<false>::words;
   const int2 tile = P.wd_tiles[blockIdx.x];
   const int s = tile.x;
   const SysDev &S = P.sys[s];
@@ -1624,10 +1640,9 @@ __global__ void __launch_bounds__(32 * WWD_WATERS, 2) k_nb_ww_direct(DevPtrs P) 
     const int ke = P.ww_n[gw];
     int k = (EONCE ? P.ww_mid[gw] : 0) + lane;
     int jn = k < ke ? (int)nb[k] : 0;
-    const double2 *rec = reinterpret_cast<const double2 *>(P.wrec + (size_t)S.woff * W);
-    const double2 *rd = rec + (size_t)iw * W;
-    const double2 d0 = rd[0], d1 = rd[1], d2 = rd[2], d3 = rd[3], d4 = rd[4];
-    const double xi[9] = {d0.x, d0.y, d1.x, d1.y, d2.x, d2.y, d3.x, d3.y, d4.x};
+    const double4 *x = P.x + S.aoff + S.nsol;
+    const double4 i0 = x[3 * iw], i1 = x[3 * iw + 1], i2 = x[3 * iw + 2];
+    const double xi[9] = {i0.x, i0.y, i0.z, i1.x, i1.y, i1.z, i2.x, i2.y, i2.z};
     const float qo = S.crg_ow, qh = S.crg_hw;
     const double qoo = (double)(qo * qo), qoh = (double)(qo * qh), qhh = (double)(qh * qh);
     const double ljd[6] = {S.A_OO, S.B_OO, S.A_OH, S.B_OH, S.A_HH, S.B_HH};
@@ -1637,10 +1652,9 @@ __global__ void __launch_bounds__(32 * WWD_WATERS, 2) k_nb_ww_direct(DevPtrs P) 
 #pragma unroll
     for (int q = 0; q < 9; q++) fd[q] = 0.0;
     for (; k < ke; k += 32) {
-      const double2 *rj = rec + (size_t)jn * W;
-      const double2 v0 = rj[0], v1 = rj[1], v2 = rj[2], v3 = rj[3], v4 = rj[4];
+      const double4 v0 = x[3 * jn], v1 = x[3 * jn + 1], v2 = x[3 * jn + 2];
       if (k + 32 < ke) jn = nb[k + 32];
-      double xj[9] = {v0.x, v0.y, v1.x, v1.y, v2.x, v2.y, v3.x, v3.y, v4.x};
+      double xj[9] = {v0.x, v0.y, v0.z, v1.x, v1.y, v1.z, v2.x, v2.y, v2.z};
       if (box) {
         const double3 t = image_shift(bx, xj[0] - xi[0], xj[1] - xi[1], xj[2] - xi[2]);
 #pragma unroll
@@ -1672,7 +1686,6 @@ __global__ void __launch_bounds__(32 * WWD_WATERS, 2) k_nb_ww_direct(DevPtrs P) 
 
 template <bool BOX>
 __global__ void __launch_bounds__(16 * WWD_WATERS, 4) k_nb_ww_x2_direct(DevPtrs P) {
-  constexpr int W = WatRec<true>::words;
   const int2 tile = P.wd_tiles[blockIdx.x];
   const int s = tile.x;
   const SysDev &S = P.sys[s];
@@ -1683,7 +1696,7 @@ __global__ void __launch_bounds__(16 * WWD_WATERS, 4) k_nb_ww_x2_direct(DevPtrs 
   const int ke = P.ww_n[gw];
   if (ke == 0) return;
   const uint16_t *nb = P.ww + (size_t)gw * P.ww_cap;
-  const float4 *rec = P.wrec32 + (size_t)S.woff * W;
+  const double4 *x = P.x + S.aoff + S.nsol;
   int jn = hl < ke ? (int)nb[hl] : 0;
   const float qo = S.crg_ow, qh = S.crg_hw;
   const float qoo = qo * qo;
@@ -1700,15 +1713,19 @@ __global__ void __launch_bounds__(16 * WWD_WATERS, 4) k_nb_ww_x2_direct(DevPtrs 
     }
   }
   WwI2 I;
-  ww_load_i(rec + (size_t)iw * W, I);
+  {
+    float4 r[3];
+    wat_record(x[3 * iw], x[3 * iw + 1], x[3 * iw + 2], r);
+    ww_load_i(r, I);
+  }
   float2 gO[3], gH[3], gHs[3];
 #pragma unroll
   for (int q = 0; q < 3; q++) gO[q] = gH[q] = gHs[q] = make_float2(0.f, 0.f);
   for (int k = hl; k < ke; k += 16) {
-    const float4 *rj = rec + (size_t)jn * W;
-    const float4 j0 = rj[0], j1 = rj[1], j2 = rj[2];
+    float4 r[3];
+    wat_record(x[3 * jn], x[3 * jn + 1], x[3 * jn + 2], r);
     if (k + 16 < ke) jn = nb[k + 16];
-    ww_force_x2<BOX>(I, j0, j1, j2, qoh2, qhh2, qoo, A, B, gO, gH, gHs, Lh, Ll, iL);
+    ww_force_x2<BOX>(I, r[0], r[1], r[2], qoh2, qhh2, qoo, A, B, gO, gH, gHs, Lh, Ll, iL);
   }
   ww_store_i(P, S.aoff + S.nsol + 3 * iw, hl, hmask, gO, gH, gHs);
 }
@@ -2469,12 +2486,7 @@ __global__ void k_atom_terms(DevPtrs P) {
 template <bool MIXED>
 __device__ __forceinline__ void put_wat_records(const DevPtrs &P, int gw, double4 a, double4 b, double4 c) {
   if (MIXED || P.wrec32) {
-    float4 *r = P.wrec32 + (size_t)gw * WatRec<true>::words;
-    float hx = (float)a.x, hy = (float)a.y, hz = (float)a.z;
-    float lx = (float)(a.x - (double)hx), ly = (float)(a.y - (double)hy), lz = (float)(a.z - (double)hz);
-    r[0] = make_float4(hx, hy, hz, lx);
-    r[1] = make_float4(ly, lz, (float)(b.x - a.x), (float)(c.x - a.x));
-    r[2] = make_float4((float)(b.y - a.y), (float)(c.y - a.y), (float)(b.z - a.z), (float)(c.z - a.z));
+    wat_record(a, b, c, P.wrec32 + (size_t)gw * WatRec<true>::words);
   }
   if (!MIXED) {
     double2 *rd = reinterpret_cast<double2 *>(P.wrec + (size_t)gw * WatRec<false>::words);
@@ -2518,21 +2530,23 @@ __global__ void k_pack_waters(DevPtrs P) {
 // polarisation angle, the second H's the water's record): three times the
 // threads of k_pack_waters for batches too small to fill the GPU with one
 // thread per water.
-template <bool MIXED>
+// EARLY: the terms alone, added to the zeroed gradient beside the other force
+// kernels (no records, no angles, nothing waits for it).
+template <bool MIXED, bool EARLY>
 __global__ void k_pack_water_atoms(DevPtrs P) {
   int s = blockIdx.y;
   const SysDev &S = P.sys[s];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int iw = t / 3, a = t - 3 * iw;     // water, and its atom this thread takes
   double elrf = 0, efix = 0, eshell = 0, erad = 0;
-  if (t < S.nsol) P.d[S.aoff + t] = make_double4(0.0, 0.0, 0.0, 0.0);   // the solute's gradient zeroed
+  if (!EARLY && t < S.nsol) P.d[S.aoff + t] = make_double4(0.0, 0.0, 0.0, 0.0);   // the solute's gradient zeroed
   if (iw < S.nwat) {
     const int o = S.aoff + S.nsol + 3 * iw, i = o + a;
     const double4 xa4 = P.x[i];
     const double3 xa = make_double3(xa4.x, xa4.y, xa4.z);
-    if (a == 1 && S.wpol && S.nshell > 0)
+    if (!EARLY && a == 1 && S.wpol && S.nshell > 0)
       watpol_angle(P, S, S.woff + iw, (P.flags[o] & F_EXCL) != 0, P.x[o], xa4, P.x[o + 2]);
-    if (a == 2) put_wat_records<MIXED>(P, S.woff + iw, P.x[o], P.x[o + 1], xa4);
+    if (!EARLY && a == 2) put_wat_records<MIXED>(P, S.woff + iw, P.x[o], P.x[o + 1], xa4);
     double g[3] = {0, 0, 0};
     const uint8_t fo = P.flags[o], fl = P.flags[i];
     if (S.use_lrf && !((fo & P.flags[o + 1] & P.flags[o + 2]) & F_EXCL) && !(fl & F_EXCL) && P.iq[i] < 0) {
@@ -2556,7 +2570,8 @@ __global__ void k_pack_water_atoms(DevPtrs P) {
       erad += e;
       for (int k = 0; k < 3; k++) g[k] += dv * dr[k];
     }
-    P.d[i] = make_double4(g[0], g[1], g[2], 0.0);
+    if (EARLY) add_grad(P, i, g);
+    else P.d[i] = make_double4(g[0], g[1], g[2], 0.0);
   }
   warp_add(&P.E[s * QB_NE + QB_E_LRF], elrf);
   warp_add(&P.E[s * QB_NE + QB_E_RST_FIX], efix);
@@ -3079,6 +3094,9 @@ __device__ __forceinline__ int wpol_bin(double th) {
   return max(min(b, WPOL_BINS - 1), 0);
 }
 
+// EARLY: the members' angles are taken here from the coordinates, so that the
+// kernel does not wait for the water pass.
+template <bool EARLY>
 __global__ void __launch_bounds__(WPOL_BLOCK) k_watpol(DevPtrs P) {
   extern __shared__ unsigned char smem[];
   const int is = blockIdx.x, s = blockIdx.y;
@@ -3102,21 +3120,47 @@ __global__ void __launch_bounds__(WPOL_BLOCK) k_watpol(DevPtrs P) {
   uint16_t *ord = kiw + nw;                     // members in bin order
   for (int w0 = 0; w0 < nw; w0 += WPOL_BLOCK) {
     const int iw = w0 + threadIdx.x;
-    const bool mine = iw < nw && wsh[iw] == is;
+    bool mine = iw < nw;
+    if (EARLY) {
+      const int o = S.aoff + S.nsol + 3 * iw;
+      mine = mine && !(P.flags[o] & F_EXCL);
+      if (mine) {
+        const double4 x = P.x[o];
+        const double rcu0[3] = {x.x - S.xw[0], x.y - S.xw[1], x.z - S.xw[2]};
+        double rc;
+        mine = watpol_shell(S, rcu0, rc) == is;
+      }
+    } else {
+      mine = mine && wsh[iw] == is;
+    }
     const unsigned bal = __ballot_sync(FULL, mine);
     int base = 0;
     if (lane == 0 && bal) base = atomicAdd(&cnt, __popc(bal));
     base = __shfl_sync(FULL, base, 0);
     if (mine) {
       const int k = base + __popc(bal & ((1u << lane) - 1u));
-      const double th = wth[iw];
-      kth[k] = __double_as_longlong(th);
       kiw[k] = (uint16_t)iw;
-      atomicAdd(&bin[wpol_bin(th)], 1);
+      if (!EARLY) {
+        const double th = wth[iw];
+        kth[k] = __double_as_longlong(th);
+        atomicAdd(&bin[wpol_bin(th)], 1);
+      }
     }
   }
   __syncthreads();
   const int n = cnt;
+  if (EARLY) {
+    for (int m = threadIdx.x; m < n; m += WPOL_BLOCK) {
+      const int o = S.aoff + S.nsol + 3 * (int)kiw[m];
+      const double4 xO = P.x[o];
+      const double rcu0[3] = {xO.x - S.xw[0], xO.y - S.xw[1], xO.z - S.xw[2]};
+      const double rc = sqrt(rcu0[0] * rcu0[0] + rcu0[1] * rcu0[1] + rcu0[2] * rcu0[2]);
+      const double th = watpol_theta(xO, P.x[o + 1], P.x[o + 2], rcu0, rc);
+      kth[m] = __double_as_longlong(th);
+      atomicAdd(&bin[wpol_bin(th)], 1);
+    }
+    __syncthreads();
+  }
   // exclusive prefix over the bins, two per thread
   {
     const int a = bin[2 * threadIdx.x], b = bin[2 * threadIdx.x + 1];
@@ -3242,6 +3286,18 @@ __device__ __forceinline__ void kin_tally(DevPtrs &P, int s, const double *acc) 
   }
 }
 
+// The step's gradient of atom g.  Early force kernels (P.dlast): it goes to
+// dlast, for the host to read, and d is zeroed for the next step, frozen
+// systems included.
+__device__ __forceinline__ double4 take_grad(const DevPtrs &P, int g) {
+  const double4 d = P.d[g];
+  if (P.dlast) {
+    P.dlast[g] = d;
+    P.d[g] = make_double4(0.0, 0.0, 0.0, 0.0);
+  }
+  return d;
+}
+
 // Leap-frog update (md.f90:4080-4108), one thread per atom of the list of
 // atoms outside 3-constraint molecules: v from the gradient with the
 // Berendsen factor of solute or solvent, x from v.  With SHAKE the reference
@@ -3254,6 +3310,8 @@ __global__ void k_leapfrog(DevPtrs P) {
   const int g = k < P.n_lf ? P.lf_atoms[k] : P.natoms_tot;   // the atoms outside 3-constraint molecules
   int s = -1;
   double acc[4] = {0, 0, 0, 0};
+  double4 d = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (g < P.natoms_tot) d = take_grad(P, g);
   // a system that raised an error stays where the failing step left it;
   // atoms of 3-constraint molecules are k_leapfrog_shake3's
   if (g < P.natoms_tot && P.st[P.asys[g]].frozen == 0 && !(P.flags[g] & F_SH3)) {
@@ -3261,7 +3319,7 @@ __global__ void k_leapfrog(DevPtrs P) {
     const SysDev &S = P.sys[s];
     double ts = (g - S.aoff) < S.nsol ? P.st[s].Tscale_sol : P.st[s].Tscale_solv;
     double w = (double)P.winv[g], dt = S.dt;
-    double4 x = P.x[g], v = P.v[g], d = P.d[g];
+    double4 x = P.x[g], v = P.v[g];
     v.x = (v.x - d.x * w * dt) * ts;
     v.y = (v.y - d.y * w * dt) * ts;
     v.z = (v.z - d.z * w * dt) * ts;
@@ -3319,12 +3377,13 @@ __device__ __forceinline__ bool shake_pair(double3 &xi, double3 &xj, const doubl
 // host so that the constraints, in their own order, join (0,1), (0,2), (1,2);
 // sweeps, readiness flags and the 1000-sweep limit are the reference's.
 // k_leapfrog's update of atom g of system sys: the new velocity and position.
-__device__ __forceinline__ void leapfrog_atom(const DevPtrs &P, int sys, int g, double4 &v, double3 &xn) {
+__device__ __forceinline__ void leapfrog_atom(const DevPtrs &P, int sys, int g, const double4 &d, double4 &v,
+                                              double3 &xn) {
   const SysDev &S = P.sys[sys];
   const double dt = S.dt;
   const double ts = (g - S.aoff) < S.nsol ? P.st[sys].Tscale_sol : P.st[sys].Tscale_solv;
   const double w = (double)P.winv[g];
-  const double4 x = P.x[g], d = P.d[g];
+  const double4 x = P.x[g];
   v = P.v[g];
   v.x = (v.x - d.x * w * dt) * ts;
   v.y = (v.y - d.y * w * dt) * ts;
@@ -3349,9 +3408,9 @@ __global__ void __launch_bounds__(128, 6) k_leapfrog_shake3(DevPtrs P) {
     double3 x0, x1, x2;
     {
       double4 v;
-      leapfrog_atom(P, sys, at.x, v, x0);
-      leapfrog_atom(P, sys, at.y, v, x1);
-      leapfrog_atom(P, sys, at.z, v, x2);
+      leapfrog_atom(P, sys, at.x, take_grad(P, at.x), v, x0);
+      leapfrog_atom(P, sys, at.y, take_grad(P, at.y), v, x1);
+      leapfrog_atom(P, sys, at.z, take_grad(P, at.z), v, x2);
     }
     const double3 r0 = ld3(P.x, at.x), r1 = ld3(P.x, at.y), r2 = ld3(P.x, at.z);
     const float w0 = P.winv[at.x], w1 = P.winv[at.y], w2 = P.winv[at.z];
@@ -3385,7 +3444,7 @@ __global__ void __launch_bounds__(128, 6) k_leapfrog_shake3(DevPtrs P) {
       for (int a = 0; a < 3; a++) {
         double4 v;
         double3 xn;
-        leapfrog_atom(P, sys, ids[a], v, xn);
+        leapfrog_atom(P, sys, ids[a], (P.dlast ? P.dlast : P.d)[ids[a]], v, xn);
         double4 o = P.x[ids[a]];
         o.x = xn.x; o.y = xn.y; o.z = xn.z;
         P.x[ids[a]] = o;
@@ -3393,6 +3452,11 @@ __global__ void __launch_bounds__(128, 6) k_leapfrog_shake3(DevPtrs P) {
       }
       set_status(&P.st[sys], QB_ERR_SHAKE);
     }
+  } else if (m < P.nsh3 && P.dlast) {   // a frozen system
+    const int4 at = P.sh3_at[m];
+    take_grad(P, at.x);
+    take_grad(P, at.y);
+    take_grad(P, at.z);
   }
   shake_tally(P, sys, its);
   kin_tally(P, sys, acc);
