@@ -48,6 +48,14 @@ __device__ __forceinline__ void atomic_add3(double4 *d, int g, double fx, double
 
 __device__ __forceinline__ void set_status(SysState *st, int code) { atomicCAS(&st->status, 0, code); }
 
+// a / b for several a and one b, r = 1 / b: Markstein's correction of a r, which
+// rounds as the quotient does.  One quotient (and its special-case branch) for
+// the reciprocal instead of one each.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+  const double q = a * r;
+  return fma(fma(-q, b, a), r, q);
+}
+
 __device__ __forceinline__ double dev_pi() { return (double)(4.0f * atanf(1.0f)); }
 
 // ------------------------------------------------------------ periodic box
@@ -1148,7 +1156,8 @@ __device__ __forceinline__ double watpol_theta(double4 xO, double4 x1, double4 x
   double rmu[3] = {x1.x + x2.x - 2. * xO.x, x1.y + x2.y - 2. * xO.y, x1.z + x2.z - 2. * xO.z};
   double rm = sqrt(rmu[0] * rmu[0] + rmu[1] * rmu[1] + rmu[2] * rmu[2]);
   double rcu[3];
-  for (int k = 0; k < 3; k++) { rmu[k] /= rm; rcu[k] = rcu0[k] / rc; }
+  const double im = 1. / rm, ic = 1. / rc;
+  for (int k = 0; k < 3; k++) { rmu[k] = div_by(rmu[k], rm, im); rcu[k] = div_by(rcu0[k], rc, ic); }
   double scp = rmu[0] * rcu[0] + rmu[1] * rcu[1] + rmu[2] * rcu[2];
   if (scp > 1.0) scp = 1.0;
   if (scp < -1.0) scp = -1.0;
@@ -3107,9 +3116,12 @@ __global__ void __launch_bounds__(WPOL_BLOCK) k_watpol(DevPtrs P) {
   __shared__ int bin[WPOL_BINS + 1];            // members per bin, then each bin's first place
   __shared__ int wsum[WPOL_BLOCK / 32];
   __shared__ double shsum[32];
-  __shared__ float tcs;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) cnt = 0;
+  // the shell's averages, loaded before they are needed
+  SysState &st = P.st[s];
+  const int istep = st.istep;
+  float avth = st.avtheta[is], avn = st.avn_insh[is], corr = st.theta_corr[is];
   for (int k = threadIdx.x; k <= WPOL_BINS; k += WPOL_BLOCK) bin[k] = 0;
   __syncthreads();
   const int8_t *wsh = P.wshell + S.woff;
@@ -3186,23 +3198,24 @@ __global__ void __launch_bounds__(WPOL_BLOCK) k_watpol(DevPtrs P) {
     tsum += th;
   }
   const double tot = block_sum(tsum, shsum);     // (its barriers also order the placing)
-  if (threadIdx.x == 0) {
-    SysState &st = P.st[s];
-    if (st.istep != 0 && st.istep % 100 == 0) {
-      st.avtheta[is] = st.avtheta[is] / (float)100;
-      st.avn_insh[is] = st.avn_insh[is] / (float)100;
-      st.theta_corr[is] = st.theta_corr[is] + st.avtheta[is] - acosf(S.ws_cstb[is]);
-      st.avtheta[is] = 0.0f;
-      st.avn_insh[is] = 0.0f;
-    }
-    if (n > 0) {
-      st.avtheta[is] = (float)((double)st.avtheta[is] + tot / (double)(float)n);
-      st.avn_insh[is] = st.avn_insh[is] + (float)n;
-    }
-    tcs = st.theta_corr[is];
+  // every thread updates its copy alike; thread 0 stores it
+  if (istep != 0 && istep % 100 == 0) {
+    avth = avth / (float)100;
+    avn = avn / (float)100;
+    corr = corr + avth - acosf(S.ws_cstb[is]);
+    avth = 0.0f;
+    avn = 0.0f;
   }
-  __syncthreads();
-  const float tc = tcs, cstb = S.ws_cstb[is];
+  if (n > 0) {
+    avth = (float)((double)avth + tot / (double)(float)n);
+    avn = avn + (float)n;
+  }
+  if (threadIdx.x == 0) {
+    st.avtheta[is] = avth;
+    st.avn_insh[is] = avn;
+    st.theta_corr[is] = corr;
+  }
+  const float tc = corr, cstb = S.ws_cstb[is];
   const double pi = dev_pi();
   double epol = 0;
   for (int m = threadIdx.x; m < n; m += WPOL_BLOCK) {
@@ -3229,10 +3242,10 @@ __global__ void __launch_bounds__(WPOL_BLOCK) k_watpol(DevPtrs P) {
     double dv = S.fkwpol * dth;
     double rmu[3] = {x1.x + x2.x - 2. * xO.x, x1.y + x2.y - 2. * xO.y, x1.z + x2.z - 2. * xO.z};
     double rm = sqrt(rmu[0] * rmu[0] + rmu[1] * rmu[1] + rmu[2] * rmu[2]);
-    for (int c = 0; c < 3; c++) rmu[c] /= rm;
     double rcu[3] = {xO.x - S.xw[0], xO.y - S.xw[1], xO.z - S.xw[2]};
     double rc = sqrt(rcu[0] * rcu[0] + rcu[1] * rcu[1] + rcu[2] * rcu[2]);
-    for (int c = 0; c < 3; c++) rcu[c] /= rc;
+    const double im = 1. / rm, ic = 1. / rc;
+    for (int c = 0; c < 3; c++) { rmu[c] = div_by(rmu[c], rm, im); rcu[c] = div_by(rcu[c], rc, ic); }
     double scp = rmu[0] * rcu[0] + rmu[1] * rcu[1] + rmu[2] * rcu[2];
     if (scp > 1.0) scp = 1.0;
     if (scp < -1.0) scp = -1.0;
@@ -3242,8 +3255,8 @@ __global__ void __launch_bounds__(WPOL_BLOCK) k_watpol(DevPtrs P) {
     f0 = dv * f0;
     double gO[3], gH[3];
     for (int c = 0; c < 3; c++) {
-      double f1 = (rcu[c] - rmu[c] * scp) / rm;
-      double f2 = (rmu[c] - rcu[c] * scp) / rc;
+      double f1 = div_by(rcu[c] - rmu[c] * scp, rm, im);
+      double f2 = div_by(rmu[c] - rcu[c] * scp, rc, ic);
       gO[c] = f0 * (-2. * f1 + f2);
       gH[c] = f0 * f1;
     }
@@ -3273,14 +3286,23 @@ __device__ __forceinline__ void kin_add(const DevPtrs &P, const SysDev &S, int g
 __device__ __forceinline__ void kin_tally(DevPtrs &P, int s, const double *acc) {
   const int lane = threadIdx.x & 31;
   unsigned todo = __ballot_sync(FULL, s >= 0);
+  // solute or solvent sums that no lane of the warp has are skipped
+  const bool any[2] = {__any_sync(FULL, acc[0] != 0.0) != 0, __any_sync(FULL, acc[2] != 0.0) != 0};
   while (todo) {
     const int leader = __ffs(todo) - 1;
     const int s0 = __shfl_sync(FULL, s, leader);
     const bool mine = s == s0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      double v = warp_sum(mine ? acc[k] : 0.0);
-      if (lane == leader && v != 0.0) atomicAdd(&P.kin[s0 * 4 + k], v);
+    for (int h = 0; h < 2; h++) {
+      if (!any[h]) continue;
+      double v = mine ? acc[2 * h] : 0.0, w = mine ? acc[2 * h + 1] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        v += __shfl_xor_sync(FULL, v, o);
+        w += __shfl_xor_sync(FULL, w, o);
+      }
+      if (lane == leader && v != 0.0) atomicAdd(&P.kin[s0 * 4 + 2 * h], v);
+      if (lane == leader && w != 0.0) atomicAdd(&P.kin[s0 * 4 + 2 * h + 1], w);
     }
     todo &= ~__ballot_sync(FULL, mine);
   }
@@ -3425,7 +3447,7 @@ __global__ void __launch_bounds__(128, 6) k_leapfrog_shake3(DevPtrs P) {
     }
     if (c0 && c1 && c2) {
       const SysDev &S = P.sys[sys];
-      const double dt = S.dt;
+      const double dt = S.dt, idt = 1. / dt;
       double3 xs[3] = {x0, x1, x2}, rs[3] = {r0, r1, r2};
 #pragma unroll
       for (int a = 0; a < 3; a++) {
@@ -3433,9 +3455,9 @@ __global__ void __launch_bounds__(128, 6) k_leapfrog_shake3(DevPtrs P) {
         o.x = xs[a].x; o.y = xs[a].y; o.z = xs[a].z;
         P.x[ids[a]] = o;
         double4 v = P.v[ids[a]];
-        v.x = (xs[a].x - rs[a].x) / dt;
-        v.y = (xs[a].y - rs[a].y) / dt;
-        v.z = (xs[a].z - rs[a].z) / dt;
+        v.x = div_by(xs[a].x - rs[a].x, dt, idt);
+        v.y = div_by(xs[a].y - rs[a].y, dt, idt);
+        v.z = div_by(xs[a].z - rs[a].z, dt, idt);
         P.v[ids[a]] = v;
         kin_add(P, S, ids[a], v, acc);
       }
@@ -3587,7 +3609,7 @@ __global__ void __launch_bounds__(KIN_BLOCK) k_kinetic(DevPtrs P) {
 // (P.E, P.EQ) are read and zeroed for the next evaluation here, the results
 // kept in P.Eo, P.EQo: two memset nodes less at the head of every step (they
 // were 2 to 3 us of a single system's 63).
-__device__ __forceinline__ void finalize_energy(DevPtrs &P, int s) {
+__device__ __forceinline__ void finalize_energy(DevPtrs &P, int s, double kinetic) {
   const SysDev &S = P.sys[s];
   const int lane = threadIdx.x;
   static_assert(QB_NE <= 32, "a lane per term");
@@ -3600,9 +3622,10 @@ __device__ __forceinline__ void finalize_energy(DevPtrs &P, int s) {
   // the states' rows through shared memory: whole-warp loads and stores
   __shared__ double row[MAXS * QB_NEQ];
   double *q = P.EQ + (size_t)s * MAXS * QB_NEQ, *qo = P.EQo + (size_t)s * MAXS * QB_NEQ;
+  const double q0 = q[lane];             // loaded before the state count is known
   const int nq = S.S * QB_NEQ;
   for (int k = lane; k < nq; k += 32) {
-    row[k] = q[k];
+    row[k] = k < 32 ? q0 : q[k];
     q[k] = 0.0;
   }
   __syncwarp();
@@ -3638,7 +3661,7 @@ __device__ __forceinline__ void finalize_energy(DevPtrs &P, int s) {
                      term(QB_E_QX_VDW) + rst + term(QB_E_LRF);
   if (lane == QB_E_RST_TOTAL) e = rst;
   if (lane == QB_E_POTENTIAL) e = pot;
-  if (lane == QB_E_KINETIC) e = P.st[s].kinetic;
+  if (lane == QB_E_KINETIC) e = kinetic;
   if (lane < QB_NE) P.Eo[s * QB_NE + lane] = e;
   if (lane == 0 && !isfinite(pot)) set_status(&P.st[s], QB_ERR_NAN);
   __syncwarp();
@@ -3655,7 +3678,12 @@ __global__ void k_finish(DevPtrs P, int mode) {
   const SysDev &S = P.sys[s];
   SysState &st = P.st[s];
   int lane = threadIdx.x;
-  if (mode != 0) finalize_energy(P, s);
+  // what the step end reads, loaded together: the kernel is a chain of loads
+  const double kinetic = st.kinetic;
+  const int is0 = st.istep, iout = S.iout, iene = S.iene;
+  double tot[4];
+  for (int k = 0; k < 4; k++) tot[k] = P.kin[s * 4 + k];
+  if (mode != 0) finalize_energy(P, s, kinetic);
   if (mode == 2) return;
   if (mode == 1 && st.status != 0) {
     // failed at this step: no records, the step count stays at the failure,
@@ -3665,8 +3693,7 @@ __global__ void k_finish(DevPtrs P, int mode) {
     return;
   }
   if (lane == 0) {
-    double tot[4];
-    for (int k = 0; k < 4; k++) { tot[k] = P.kin[s * 4 + k]; P.kin[s * 4 + k] = 0.0; }
+    for (int k = 0; k < 4; k++) P.kin[s * 4 + k] = 0.0;
     const double kb = (double)kBoltzF;
     double Tfree_sol = tot[1], Tfree_solv = tot[3];
     double Tfree = Tfree_solv + Tfree_sol;
@@ -3698,10 +3725,10 @@ __global__ void k_finish(DevPtrs P, int mode) {
   __syncwarp();
   if (mode == 1) {
     // output and energy-file records of this step, copied by the whole warp
-    const int is = st.istep;
+    const int is = is0;
     const int rec_len = HIST_REC;
     for (int kind = 0; kind < 2; kind++) {
-      int cyc = kind == 0 ? S.iout : S.iene;
+      int cyc = kind == 0 ? iout : iene;
       bool want = (is % cyc == 0) && (kind == 0 || is > 0);
       if (!want) continue;
       int c = st.hist_n[kind];
