@@ -1,10 +1,15 @@
 """Kernels whose launch shape follows the batch: the same system gives the
 same forces and energies whatever shares the batch with it, and the shapes'
 edges (few and many members, partial groups) match the oracle."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from q_b200 import FP64, MIXED, Batch, System, synth
+from q_b200 import FP64, MIXED, Batch, System, mlp, synth
+from q_b200._lib import check, lib
+from q_b200.api import Tuning
+from oracle import mlp_oracle as M
 from tests.oracle_binding import load_oracle
 
 pytestmark = pytest.mark.gpu
@@ -48,3 +53,132 @@ def test_polarisation_shells_match_oracle(tmp_path, radius):
     assert np.abs(b.energy_vectors(0)[0] - o.energy_vectors()[0]).max() < 1e-3
     go = o.gradient()
     assert np.abs(b.gradient(0) - go).max() < 1e-4 * np.abs(go).max()
+
+
+def _both(systems, precision):
+    """The batch with its default shapes, and with other staging blocks and one
+    block per LRF tile.  The LRF's FP32 partial sums follow its tiles, so the
+    mixed batches both have one tile per block."""
+    a, b = Batch(systems, precision=precision), Batch(systems, precision=precision)
+    t = Tuning()
+    check(lib.qb_batch_get_tuning(b._b, C.addressof(t)))
+    b.set_tuning(ww_waters_per_block=128 if t.ww_waters_per_block == 256 else 256, lrf_tiles_per_block=1)
+    if precision == MIXED:
+        a.set_tuning(lrf_tiles_per_block=1)
+    return a, b
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+@pytest.mark.parametrize("kind", ["sphere5", "sphere15", "fep20", "box30"])
+def test_small_batch_water_kernels(tmp_path, precision, kind):
+    """A small batch (water-water without staging, every force from the head of
+    the step, in FP64 LRF tiles shared by blocks) against the staged kernels
+    and whole tiles for the same system: single points of both kinds.  FP64
+    sums of up to ~1e3 terms in another order: 1e3 x 2^-53 = 1e-13 of the
+    largest, bar 1e-11.  The mixed engine's FP32 sums are the same in both."""
+    if kind == "fep20":
+        g, lam = synth.fep_solute(str(tmp_path), radius=20.0, seed=5), (0.3, 0.7)
+    elif kind == "box30":
+        g, lam = synth.fep_box(str(tmp_path), edge=30.0, seed=5), (0.3, 0.7)
+    else:
+        g, lam = synth.water_sphere(str(tmp_path), radius=float(kind[6:]), seed=5), None
+    s = System.open(g.inp, lambdas=lam, seed=3)
+    a, b = _both([s], precision)
+    for energies in (True, False):
+        a.evaluate(energies)
+        b.evaluate(energies)
+        ga, gb = a.gradient(0), b.gradient(0)
+        assert np.abs(ga - gb).max() <= 1e-11 * np.abs(gb).max(), energies
+        ea, eb = a.energy_vectors(0)[0], b.energy_vectors(0)[0]
+        assert np.abs(ea - eb).max() <= 1e-11 * np.abs(eb).max(), energies
+    # After steps the gradient is the last step's, and an evaluation after them
+    # starts from a clean one.  Three steps amplify the FP64 order of sums by far
+    # less than 1e4; mixed, a position next to a rounding boundary may move one
+    # FP32 offset by 6e-8 A, about 1e-6 of the largest force.
+    bar = 1e-7 if precision == FP64 else 1e-5
+    for _ in range(2):
+        a.run(3)
+        b.run(3)
+        assert np.abs(a.gradient(0) - b.gradient(0)).max() <= bar * np.abs(gb).max()
+        a.evaluate(True)
+        b.evaluate(True)
+        assert np.abs(a.gradient(0) - b.gradient(0)).max() <= bar * np.abs(gb).max()
+
+
+@pytest.mark.parametrize("nwat", [1, 3, 4, 5, 127, 129, 1000])
+def test_static_water_blocks(nwat):
+    """qb_ww_energy_static at the edges of its blocks (4 waters) and scan rounds
+    (128 candidates) against a dense FP64 evaluation; sums of up to ~1e3 terms
+    and single-precision charge products on both sides: 1e-9 relative."""
+    import torch
+    rng = np.random.default_rng(nwat)
+    side = int(np.ceil(nwat ** (1 / 3)))
+    o = 3.1 * np.array([(i, j, k) for i in range(side) for j in range(side) for k in range(side)], float)[:nwat]
+    h = rng.normal(size=(nwat, 2, 3))
+    h *= 0.96 / np.linalg.norm(h, axis=2, keepdims=True)
+    x = np.concatenate([o[:, None], o[:, None] + h], axis=1)
+    excl = np.zeros(nwat, np.uint8)
+    if nwat > 4:
+        excl[nwat // 2] = 1
+    qo, qh, A, B, rc = np.float32(-15.2), np.float32(7.6), 5.8e5, 595.0, 7.0
+    xd, ed = torch.from_numpy(x).cuda(), torch.from_numpy(excl).cuda()
+    grad = torch.full((9 * nwat,), 7.0, dtype=torch.float64, device="cuda")
+    energy = torch.full((2,), 7.0, dtype=torch.float64, device="cuda")
+    status = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+    check(lib.qb_ww_energy_static(xd.data_ptr(), nwat, float(qo), float(qh), A, B, rc, ed.data_ptr(), grad.data_ptr(),
+                                  energy.data_ptr(), status.data_ptr(), C.c_void_p(0)))
+    torch.cuda.synchronize()
+    q = np.array([qo, qh, qh], np.float32)
+    qq = (q[:, None] * q[None]).astype(np.float64)
+    g, el, vdw = np.zeros((nwat, 3, 3)), 0.0, 0.0
+    for i in range(nwat):
+        for j in range(i + 1, nwat):
+            if excl[i] or excl[j] or ((o[i] - o[j]) ** 2).sum() > rc * rc:
+                continue
+            d = x[j][None] - x[i][:, None]
+            r = np.sqrt((d ** 2).sum(-1))
+            dv = -qq / r ** 3
+            r6 = r[0, 0] ** -6
+            dv[0, 0] += (-12 * A * r6 * r6 + 6 * B * r6) / r[0, 0] ** 2
+            f = dv[..., None] * d
+            g[i] -= f.sum(1)
+            g[j] += f.sum(0)
+            el += (qq / r).sum()
+            vdw += A * r6 * r6 - B * r6
+    assert int(status.item()) == 0
+    scale = max(np.abs(g).max(), 1.0)
+    assert np.abs(grad.cpu().numpy() - g.reshape(-1)).max() <= 1e-9 * scale
+    assert abs(energy[0].item() - el) <= 1e-9 * max(1.0, abs(el))
+    assert abs(energy[1].item() - vdw) <= 1e-9 * max(1.0, abs(vdw))
+
+
+@pytest.mark.parametrize("n", [127, 129, 385])
+def test_network_tiles(n):
+    """The network's kernels one sample short of, past and three tiles past a
+    tile of 128, against the oracle that rounds to BF16 as they do; bars as for
+    the other sizes (2e-3 of the largest output, 1e-2 of each gradient's norm)."""
+    rng = np.random.default_rng(n)
+    p = mlp.init(6)
+    x = rng.normal(size=(n, M.IN)).astype(np.float32)
+    t = M.forward(M.init(9), x)[0].astype(np.float32)
+    t += rng.normal(0, 0.3, t.shape).astype(np.float32)
+    yb = M.forward(p, x, bf=True)[0]
+    assert np.abs(mlp.forward(p, x) - yb).max() <= 2e-3 * np.abs(yb).max()
+    loss, g = mlp.loss_grad(p, x, t)
+    lb, gb = M.loss_grad(p, x, t, bf=True)
+    assert abs(loss - lb) <= 1e-3 * lb
+    for (k, _), a, b in zip(M.SHAPES, M.unpack(g).values(), M.unpack(gb).values()):
+        assert np.linalg.norm(a - b) <= 1e-2 * np.linalg.norm(b), k
+
+
+@pytest.mark.parametrize("n,nskip", [(2, 1), (33, 0), (260, 3), (1300, 0)])
+def test_analysis_block_edges(n, nskip):
+    """The analysis' per-file kernel with one record left, a record past a warp
+    and past a block, and several per thread, files of uneven length: against
+    the restatement, with the bars of the other analyses."""
+    from oracle.qfep_oracle import FepInput, analyze as oracle_analyze
+    from q_b200.fep import analyze, params
+    from tests.test_gpu_fep import compare, random_series
+    S = random_series(3, n, 2, seed=n)
+    kw = dict(nbins=5, nmin=1, coeff=[1.0, -1.0])
+    compare(analyze(S, params(0.592, nskip, **kw)), oracle_analyze(FepInput(S, 0.592, nskip, **kw)), 3)
