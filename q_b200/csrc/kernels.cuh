@@ -28,6 +28,56 @@ __device__ __forceinline__ float warp_sumf(float v) {
   return v;
 }
 
+// Sums of several values over a warp (or half of one) at once: at each level of
+// the tree a lane keeps half of its values and hands its partner the other
+// half, so nine values take 11 exchanges over 16 lanes (12 over 32) instead of 36
+// (45), three over 32 lanes 6 instead of 15.  Each sum is the same tree of
+// pairs as warp_sum's, bit for bit.  50 steps of the
+// 15 A sphere 1.348 to 1.330 ms, one FEP window 1.830 to 1.805, 41 FP64 windows 11.12 to
+// 10.94.
+template <class T>
+__device__ __forceinline__ T fold_step(T lo, T hi, bool up, int o, unsigned m) {
+  const T keep = up ? hi : lo, send = up ? lo : hi;
+  return keep + __shfl_xor_sync(m, send, o);
+}
+
+// Nine values over W = 16 or 32 lanes; the sum of component c ends in the lane
+// l (of W) with fold9_component<W>(l) == c, one lane each.
+template <int W, class T>
+__device__ __forceinline__ T fold9(const T *v, int l, unsigned m) {
+  const bool b0 = l & (W / 2), b1 = l & (W / 4), b2 = l & (W / 8), b3 = l & (W / 16);
+  T a[5];
+#pragma unroll
+  for (int q = 0; q < 4; q++) a[q] = fold_step(v[q], v[5 + q], b0, W / 2, m);
+  a[4] = v[4] + __shfl_xor_sync(m, v[4], W / 2);
+  const T c0 = fold_step(a[0], a[3], b1, W / 4, m), c1 = fold_step(a[1], a[4], b1, W / 4, m);
+  const T c2 = a[2] + __shfl_xor_sync(m, a[2], W / 4);
+  const T d0 = fold_step(c0, c2, b2, W / 8, m), d1 = c1 + __shfl_xor_sync(m, c1, W / 8);
+  T r = fold_step(d0, d1, b3, W / 16, m);
+  if (W == 32) r += __shfl_xor_sync(m, r, 1);
+  return r;
+}
+
+template <int W>
+__device__ __forceinline__ int fold9_component(int l) {
+  if (W == 32 && (l & 1)) return 15;
+  return (int)((0xfff8f765ff43f210ull >> (4 * (W == 32 ? l >> 1 : l))) & 15);
+}
+
+// Three values over the warp: component 0 in lane 0, 1 in lane 16, 2 in lane 8
+// (fold3_component: 3 in the other lanes).
+template <class T>
+__device__ __forceinline__ T fold3(const T *v, int l) {
+  const bool b0 = l & 16, b1 = l & 8;
+  const T a0 = fold_step(v[0], v[1], b0, 16, FULL), a1 = v[2] + __shfl_xor_sync(FULL, v[2], 16);
+  T r = fold_step(a0, a1, b1, 8, FULL);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(FULL, r, o);
+  return r;
+}
+
+__device__ __forceinline__ int fold3_component(int l) { return l == 0 ? 0 : l == 16 ? 1 : l == 8 ? 2 : 3; }
+
 // Reduce v over the warp and add it to *dst once (lane 0).  All 32 lanes of
 // the warp must call it.
 __device__ __forceinline__ void warp_add(double *dst, double v) {
@@ -1334,7 +1384,7 @@ __global__ void __launch_bounds__(WW_BLOCK, MIXED ? 2 : 1) k_nb_ww(DevPtrs P, in
       const uint16_t *nb = P.ww + (size_t)gw * P.ww_cap;
       const float4 *ri = (iw >= c0 && iw < c0 + cn) ? wsm + (iw - c0) * W : rec + (size_t)iw * W;
       const int oi = S.aoff + S.nsol + 3 * iw;
-      double fd[9];
+      double g = 0.0;                       // the lane's component of the water's gradient
       int k = kb + hl;
       if (MIXED) {
         float xi[12];
@@ -1368,19 +1418,14 @@ __global__ void __launch_bounds__(WW_BLOCK, MIXED ? 2 : 1) k_nb_ww(DevPtrs P, in
         }
         el += (double)e_el;
         vdw += (double)e_vdw;
-#pragma unroll
-        for (int q = 0; q < 9; q++) {
-          float t = f[q];
-#pragma unroll
-          for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(hmask, t, o);
-          fd[q] = (double)t;
-        }
+        g = (double)fold9<16>(f, hl, hmask);
       } else {
         const double2 *rd = reinterpret_cast<const double2 *>(ri);
         double2 d0 = rd[0], d1 = rd[1], d2 = rd[2], d3 = rd[3], d4 = rd[4];
         const double xi[9] = {d0.x, d0.y, d1.x, d1.y, d2.x, d2.y, d3.x, d3.y, d4.x};
         const double qoo = (double)(qo * qo), qoh = (double)(qo * qh), qhh = (double)(qh * qh);
         const double ljd[6] = {S.A_OO, S.B_OO, S.A_OH, S.B_OH, S.A_HH, S.B_HH};
+        double fd[9];
 #pragma unroll
         for (int q = 0; q < 9; q++) fd[q] = 0.0;
         for (; k < ke; k += 16) {
@@ -1396,19 +1441,11 @@ __global__ void __launch_bounds__(WW_BLOCK, MIXED ? 2 : 1) k_nb_ww(DevPtrs P, in
           }
           ww_pair_f64<HLJ>(xi, xj, qoo, qoh, qhh, ljd, fd, el, vdw);
         }
-        if (!EONCE) {
-#pragma unroll
-          for (int q = 0; q < 9; q++) {
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) fd[q] += __shfl_xor_sync(hmask, fd[q], o);
-          }
-        }
+        if (!EONCE) g = fold9<16>(fd, hl, hmask);
       }
       // fire-and-forget adds: the half-warp does not wait for the gradient
-      if (!EONCE && hl == 0) {
-#pragma unroll
-        for (int a = 0; a < 3; a++) atomic_add3(P.d, oi + a, fd[3 * a], fd[3 * a + 1], fd[3 * a + 2]);
-      }
+      const int gc = fold9_component<16>(hl);
+      if (!EONCE && gc < 9) atomicAdd(&P.d[oi + gc / 3].x + gc % 3, g);
     }
   }
   warp_add(&P.E[s * QB_NE + QB_E_WW_EL], EONCE ? el : 0.5 * el);
@@ -1513,15 +1550,9 @@ __device__ __forceinline__ void ww_store_i(const DevPtrs &P, int o, int hl, unsi
     g[3 + q] = gH[q].x + gHs[q].y;
     g[6 + q] = gH[q].y + gHs[q].x;
   }
-#pragma unroll
-  for (int q = 0; q < 9; q++) {
-#pragma unroll
-    for (int u = 8; u > 0; u >>= 1) g[q] += __shfl_xor_sync(hmask, g[q], u);
-  }
-  float f = g[0];
-#pragma unroll
-  for (int q = 1; q < 9; q++) f = hl == q ? g[q] : f;
-  if (hl < 9) atomicAdd(&P.d[o + hl / 3].x + hl % 3, (double)f);
+  const float f = fold9<16>(g, hl, hmask);
+  const int c = fold9_component<16>(hl);
+  if (c < 9) atomicAdd(&P.d[o + c / 3].x + c % 3, (double)f);
 }
 
 // nonbond_ww_spc (md.f90:11823) forces of the mixed-precision engine on steps
@@ -1672,13 +1703,9 @@ __global__ void __launch_bounds__(32 * WWD_WATERS, 2) k_nb_ww_direct(DevPtrs P) 
       ww_pair_f64<HLJ>(xi, xj, qoo, qoh, qhh, ljd, fd, el, vdw);
     }
     if (!EONCE) {
-      double f = 0.0;
-#pragma unroll
-      for (int q = 0; q < 9; q++) {
-        const double t = warp_sum(fd[q]);
-        if (lane == q) f = t;
-      }
-      if (lane < 9 && ke > 0) atomicAdd(&P.d[S.aoff + S.nsol + 3 * iw + lane / 3].x + lane % 3, f);
+      const double f = fold9<32>(fd, lane, FULL);
+      const int c = fold9_component<32>(lane);
+      if (c < 9 && ke > 0) atomicAdd(&P.d[S.aoff + S.nsol + 3 * iw + c / 3].x + c % 3, f);
     }
     el = warp_sum(el);
     vdw = warp_sum(vdw);
@@ -1791,9 +1818,9 @@ __device__ __forceinline__ void nb_pp_body(DevPtrs &P, int bx, int s, int gx) {
       el += Vel;
       vdw += Va - Vb;
     }
-#pragma unroll
-    for (int c = 0; c < 3; c++) gi[c] = warp_sum(gi[c]);
-    if (lane == 0) atomic_add3(P.d, i, gi[0], gi[1], gi[2]);
+    const double g = fold3(gi, lane);
+    const int c = fold3_component(lane);
+    if (c < 3) atomicAdd(&P.d[i].x + c, g);
   }
   warp_add(&P.E[s * QB_NE + QB_E_PP_EL], 0.5 * el);
   warp_add(&P.E[s * QB_NE + QB_E_PP_VDW], 0.5 * vdw);
@@ -1839,11 +1866,13 @@ __global__ void __launch_bounds__(PW_BLOCK) k_nb_pw(DevPtrs P) {
   // the group's atoms, parameters and positions staged once per block
   __shared__ PwAtom sa[PW_MAXA];
   __shared__ double4 sx[PW_MAXA];
+  __shared__ float4 sl[F32 ? PW_MAXA : 1];     // the LJ products in FP32: converted once a block, not once a water
   const int ta = P.pwg_off[sg], na = min(P.pwg_off[sg + 1] - ta, PW_MAXA);
   if (threadIdx.x < na) {
     const PwAtom A = P.pwa[ta + threadIdx.x];
     sa[threadIdx.x] = A;
     sx[threadIdx.x] = P.x[A.atom];
+    if (F32) sl[F32 ? threadIdx.x : 0] = make_float4((float)A.lj.x, (float)A.lj.y, (float)A.lj.z, (float)A.lj.w);
   }
   __syncthreads();
   double fw[9];
@@ -1851,7 +1880,7 @@ __global__ void __launch_bounds__(PW_BLOCK) k_nb_pw(DevPtrs P) {
 #pragma unroll
   for (int c = 0; c < 9; c++) { fw[c] = 0.0; fw32[c] = 0.f; }
   double el = 0, vdw = 0;
-  const int t1 = P.pwg_off[sg + 1];
+  const int t1 = P.pwg_off[sg + 1], comp = fold3_component(lane);
   for (int t = ta; t < t1; t++) {
     const PwAtom A = t - ta < PW_MAXA ? sa[t - ta] : P.pwa[t];
     const double4 x4 = t - ta < PW_MAXA ? sx[t - ta] : P.x[A.atom];
@@ -1860,6 +1889,8 @@ __global__ void __launch_bounds__(PW_BLOCK) k_nb_pw(DevPtrs P) {
     if (F32) {
       // forces alone: the group atom's FP32 terms summed over the warp in FP32
       float gi[3] = {0.f, 0.f, 0.f};
+      const float4 lj = t - ta < PW_MAXA ? sl[F32 ? t - ta : 0]
+                                         : make_float4((float)A.lj.x, (float)A.lj.y, (float)A.lj.z, (float)A.lj.w);
 #pragma unroll
       for (int b = 0; b < 3; b++) {
         if (!act) break;
@@ -1867,15 +1898,14 @@ __global__ void __launch_bounds__(PW_BLOCK) k_nb_pw(DevPtrs P) {
         const float r = rsqrt_ftz(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
         const float r2 = r * r, r6 = r2 * r2 * r2;
         const float Vel = (b == 0 ? A.q.x : A.q.y) * r;
-        const float Va = (float)(b == 0 ? A.lj.x : A.lj.z) * r6 * r6, Vb = (float)(b == 0 ? A.lj.y : A.lj.w) * r6;
+        const float Va = (b == 0 ? lj.x : lj.z) * r6 * r6, Vb = (b == 0 ? lj.y : lj.w) * r6;
         const float dv = r2 * (-Vel - 12.f * Va + 6.f * Vb);
         gi[0] = fmaf(-dv, dx, gi[0]); gi[1] = fmaf(-dv, dy, gi[1]); gi[2] = fmaf(-dv, dz, gi[2]);
         fw32[3 * b] = fmaf(dv, dx, fw32[3 * b]); fw32[3 * b + 1] = fmaf(dv, dy, fw32[3 * b + 1]);
         fw32[3 * b + 2] = fmaf(dv, dz, fw32[3 * b + 2]);
       }
-#pragma unroll
-      for (int c = 0; c < 3; c++) gi[c] = warp_sumf(gi[c]);
-      if (lane == 0) atomic_add3(P.d, A.atom, (double)gi[0], (double)gi[1], (double)gi[2]);
+      const float g = fold3(gi, lane);
+      if (comp < 3) atomicAdd(&P.d[A.atom].x + comp, (double)g);
       continue;
     }
     if (act) {
@@ -1893,9 +1923,8 @@ __global__ void __launch_bounds__(PW_BLOCK) k_nb_pw(DevPtrs P) {
         vdw += Va - Vb;
       }
     }
-#pragma unroll
-    for (int c = 0; c < 3; c++) fi[c] = warp_sum(fi[c]);
-    if (lane == 0) atomic_add3(P.d, A.atom, fi[0], fi[1], fi[2]);
+    const double g = fold3(fi, lane);
+    if (comp < 3) atomicAdd(&P.d[A.atom].x + comp, g);
   }
   if (F32)
 #pragma unroll
@@ -1993,10 +2022,11 @@ __device__ __forceinline__ void nb_qp_body(DevPtrs &P, int bx, int s, int gx) {
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         fj[c] += f[c];
-        t[c] = warp_sum(-f[c]);
+        t[c] = -f[c];
       }
-      const double g = lane == 0 ? t[0] : lane == 1 ? t[1] : t[2];
-      if (lane < 3 && g != 0.0) atomicAdd(&P.d[i].x + lane, g);
+      const double g = fold3(t, lane);
+      const int c = fold3_component(lane);
+      if (c < 3 && g != 0.0) atomicAdd(&P.d[i].x + c, g);
     }
     __syncthreads();
 #pragma unroll
@@ -2062,7 +2092,10 @@ __global__ void __launch_bounds__(32 * QW_MAXWARPS, NSC > 0 ? 2 : 1) k_nb_qw(Dev
   if (tile.y >= n) return;
   __shared__ QwAtom sqa[QW_CHUNK];
   __shared__ double4 sqx[QW_CHUNK];
-  __shared__ QwState sqs[QW_CHUNK * NA];
+  __shared__ QwState sqs[F32 ? 1 : QW_CHUNK * NA];
+  // F32: the parameters rounded once a block, not once a water
+  __shared__ float2 sqa32[F32 ? QW_CHUNK : 1], sqe32[F32 ? QW_CHUNK * NA : 1];
+  __shared__ float4 sqs32[F32 ? QW_CHUNK * NA : 1];
   // F32: force factors [Q atom][site][warp's group of waters]; FP64: each warp's gradients
   __shared__ R red[F32 ? QW_CHUNK * 3 * (QW_MAXWARPS / 2) * 32 : QW_MAXWARPS * 9 * 32];
   __shared__ double ered[QW_MAXWARPS * 2 * NA];
@@ -2094,14 +2127,23 @@ __global__ void __launch_bounds__(32 * QW_MAXWARPS, NSC > 0 ? 2 : 1) k_nb_qw(Dev
       const QwAtom A = P.qwa[S.qoff + q0 + t];
       sqa[t] = A;
       sqx[t] = P.x[A.atom];
+      if (F32) sqa32[F32 ? t : 0] = make_float2((float)A.A, (float)A.B);
     }
-    for (int t = threadIdx.x; t < qn * NS; t += blockDim.x)
-      sqs[t / NS * NA + t % NS] = P.qws[(size_t)(S.qoff + q0 + t / NS) * MAXS + t % NS];
+    for (int t = threadIdx.x; t < qn * NS; t += blockDim.x) {
+      const int st = t % NS, to = t / NS * NA + st;
+      const QwState &q = P.qws[(size_t)(S.qoff + q0 + t / NS) * MAXS + st];
+      if (F32) {
+        sqs32[F32 ? to : 0] = make_float4(q.qO, q.qH, (float)q.A, (float)q.B);
+        sqe32[F32 ? to : 0] = make_float2((float)q.sc, (float)S.lambda[st]);
+      } else {
+        sqs[F32 ? 0 : to] = q;
+      }
+    }
     __syncthreads();
     for (int iq = sub; iq < qn; iq += qg) {
       const QwAtom &QA = sqa[iq];
       const double4 xi = sqx[iq];
-      const QwState *qst = sqs + iq * NA;
+      const QwState *qst = sqs + (F32 ? 0 : iq * NA);
       R qacc[3];
       if (F32) {
         // differences of the FP64 positions rounded to FP32, MUFU reciprocal
@@ -2118,25 +2160,26 @@ __global__ void __launch_bounds__(32 * QW_MAXWARPS, NSC > 0 ? 2 : 1) k_nb_qw(Dev
         float Va0 = 0.f, Vb0 = 0.f;
         if (!S.qvdw) {
           const float r6 = r2Oi * r2Oi * r2Oi;
-          Va0 = (float)QA.A * r6 * r6;
-          Vb0 = (float)QA.B * r6;
+          Va0 = sqa32[F32 ? iq : 0].x * r6 * r6;
+          Vb0 = sqa32[F32 ? iq : 0].y * r6;
         }
         float dvO = 0.f, dvH1 = 0.f, dvH2 = 0.f;
 #pragma unroll
         for (int st = 0; st < NA; st++) {
           if (st >= NS) break;
-          const QwState &q = qst[st];
+          const float4 q = sqs32[F32 ? iq * NA + st : 0];       // {qO, qH, A, B}
+          const float2 e = sqe32[F32 ? iq * NA + st : 0];       // {soft-core shift, lambda}
           float Va = Va0, Vb = Vb0, fsc = 1.f;
           if (S.qvdw) {
-            const float inv = 1.f / (r6hc + (float)q.sc);
-            Va = (float)q.A * inv * inv;
-            Vb = (float)q.B * inv;
+            const float inv = 1.f / (r6hc + e.x);
+            Va = q.z * inv * inv;
+            Vb = q.w * inv;
             fsc = r6hc * inv;
           }
-          const float lam = (float)S.lambda[st];
-          dvO += r2Oi * (-q.qO * rO - (12.f * Va - 6.f * Vb) * fsc) * lam;
-          dvH1 -= r2H1 * (q.qH * rH1) * lam;
-          dvH2 -= r2H2 * (q.qH * rH2) * lam;
+          const float lam = e.y;
+          dvO += r2Oi * (-q.x * rO - (12.f * Va - 6.f * Vb) * fsc) * lam;
+          dvH1 -= r2H1 * (q.y * rH1) * lam;
+          dvH2 -= r2H2 * (q.y * rH2) * lam;
         }
         if (qg > 1) {
           R *f = red + ((size_t)iq * 3 * ng + grp) * 32 + lane;
@@ -2152,7 +2195,6 @@ __global__ void __launch_bounds__(32 * QW_MAXWARPS, NSC > 0 ? 2 : 1) k_nb_qw(Dev
             fw[3 + c] = fmaf(dvH1, h1[c], (float)fw[3 + c]);
             fw[6 + c] = fmaf(dvH2, h2[c], (float)fw[6 + c]);
           }
-          qacc[c] = warp_sumf((float)qacc[c]);
         }
       } else {
         double dO[3] = {xO.x - xi.x, xO.y - xi.y, xO.z - xi.z};
@@ -2222,12 +2264,12 @@ __global__ void __launch_bounds__(32 * QW_MAXWARPS, NSC > 0 ? 2 : 1) k_nb_qw(Dev
           fw[c] += dvO * dO[c];
           fw[3 + c] += dvH1 * dH1[c];
           fw[6 + c] += dvH2 * dH2[c];
-          qacc[c] = warp_sum(qacc[c]);
         }
       }
-      // the Q atom's gradient from this warp's waters: lane c adds component c
-      const double t = lane == 0 ? (double)qacc[0] : lane == 1 ? (double)qacc[1] : (double)qacc[2];
-      if (lane < 3 && t != 0.0) atomicAdd(&P.d[QA.atom].x + lane, t);
+      // the Q atom's gradient from this warp's waters
+      const R t = fold3(qacc, lane);
+      const int c = fold3_component(lane);
+      if (c < 3 && t != 0) atomicAdd(&P.d[QA.atom].x + c, (double)t);
     }
     if (F32 && qg > 1) {
       // component c of the group's waters by warp c % qg, Q atoms in order

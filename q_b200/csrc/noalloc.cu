@@ -52,11 +52,11 @@ __device__ __forceinline__ double wsum(double v) {
 // whose O lies within the cut-off) compacted into shared memory, then lanes
 // over them, the water's 9 gradient components reduced with warp shuffles;
 // every pair is seen from both waters, so each side adds half of the pair
-// energy.  The last block to finish adds the blocks' energies in order.
-// One launch: a small sphere is bound by launches and by the chain of one
-// warp (list scan, then about three rounds of pairs), so the list in memory,
-// the zeroing memsets and a quotient and a root per atom pair go.  480 waters: 23.5 to 14.3 us a
-// call.
+// energy.  k_static_ww_sum adds the blocks' energies in order.  Two launches
+// in all: a small sphere is bound by launches and by the chain of one warp
+// (list scan, then about three rounds of pairs), so there is no list in
+// memory, nothing to zero, and one rsqrt per atom pair.  480 waters: 23.5 to
+// 14.3 us a call.
 __global__ void __launch_bounds__(32 * kWaters) k_static_ww(const double *__restrict__ x, int nwat, double rc2,
                                                             const unsigned char *__restrict__ excl, float qo, float qh,
                                                             double A_OO, double B_OO, Scratch *scratch,
