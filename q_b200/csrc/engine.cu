@@ -1605,6 +1605,17 @@ void build(Batch &B, qb_handle *const *hs, int n) {
       return t;
     };
     while (B.ww_wpb > 32 && blocks(B.ww_wpb) < 2LL * sms) B.ww_wpb /= 2;
+    // FP64: one block per SM, so the launch takes as long as its rounds of
+    // blocks: the size with the least rounds x (waters + staging, about 24
+    // waters' time).  41 windows of 1,035 waters: 160 waters a block, two rounds,
+    // against 128 and three: 108 to 94 us, the step 183 to 177.  The packed kernel keeps the halving rule:
+    // its two blocks per SM overlap, other kernels fill its last round, and
+    // sizes that shortened it alone by 5% left the step as it was or slower.
+    if (B.opt.precision == QB_FP64 && blocks(32) > sms) {
+      auto cost = [&](int wpb) { return (blocks(wpb) + sms - 1) / sms * (wpb + 24); };
+      for (int wpb = 32; wpb <= WW_WPB; wpb += 32)
+        if (cost(wpb) < cost(B.ww_wpb)) B.ww_wpb = wpb;
+    }
     long long nw = 0;
     for (int s = 0; s < n; s++) nw += B.sysh[s].nwat;
     int thr = 2048;
