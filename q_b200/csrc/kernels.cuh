@@ -734,7 +734,11 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
 // Block = WL_WPB waters of one system, one warp per water at a time; the
 // system's O positions are staged in shared memory WL_STAGE waters at a time
 // in FP32, relative to the solvent centre (w = -1 for excluded waters), and
-// scanned 64 at a time (two per lane, packed FP32x2) with a ballot per 32.
+// scanned 64 at a time (two per lane, packed FP32x2) with a ballot per 32.  The
+// scan is bound by its instructions; waters lie near their neighbours in the
+// list's order, so most rounds have no water within the cut-off and end after
+// the distances: 100 systems of 1,390 waters 341 to 241 us, 41 of 1,035 143 to
+// 114.
 // The FP32 squared distance decides every pair farther than WL_EPS2 from the
 // cut-off; the few within it are decided in FP64 from the coordinates, so the
 // list is the reference's FP64 list exactly.  (|x| <= ~30 A from the centre:
@@ -755,7 +759,7 @@ __global__ void __launch_bounds__(WL_BLOCK) k_list_ww(DevPtrs P, int force) {
   const int obase = S.aoff + S.nsol;
   const double cx = S.pbc ? S.origin[0] : S.xw[0], cy = S.pbc ? S.origin[1] : S.xw[1],
                cz = S.pbc ? S.origin[2] : S.xw[2];
-  const float rc2 = (float)S.Rcww2;
+  const float rc2 = (float)S.Rcww2, far2 = rc2 + 2.f * WL_EPS2;
   // periodic box (nbwwlist_box, md.f90:8298): O-O distances of the nearest
   // image; FP32 edge lengths for the scan (the few pairs near the cut-off
   // are decided in FP64)
@@ -772,6 +776,8 @@ __global__ void __launch_bounds__(WL_BLOCK) k_list_ww(DevPtrs P, int force) {
       double4 x = P.x[o];
       so[t] = make_float4((float)(x.x - cx), (float)(x.y - cy), (float)(x.z - cz), (P.flags[o] & F_EXCL) ? -1.f : 1.f);
     }
+    // whole rounds of 64: the padding is excluded
+    for (int t = cn + threadIdx.x; t < (cn + 63) / 64 * 64; t += WL_BLOCK) so[t] = make_float4(0.f, 0.f, 0.f, -1.f);
     __syncthreads();
     for (int iw = i0 + warp; iw < i1; iw += nwarp) {
       const int gw = S.woff + iw;
@@ -787,10 +793,8 @@ __global__ void __launch_bounds__(WL_BLOCK) k_list_ww(DevPtrs P, int force) {
       int nxt = max(P.ww_chunk, (c0 + P.ww_chunk - 1) / P.ww_chunk * P.ww_chunk);
       for (int b = 0; b < cn; b += 64) {
         // lane takes j = b + lane and b + 32 + lane
-        float4 a = make_float4(0.f, 0.f, 0.f, -1.f), e = a;
         const int jl0 = b + lane, jl1 = b + 32 + lane;
-        if (jl0 < cn) a = so[jl0];
-        if (jl1 < cn) e = so[jl1];
+        const float4 a = so[jl0], e = so[jl1];
         float2 dx = __fadd2_rn(make_float2(a.x, e.x), nx), dy = __fadd2_rn(make_float2(a.y, e.y), ny),
                dz = __fadd2_rn(make_float2(a.z, e.z), nz);
         if (box) {
@@ -803,12 +807,15 @@ __global__ void __launch_bounds__(WL_BLOCK) k_list_ww(DevPtrs P, int force) {
           dz = wrap(dz, bL[2], biL[2]);
         }
         const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        // nothing near in the round, water i itself included, and no chunk
+        // ends in it: the next round
+        if (!__any_sync(FULL, fminf(r2.x, r2.y) <= far2) && nxt >= c0 + b + 64) continue;
         bool ok2[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int jl = h ? jl1 : jl0, jw = c0 + jl;
           const float w = h ? e.w : a.w, rr = h ? r2.y : r2.x;
-          bool ok = jl < cn && jw != iw && w > 0.f;
+          bool ok = jw != iw && w > 0.f;
           if (ok) {
             if (fabsf(rr - rc2) <= WL_EPS2) {
               // near the cut-off: the reference's FP64 test
