@@ -104,6 +104,11 @@ struct Batch {
   // 23 / 18, 8 and more the same, and the step gains only where the others
   // leave it SMs (1 to 3 windows)
   bool ww_direct = false;
+  // waters per block of the water list: WL_WPB, halved to no less than a warp
+  // each (16) while the blocks are fewer than two per SM.  A warp's waters
+  // follow each other, 3.5 us each: one window of 1,035 waters 63 to 10 us a
+  // rebuild, 21 windows 92 to 62.
+  int wl_wpb = WL_WPB;
   int ww_wpb0 = WW_WPB;         // the default of ww_wpb for this batch
   int max_nshell = 0;           // polarisation shells of the batch's systems, at most
   // the water pass takes a thread per water atom when that many threads
@@ -258,7 +263,7 @@ struct Batch {
       });
     }
     if (max_nwat > 0)
-      launch("list_ww", [&] { k_list_ww<<<dim3(cdiv(max_nwat, WL_WPB), nsys), WL_BLOCK, 0, s2>>>(p, force); });
+      launch("list_ww", [&] { k_list_ww<<<dim3(cdiv(max_nwat, wl_wpb), nsys), WL_BLOCK, 0, s2>>>(p, force, wl_wpb); });
     if (!any_any_atom) solute_lists();
     if (max_nsol > 0)
       launch("list_pp", [&] { k_list_pp<<<dim3(cdiv(max_nsol, PP_BLOCK / 32), nsys), PP_BLOCK, 0, stream>>>(p, force); });
@@ -1608,14 +1613,16 @@ void build(Batch &B, qb_handle *const *hs, int n) {
     // FP64: one block per SM, so the launch takes as long as its rounds of
     // blocks: the size with the least rounds x (waters + staging, about 24
     // waters' time).  41 windows of 1,035 waters: 160 waters a block, two rounds,
-    // against 128 and three: 108 to 94 us, the step 183 to 177.  The packed kernel keeps the halving rule:
-    // its two blocks per SM overlap, other kernels fill its last round, and
-    // sizes that shortened it alone by 5% left the step as it was or slower.
+    // against 128 and three: 108 to 94 us, the step 183 to 177.  The packed
+    // kernel keeps the halving rule: its two blocks per SM overlap, other
+    // kernels fill its last round, and sizes that shortened it alone by 5%
+    // left the step as it was or slower.
     if (B.opt.precision == QB_FP64 && blocks(32) > sms) {
       auto cost = [&](int wpb) { return (blocks(wpb) + sms - 1) / sms * (wpb + 24); };
       for (int wpb = 32; wpb <= WW_WPB; wpb += 32)
         if (cost(wpb) < cost(B.ww_wpb)) B.ww_wpb = wpb;
     }
+    while (B.wl_wpb > WL_BLOCK / 32 && blocks(B.wl_wpb) < 2LL * sms) B.wl_wpb /= 2;
     long long nw = 0;
     for (int s = 0; s < n; s++) nw += B.sysh[s].nwat;
     int thr = 2048;

@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
 // force-kernel chunk c (chunks of ww_chunk waters, a multiple of 32), so the
 // force kernel finds each chunk's slice of the list directly; ww_mid[gw]
 // counts the entries below i itself.
-// Block = WL_WPB waters of one system, one warp per water at a time; the
+// Block = wpb waters of one system, one warp per water at a time; the
 // system's O positions are staged in shared memory WL_STAGE waters at a time
 // in FP32, relative to the solvent centre (w = -1 for excluded waters), and
 // scanned 64 at a time (two per lane, packed FP32x2) with a ballot per 32.  The
@@ -746,13 +746,13 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
 constexpr int WL_BLOCK = 512, WL_WPB = 128, WL_STAGE = 2816;   // 44 KB of staged O positions
 constexpr float WL_EPS2 = 4e-3f;
 
-__global__ void __launch_bounds__(WL_BLOCK) k_list_ww(DevPtrs P, int force) {
+__global__ void __launch_bounds__(WL_BLOCK) k_list_ww(DevPtrs P, int force, int wpb) {
   int s = blockIdx.y;
   if (!list_due(P, s, force)) return;
   const SysDev &S = P.sys[s];
-  const int i0 = blockIdx.x * WL_WPB;
+  const int i0 = blockIdx.x * wpb;
   if (i0 >= S.nwat) return;
-  const int i1 = min(i0 + WL_WPB, S.nwat);
+  const int i1 = min(i0 + wpb, S.nwat);
   __shared__ float4 so[WL_STAGE];
   __shared__ int scnt[WL_WPB];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = WL_BLOCK / 32;

@@ -182,3 +182,21 @@ def test_analysis_block_edges(n, nskip):
     S = random_series(3, n, 2, seed=n)
     kw = dict(nbins=5, nmin=1, coeff=[1.0, -1.0])
     compare(analyze(S, params(0.592, nskip, **kw)), oracle_analyze(FepInput(S, 0.592, nskip, **kw)), 3)
+
+
+@pytest.mark.parametrize("radius,copies", [(28.0, 1), (15.0, 20), (15.0, 80)])
+def test_water_list_rounds(tmp_path, radius, copies):
+    """The water list's rounds of 64 waters with nothing near, chunks' ends
+    inside such rounds (chunks of 256), more waters than one staging (2,816)
+    and 16, 32 and 128 waters per block: the same pairs whatever the chunks, so
+    the FP64 forces differ by the order of ~1e3 terms (1e-13; bar 1e-11)."""
+    s = System.open(synth.water_sphere(str(tmp_path), radius=radius, seed=6).inp, seed=3)
+    a, b = Batch([s] * copies, precision=FP64), Batch([s], precision=FP64)
+    b.set_tuning(ww_chunk=256)
+    a.evaluate(True)
+    b.evaluate(True)
+    ga, gb = a.gradient(copies - 1), b.gradient(0)
+    assert np.abs(ga - gb).max() <= 1e-11 * np.abs(gb).max()
+    o = load_oracle().create(s)
+    o.final_energy()
+    assert np.abs(ga - o.gradient()).max() < 1e-4 * np.abs(ga).max()
