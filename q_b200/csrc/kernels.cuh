@@ -22,12 +22,6 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__device__ __forceinline__ float warp_sumf(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  return v;
-}
-
 // Sums of several values over a warp (or half of one) at once: at each level of
 // the tree a lane keeps half of its values and hands its partner the other
 // half, so nine values take 11 exchanges over 16 lanes (12 over 32) instead of 36
@@ -3140,8 +3134,9 @@ __global__ void __launch_bounds__(32 * QP_WARPS) k_solute_terms(DevPtrs P, Solut
 // The work is linear in the members.  Ranking by comparing every pair of
 // members and the force in a second launch took 7.5 + 5 us on one 1,000-water
 // sphere and 16 + 8 us on 100 systems, all of it latency; as one launch with
-// the counting sort 8.5 and 16.5 us (one FP64 chain of a dozen quotients and
-// roots per member, and the blocks' barriers, bound it now).
+// the counting sort 8.5 and 16.5 us, with its quotients by shared reciprocals
+// and the averages loaded ahead 14.6 on the 100 (one FP64 chain of roots and
+// angles per member, and the blocks' barriers, bound it now).
 // Shared memory: 12 bytes per water, as before (angle, 16-bit water index,
 // 16-bit place in the bin order).
 constexpr int WPOL_BLOCK = 512, WPOL_BINS = 1024;
