@@ -76,6 +76,8 @@ struct KernelStat { double ms = 0; long long launches = 0; };
 // Blocks per SM (of the one-part form) up to which the mixed LRF gather splits
 // its sums over a block's warps.
 constexpr int LRFX_CS_BLOCKS = 1;
+// Blocks per SM up to which its blocks are halved: all of them resident at once.
+constexpr int LRFX_NT_BLOCKS = 4;
 // Most waters of a batch that takes the water-water kernels without staging.
 constexpr int WWD_MAX_WATERS = 4096;
 
@@ -309,12 +311,18 @@ struct Batch {
   // block pays its staging and 20 atomics per target for a shorter chain).
   // Mixed: four warps share the sums of a block's targets (lrfx_cs 4) while the
   // launch has at most LRFX_CS_BLOCKS blocks per SM: at 315 blocks (21
-  // windows) sharing took 518 us a rebuild against 461.
-  int lrfx_cs = 1;
+  // windows) sharing took 518 us a rebuild against 461.  Up to LRFX_NT_BLOCKS
+  // blocks per SM, all run at once and the fullest SM decides (three of 315 on
+  // some of 148), and the last of a system's blocks is mostly idle (1,054
+  // targets in five blocks of 256): blocks of half the size (lrfx_nt) even
+  // both out, 21 windows 432 to 304 us.  Past that the blocks come in many
+  // rounds and the staging counts: 100 systems 1,086 to 1,173.
+  int lrfx_cs = 1, lrfx_nt = LRFX_BLOCK;
   void set_lrf_tpb(int tpb, bool share = true, int sms = 148) {
     P.lrf_tpb = tpb;
     P.lrf_sub = 1;
     lrfx_cs = 1;
+    lrfx_nt = LRFX_BLOCK;
     int blocks = 1;
     long long all = 0, allx = 0;
     for (const int2 &d : lrf_dims) {
@@ -326,16 +334,18 @@ struct Batch {
     if (share && tpb == 1)
       while (P.lrf_sub < 8 && all * P.lrf_sub * 2 <= 4LL * sms) P.lrf_sub *= 2;
     if (allx <= LRFX_CS_BLOCKS * (long long)sms) lrfx_cs = 4;
+    else if (allx <= LRFX_NT_BLOCKS * (long long)sms) lrfx_nt = LRFX_BLOCK / 2;
     max_lrf_blocks = blocks * P.lrf_sub;
     max_lrfx_blocks = 1;
     for (const int2 &d : lrf_dims)
-      max_lrfx_blocks = std::max(max_lrfx_blocks, cdiv(d.x, lrfx_targets(lrfx_cs)) * cdiv(d.y, tpb));
+      max_lrfx_blocks = std::max(max_lrfx_blocks, cdiv(d.x, lrfx_targets(lrfx_cs, lrfx_nt)) * cdiv(d.y, tpb));
   }
   template <bool BOX, bool ANY>
   void lrf_gather_mixed(cudaStream_t st, int force) {
     const dim3 g(max_lrfx_blocks, nsys);
-    if (lrfx_cs == 4) k_lrf_gather_x2<BOX, ANY, 4><<<g, LRFX_BLOCK, 0, st>>>(P, force);
-    else k_lrf_gather_x2<BOX, ANY, 1><<<g, LRFX_BLOCK, 0, st>>>(P, force);
+    if (lrfx_cs == 4) k_lrf_gather_x2<BOX, ANY, 4, LRFX_BLOCK><<<g, LRFX_BLOCK, 0, st>>>(P, force);
+    else if (lrfx_nt < LRFX_BLOCK) k_lrf_gather_x2<BOX, ANY, 1, LRFX_BLOCK / 2><<<g, LRFX_BLOCK / 2, 0, st>>>(P, force);
+    else k_lrf_gather_x2<BOX, ANY, 1, LRFX_BLOCK><<<g, LRFX_BLOCK, 0, st>>>(P, force);
   }
   void fork_streams(unsigned mask) {
     if (!forking()) return;

@@ -544,10 +544,10 @@ __device__ __forceinline__ void lrfx_fold(double *m, const double *t) {
 // thread and four times the blocks for a batch that cannot fill the chip: the
 // 518-group polymer 76 us a rebuild against about 300.
 constexpr int LRFX_BLOCK = 128;
-__host__ __device__ constexpr int lrfx_targets(int cs) { return 2 * LRFX_BLOCK / cs; }
+__host__ __device__ constexpr int lrfx_targets(int cs, int nt = LRFX_BLOCK) { return 2 * nt / cs; }
 
-template <bool BOX, bool ANY, int CS>
-__global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int force) {
+template <bool BOX, bool ANY, int CS, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) k_lrf_gather_x2(DevPtrs P, int force) {
   const int s = blockIdx.y;
   if (!list_due(P, s, force)) return;
   const SysDev &S = P.sys[s];
@@ -555,14 +555,14 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
   const int tpb = P.lrf_tpb;
   const int hsplit = max((S.nlrft + tpb - 1) / tpb, 1);
   const int gchunk = blockIdx.x / hsplit, hpart = blockIdx.x % hsplit;
-  if (S.nlrft == 0 || gchunk * lrfx_targets(CS) >= S.ncgp) return;
+  if (S.nlrft == 0 || gchunk * lrfx_targets(CS, NT) >= S.ncgp) return;
   const int t0 = hpart * tpb, t1 = min(t0 + tpb, S.nlrft);
   __shared__ double4 hsw[LRF_TILE_G];
   __shared__ int2 hrange[LRF_TILE_G];
   __shared__ float4 hxy[LRF_TILE_A], hzq[LRF_TILE_A];   // {x, x, y, y}, {z, z, q, q}
   __shared__ float2 psum[CS == 1 ? 1 : 24][CS == 1 ? 1 : 32];
   const double ox = S.origin[0], oy = S.origin[1], oz = S.origin[2];
-  // CS 1: thread t takes targets t and t + 128 of the block's 256; CS 4: lane
+  // CS 1: thread t takes targets t and t + NT of the block's 2 NT; CS 4: lane
   // l of every warp targets l and l + 32 of 64
   const int part = CS == 1 ? 0 : threadIdx.x >> 5;
   const int slot = CS == 1 ? threadIdx.x : threadIdx.x & 31;
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
   float cc[2][3];
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    gl[h] = gchunk * lrfx_targets(CS) + h * (lrfx_targets(CS) / 2) + slot;
+    gl[h] = gchunk * lrfx_targets(CS, NT) + h * (lrfx_targets(CS, NT) / 2) + slot;
     act[h] = gl[h] < S.ncgp;
     gsol[h] = gl[h] < S.ncgp_sol;
     xs[h] = cen[h] = make_double3(0, 0, 0);
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
     const int a0 = P.cg_first[S.coff + tile.x];
     const int na = P.cg_last[S.coff + tile.y - 1] - a0 + 1;
     __syncthreads();
-    for (int i = threadIdx.x; i < nh; i += LRFX_BLOCK) {
+    for (int i = threadIdx.x; i < nh; i += NT) {
       const int h = S.coff + tile.x + i;
       const int sw = P.cg_sw[h];
       const double3 p = ld3(P.x, ANY ? lrf_ref_atom(P, S, tile.x + i) : sw);
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(LRFX_BLOCK, 4) k_lrf_gather_x2(DevPtrs P, int 
       hsw[i] = make_double4(p.x, p.y, p.z, w);
       hrange[i] = make_int2(P.cg_first[h] - a0, P.cg_last[h] - P.cg_first[h] + 1);
     }
-    for (int i = threadIdx.x; i < na; i += LRFX_BLOCK) {
+    for (int i = threadIdx.x; i < na; i += NT) {
       const int at = P.cg_atoms[a0 + i];
       const double4 p = P.x[at];
       const bool qsol = (at - S.aoff) < S.nsol && P.iq[at] >= 0;

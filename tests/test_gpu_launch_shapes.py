@@ -200,3 +200,19 @@ def test_water_list_rounds(tmp_path, radius, copies):
     o = load_oracle().create(s)
     o.final_energy()
     assert np.abs(ga - o.gradient()).max() < 1e-4 * np.abs(ga).max()
+
+
+def test_field_gather_blocks(tmp_path):
+    """The mixed LRF gather with a block's sums shared by its warps, with blocks
+    of 64 threads and of 128 (1, 40 and 100 systems of 480 groups): the same
+    FP32 sums, FP64 atomics in another order (1e3 x 2^-53; bar 1e-11)."""
+    s = System.open(synth.water_sphere(str(tmp_path), radius=15.0, seed=6).inp, seed=3)
+    ref = None
+    for n in (1, 40, 100):
+        b = Batch([s] * n, precision=MIXED)
+        b.set_tuning(lrf_tiles_per_block=1)
+        b.evaluate(True)
+        g = b.gradient(n - 1)
+        ref = g if ref is None else ref
+        assert np.abs(g - ref).max() <= 1e-11 * np.abs(ref).max(), n
+        b.close()
