@@ -1652,7 +1652,11 @@ void build(Batch &B, qb_handle *const *hs, int n) {
   {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B.opt.device);
-    int tpb = LRF_TILES_PER_BLOCK;
+    // FP64: a tile per block always.  A target's 20 atomics are nothing beside
+    // a tile's FP64 work, and blocks of equal length fill the last round: 41
+    // windows with 4, 2 and 1 tiles 798, 717 and 667 us a rebuild, 100 systems
+    // 1,838, 1,732 and 1,701.
+    int tpb = B.opt.precision == QB_FP64 ? 1 : LRF_TILES_PER_BLOCK;
     B.set_lrf_tpb(tpb);
     while (tpb > 1 && (long long)B.max_lrf_blocks * n < 2LL * sms) B.set_lrf_tpb(tpb /= 2);
   }
